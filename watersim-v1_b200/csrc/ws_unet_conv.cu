@@ -27,6 +27,7 @@
 namespace unet {
 
 static constexpr long long kWaitLimit = 1LL << 24;
+constexpr int kConvThreads = 256;                   // threads of every kernel here
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -95,6 +96,7 @@ template <int COUT> struct ConvShape {
   static constexpr int MAXCTA = 512 / TCOLS;
   static constexpr int SMEM_MIN = 233472 / (MAXCTA + 1) + 1;
   static constexpr int SMEM = 2 * KSTR + WCH > SMEM_MIN ? 2 * KSTR + WCH : SMEM_MIN;
+  static constexpr int PERSM = 233472 / (SMEM + 1280) > 1 ? 233472 / (SMEM + 1280) : 1;   // CTAs one SM holds
 };
 
 // 16-byte asynchronous global -> shared copy; src_size 0 writes zeros
@@ -121,24 +123,27 @@ __device__ __forceinline__ void stage_halo(const ConvArgs& a, int X0, int Y0, in
   }
   __syncthreads();
   const int cnx = (a.nx + 1) >> 1, cny = (a.ny + 1) >> 1;
-  // one voxel per thread and pass, both 8-channel chunks of the slice (the
-  // channel splits c0 are multiples of 16, so both come from one source)
-  for (int hv = threadIdx.x; hv < HV; hv += blockDim.x) {
+  // the slice's source: both 8-channel chunks come from one (the channel
+  // splits c0 are multiples of 16)
+  const int c = kk * 16;
+  const bool first = c < a.c0, up = first && a.up0;
+  const bf16* src = first ? a.src0 + c : a.src1 + (c - a.c0);
+  const int stride = first ? a.c0 : a.c1;
+  const int sx = up ? cnx : a.nx, sy = up ? cny : a.ny, sh = up ? 1 : 0;
+  // one voxel per thread and pass, both 8-channel chunks of the slice; the
+  // passes are unrolled so that their address chains overlap (a block has two
+  // warps per scheduler: one chain after the other took 4.4 us per tile)
+  constexpr int PASSES = (HV + kConvThreads - 1) / kConvThreads;
+#pragma unroll
+  for (int it = 0; it < PASSES; it++) {
+    const int hv = (int)threadIdx.x + it * kConvThreads;
+    if (it == PASSES - 1 && hv >= HV) break;
     const int hx = hv % HX, t2 = hv / HX, hy = t2 % HY, hz = t2 / HY;
     const int gx = X0 - 1 + hx, gy = Y0 - 1 + hy, gz = Z0 - 1 + hz;
-    const bf16* p = a.src1 ? a.src1 : a.src0;             // any valid address when nothing is read
-    uint32_t n = 0;
-    if (gx >= 0 && gy >= 0 && gz >= 0 && gx < a.nx && gy < a.ny && gz < a.nz &&
-        s_act[((gz / kTZ - tz0) * 3 + (gy / kTY - ty0)) * 3 + (gx / kTX - tx0)]) {
-      const int c = kk * 16;
-      if (c < a.c0) {
-        p = a.up0 ? a.src0 + ((size_t)((gz >> 1) * cny + (gy >> 1)) * cnx + (gx >> 1)) * a.c0 + c
-                  : a.src0 + ((size_t)(gz * a.ny + gy) * a.nx + gx) * a.c0 + c;
-      } else {
-        p = a.src1 + ((size_t)(gz * a.ny + gy) * a.nx + gx) * a.c1 + (c - a.c0);
-      }
-      n = 16;
-    }
+    const bool in = (unsigned)gx < (unsigned)a.nx && (unsigned)gy < (unsigned)a.ny && (unsigned)gz < (unsigned)a.nz &&
+                    s_act[((gz / kTZ - tz0) * 3 + (gy / kTY - ty0)) * 3 + (gx / kTX - tx0)];
+    const bf16* p = in ? src + ((size_t)((gz >> sh) * sy + (gy >> sh)) * sx + (gx >> sh)) * stride : src;   // any valid address when nothing is read
+    const uint32_t n = in ? 16u : 0u;
     cp_async16(hbase + (uint32_t)(hv * 16), p, n);
     cp_async16(hbase + (uint32_t)(KSTR + hv * 16), p + 8, n);
   }
@@ -147,7 +152,8 @@ template <int COUT>
 __device__ __forceinline__ void stage_weights(const ConvArgs& a, int kk, uint32_t wbase) {
   constexpr int WCH = ConvShape<COUT>::WCH;
   const char* src = reinterpret_cast<const char*>(a.w) + (size_t)kk * WCH;
-  for (int i = threadIdx.x; i < WCH / 16; i += blockDim.x) cp_async16(wbase + (uint32_t)(i * 16), src + (size_t)i * 16, 16);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < WCH / 16; i += kConvThreads) cp_async16(wbase + (uint32_t)(i * 16), src + (size_t)i * 16, 16);
 }
 
 // Persistent over the work items (active tile x z sub-tile): tensor memory
@@ -155,7 +161,7 @@ __device__ __forceinline__ void stage_weights(const ConvArgs& a, int kk, uint32_
 // single 16-channel slice; the next item's first slice is fetched while
 // the current item's accumulators are drained.
 template <int COUT>
-__global__ void __launch_bounds__(256) k_conv3(ConvArgs a) {
+__global__ void __launch_bounds__(kConvThreads, ConvShape<COUT>::PERSM) k_conv3(ConvArgs a) {
   using S = ConvShape<COUT>;
   constexpr int ZT = S::ZT, HX = S::HX, HY = S::HY, KSTR = S::KSTR;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -312,97 +318,167 @@ __global__ void __launch_bounds__(256) k_conv3(ConvArgs a) {
 
 // ------------------------------------------------------------ weight gradient
 // dW[co][ci][t] += sum_v X(v + off_t)[ci] dZ(v)[co] over the voxels of
-// active tiles, on the tensor cores. One CTA per (active tile, 16-channel
-// input slice), persistent, one per SM. Per tap t the GEMM is D[co][ci] =
-// sum over voxels: A = dZ (M = 64 rows, cout <= 64 real), B = the input halo
-// shifted by the tap (N = 16 channels), K = 16 voxels (two x-rows of a plane)
-// per MMA. Both operands are MN-major: a core matrix is 8 channels (16
-// bytes) by 8 consecutive voxels; K groups are 128 bytes apart in the staged
-// dZ and one halo row (160 bytes) apart in the halo. The whole tile's dZ and
-// halo are staged once; the 8 planes x 8 K steps x 27 taps = 1728 MMAs are
-// issued back to back (taps innermost: 27 independent accumulators of 16
-// columns) with descriptors formed by adding 16-byte offsets to two base
-// descriptors, and drained once per item.
+// active tiles, on the tensor cores. A work item is one active tile and one
+// 16-channel input slice; the tile's dZ and the slice's halo are staged in
+// shared memory. K is voxels: 16 (two x-rows of a plane) per MMA, both
+// operands MN-major (a core matrix is 8 channels, 16 bytes, by 8 voxels).
+//
+// An MMA this small is bound by the shared-memory reads of its operands, so
+// one MMA covers as many taps as the operands' strides allow:
+//  - along M the z taps: with dZ stored plane by plane, the rows of planes
+//    p - 2, p - 1, p, ... are one run of 8-channel chunks at a fixed stride,
+//    and against halo plane p they are the taps dz = 2, 1, 0. 16 and 32
+//    output channels take four planes (M = 64, 128; the fourth is not used),
+//    64 take p - 1, p (M = 128) and p - 2 (M = 64). Zero planes below and
+//    above the tile stand for the planes that are not there.
+//  - along N the x taps: the B rows of taps dx = 0, 1, 2 are the same halo
+//    bytes one voxel (16 bytes) further, so the stride between 8-channel
+//    groups is 16 bytes and N = 24 holds three taps of 8 input channels
+//    (M = 128 wants a multiple of 16: N = 32, the fourth group not used).
+// That leaves (dy, channel half) = 6 accumulators and 10 planes x 8 K steps x
+// 6 = 480 MMAs per item (C = 64: 432 + 384) instead of 1728 of M = 64, N = 16
+// with one tap each, a quarter of the rows used at 16 channels.
+//
+// The accumulators stay in tensor memory over a CTA's whole run of items of
+// one slice (items are slice-major, a contiguous range per CTA) and drain
+// once per run into FP32 atomics. The bias gradient (slice 0) is summed by all
+// threads from the staged dZ while the MMAs run. Of an item's time at 16 channels
+// (two CTAs per SM) the MMAs are about 60% (23 cycles each, their operands'
+// 2.8 KB at 128 bytes per cycle); at 32 and 64 (one CTA) 63% and 58%, staging the
+// rest. Measured on the 128^3 planet (627 finest tiles): the ten layers of a
+// sample 2.89 -> 0.59 ms.
+//
 // one pass covers output channels coOff .. coOff + cout - 1 (cout <= 64) of a
 // dZ with dzStride channels per voxel
 struct DwTcArgs { ConvArgs src; const bf16* dz; int cout, dzStride, coOff; float* dw; float* db; };
-constexpr int kDzPlane = 128 * 16;                // bytes of one plane of one 8-channel chunk of dZ
-constexpr int kDzChunk = kTZ * kDzPlane;          // one 8-channel chunk of the tile's dZ
-constexpr int kDwTcSmem = 2 * ConvShape<16>::KSTR + 8 * kDzChunk;
-static_assert(kDwTcSmem + 1024 <= 232448, "halo and dZ of a tile fit one CTA's shared memory");
-// instruction descriptor: D f32, A and B bf16, both MN-major, M = 64, N = 16.
-// With M = 64 the accumulator rows 16q..16q+15 sit in tensor-memory lanes
-// 32q..32q+15 (the lower half of each 32-lane subpartition).
-constexpr uint32_t kIdescDw = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
-                              ((uint32_t)(16 >> 3) << 17) | ((uint32_t)(64 >> 4) << 24);
+template <int C> struct DwShape {
+  static constexpr int CH = C / 8;                  // 8-channel chunks of dZ
+  static constexpr int PLANE = CH * 128 * 16;       // bytes of one z plane of dZ
+  static constexpr int ZPAD = C == 64 ? 1 : 2;      // zero planes on either side of the tile
+  static constexpr int NPLANE = kTZ + 2 * ZPAD;
+  static constexpr int HALO = 2 * ConvShape<16>::KSTR;
+  // the halo lies behind the dZ: the rows of the unused fourth plane at the
+  // tile's top read its bytes, and 16 spare bytes end the last x tap group
+  static constexpr int SMEM = NPLANE * PLANE + HALO + 128;
+  static constexpr int ROWS = C == 16 ? 64 : 128;   // M of the first MMA kind
+  static constexpr int NCOL = C == 16 ? 24 : 32;
+  static constexpr int TCOLS = C == 64 ? 512 : 256; // 6 accumulators of 32 columns, twice at 64 channels
+  static constexpr int PERSM = C == 16 ? 2 : 1;     // CTAs one SM holds (shared memory)
+};
+static_assert(DwShape<16>::SMEM * 2 + 4096 <= 233472 && DwShape<32>::SMEM <= 231424 && DwShape<64>::SMEM <= 231424,
+              "halo and dZ of a tile fit the CTAs' shared memory");
+// instruction descriptor: D f32, A and B bf16, both MN-major. With M = 64 the
+// accumulator rows 16q..16q+15 sit in tensor-memory lanes 32q..32q+15 (the
+// lower half of each 32-lane subpartition).
+constexpr uint32_t idesc_dw(int m, int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(n >> 3) << 17) |
+         ((uint32_t)(m >> 4) << 24);
+}
 
-__global__ void __launch_bounds__(256, 1) k_dw_tc(DwTcArgs A) {
+template <int C>
+__global__ void __launch_bounds__(256, DwShape<C>::PERSM) k_dw_tc(DwTcArgs A) {
   const ConvArgs& a = A.src;
   using S = ConvShape<16>;                          // ZT = 8: the whole tile's halo of one slice
+  using D = DwShape<C>;
   constexpr int HX = S::HX, HY = S::HY, KSTR = S::KSTR;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
   __shared__ uint8_t s_act[27];
+  __shared__ float s_bias[8][64];
   const int cin = a.c0 + a.c1, nsl = cin >> 4, cout = A.cout;
-  const int nItems = *a.nTiles * nsl;
-  if ((int)blockIdx.x >= nItems) return;
+  const int nT = *a.nTiles;
+  const long long nItems = (long long)nT * nsl;
+  const int lo = (int)(nItems * blockIdx.x / gridDim.x), hi = (int)(nItems * (blockIdx.x + 1) / gridDim.x);
+  if (lo >= hi) return;                             // uniform over the CTA
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t hbase = smem_u32(smem), zbase = hbase + 2 * KSTR;
-  unsigned char* zbuf = smem + 2 * KSTR;
+  const uint32_t zbase = smem_u32(smem), hbase = zbase + (uint32_t)(D::NPLANE * D::PLANE);
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&s_tmem)), "r"(512u) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(smem_u32(&s_tmem)), "r"((uint32_t)D::TCOLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  if (threadIdx.x == 32) { mbar_init(&mbar, 1); s_abort = 0; }
-  // rows co >= cout of the A operand read zeros
-  for (int i = threadIdx.x; i < 8 * kDzChunk / 16; i += blockDim.x) reinterpret_cast<uint4*>(zbuf)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (threadIdx.x == 32) { mbar_init(&mbar, 3); s_abort = 0; }
+  // the zero planes, the rows co >= cout and the spare bytes
+  for (int i = threadIdx.x; i < D::SMEM / 16; i += blockDim.x) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = s_tmem;
-  const uint64_t adesc0 = smem_desc(zbase, 128, kDzChunk), bdesc0 = smem_desc(hbase, HX * 16, KSTR);
+  const uint64_t ad0 = smem_desc(zbase, 128, 128 * 16), bd0 = smem_desc(hbase, HX * 16, 16);
   uint32_t phase = 0;
-  bool pending = false;
-  for (int item = blockIdx.x; item < nItems && !s_abort; item += gridDim.x) {
-    const int tile = a.tiles[item / nsl], kk = item % nsl;
+  bool pending = false, fresh = true;
+  float bs[8] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };   // bias gradient of chunk (thread % CH)
+  for (int item = lo; item < hi; item++) {
+    const int kk = item / nT, tile = a.tiles[item - kk * nT];
     const int tx = tile % a.ntx, ty = (tile / a.ntx) % a.nty, tz = tile / (a.ntx * a.nty);
     const int X0 = tx * kTX, Y0 = ty * kTY, Z0 = tz * kTZ;
     stage_halo<16>(a, X0, Y0, Z0, kk, hbase, s_act);
-    for (int i = threadIdx.x; i < (cout >> 3) * kTZ * 128; i += blockDim.x) {
-      const int c = i / (kTZ * 128), r = i - c * (kTZ * 128), z = r >> 7, m = r & 127;
-      const int gx = X0 + (m & 7), gy = Y0 + (m >> 3), gz = Z0 + z;
-      const bool in = gx < a.nx && gy < a.ny && gz < a.nz;
-      const bf16* src = in ? A.dz + (((size_t)gz * a.ny + gy) * a.nx + gx) * A.dzStride + A.coOff + c * 8 : A.dz;
-      cp_async16(zbase + (uint32_t)(c * kDzChunk + z * kDzPlane + m * 16), src, in ? 16u : 0u);
+    {
+      // dZ: thread m of a 128-thread half takes voxel m of planes half, half + 2, ...
+      const int m = threadIdx.x & 127, gx = X0 + (m & 7), gy = Y0 + (m >> 3);
+      const bool inXY = gx < a.nx && gy < a.ny;
+      const bf16* col = A.dz + ((size_t)gy * a.nx + gx) * A.dzStride + A.coOff;
+      const size_t plane = (size_t)a.ny * a.nx * A.dzStride;
+#pragma unroll
+      for (int z = 0; z < kTZ; z += 2) {
+        const int zz = z + (int)(threadIdx.x >> 7);
+        const bool in = inXY && Z0 + zz < a.nz;
+        const bf16* src = in ? col + plane * (size_t)(Z0 + zz) : A.dz;
+#pragma unroll
+        for (int c = 0; c < D::CH; c++)
+          if (c * 8 < cout)
+            cp_async16(zbase + (uint32_t)((zz + D::ZPAD) * D::PLANE + c * 2048 + m * 16), in ? src + c * 8 : src, in ? 16u : 0u);
+      }
     }
     cp_async_wait_all();
     fence_proxy_async();
     __syncthreads();
-    if (threadIdx.x == 0) {
+    // One thread keeps the tensor pipe about half busy with MMAs this small,
+    // so three issue: warp w the accumulators of y tap w.
+    if (lane == 0 && warp < 3) {
       fence_after();
+      const uint32_t dcol = tmem + (uint32_t)(warp * 64);
+      const uint64_t bw = bd0 + (uint64_t)(warp * HX);
+      // halo plane p (voxel z = p - 1) against the dZ planes p - 2 .. p (taps dz = 2 .. 0)
 #pragma unroll 1
-      for (int z = 0; z < kTZ; z++) {
-#pragma unroll 1
-        for (int ks = 0; ks < 8; ks++) {
-          const uint64_t ad = adesc0 + (uint64_t)((z * kDzPlane + ks * 256) >> 4);
-          const uint32_t rowb = (uint32_t)(z * HY + 2 * ks) * HX;       // halo row of tap (0, 0, 0), 16-byte units
+      for (int p = 0; p < kTZ + 2; p++) {
+        const uint64_t bp = bw + (uint64_t)(p * HY * HX), ap = ad0 + (uint64_t)((p * D::PLANE) >> 4);
 #pragma unroll
-          for (int t = 0; t < 27; t++) {
-            const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;
-            const uint64_t bd = bdesc0 + (uint64_t)(rowb + (uint32_t)((dz * HY + dy) * HX + dx));
-            mma_bf16(tmem + (uint32_t)(t * 16), ad, bd, kIdescDw, (z | ks) != 0);
+        for (int ks = 0; ks < 8; ks++) {
+          const uint64_t bk = bp + (uint64_t)(2 * ks * HX), ak = ap + (uint64_t)(ks * 16);
+          const uint32_t first = (fresh && p == 0 && ks == 0) ? 0u : 1u;
+          if (C != 64) {                             // plane p - 2 up, two zero planes below
+            mma_bf16(dcol, ak, bk, idesc_dw(D::ROWS, D::NCOL), first);
+            mma_bf16(dcol + 32, ak, bk + (uint64_t)(KSTR >> 4), idesc_dw(D::ROWS, D::NCOL), first);
+          } else {
+            if (p < kTZ + 1) {                       // planes p - 1, p (one zero plane below)
+              mma_bf16(dcol, ak, bk, idesc_dw(128, 32), first);
+              mma_bf16(dcol + 32, ak, bk + (uint64_t)(KSTR >> 4), idesc_dw(128, 32), first);
+            }
+            if (p >= 2) {                            // plane p - 2
+              const uint32_t first2 = (fresh && p == 2 && ks == 0) ? 0u : 1u;
+              const uint64_t am = ak - (uint64_t)(D::PLANE >> 4);
+              mma_bf16(dcol + 192, am, bk, idesc_dw(64, 24), first2);
+              mma_bf16(dcol + 224, am, bk + (uint64_t)(KSTR >> 4), idesc_dw(64, 24), first2);
+            }
           }
         }
       }
       mma_commit(&mbar);
     }
     pending = true;
-    float bsum = 0.f;                                // bias gradient while the MMAs run
-    if (kk == 0 && (int)threadIdx.x < cout) {
-      const bf16* col = reinterpret_cast<const bf16*>(zbuf + (threadIdx.x >> 3) * kDzChunk) + (threadIdx.x & 7);
-      for (int m = 0; m < kTZ * 128; m++) bsum += __bfloat162float(col[m * 8]);
+    fresh = false;
+    if (kk == 0) {                                   // bias gradient while the MMAs run
+      const int c = threadIdx.x % D::CH;
+#pragma unroll 4
+      for (int v = threadIdx.x / D::CH; v < kTZ * 128; v += kConvThreads / D::CH) {
+        const uint4 u = *reinterpret_cast<const uint4*>(smem + ((v >> 7) + D::ZPAD) * D::PLANE + c * 2048 + (v & 127) * 16);
+        const bf16* e = reinterpret_cast<const bf16*>(&u);
+#pragma unroll
+        for (int q = 0; q < 8; q++) bs[q] += __bfloat162float(e[q]);
+      }
     }
     const bool ok = mbar_wait(&mbar, phase);
     if (!ok) { s_abort = 1; atomicOr(a.err, WS_DERR_TIMEOUT); }
@@ -410,40 +486,88 @@ __global__ void __launch_bounds__(256, 1) k_dw_tc(DwTcArgs A) {
     if (s_abort) break;
     pending = false;
     phase ^= 1u;
+    if (item + 1 < hi && (item + 1) / nT == kk) continue;   // the run goes on: the accumulators stay
     fence_after();
-    {
-      const int q = warp & 3, co = lane < 16 ? q * 16 + lane : 1 << 20;   // accumulator row of this lane
-      for (int t = warp >> 2; t < 27; t += 2) {
-        uint32_t r[16];
-        tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(t * 16), r);
-        if (co < cout) {
+    // Accumulator columns dx * 8 + (input channel of the half); rows: see
+    // above. One channel half at a time goes to shared memory (over the halo,
+    // which the next item stages anew) in the order of dW, a row of 8 x 27 per
+    // output channel padded to an odd stride, and from there to global memory
+    // with neighbouring lanes on neighbouring addresses: an atomic per lane on
+    // a sector of its own cost 8 us more at 16 channels, where 296 CTAs add to
+    // the same 27 KB.
+    const int q = warp & 3;
+    float* st = reinterpret_cast<float*>(smem + D::NPLANE * D::PLANE);
+    constexpr int ROW = 8 * 27 + 1;
+    static_assert(C * ROW * 4 <= D::HALO, "one channel half of dW fits the halo's place");
+    for (int half = 0; half < 2; half++) {
+      for (int jj = warp >> 2; jj < (C == 64 ? 6 : 3); jj += 2) {
+        const int dy = jj % 3, j = 2 * dy + half + (jj >= 3 ? 6 : 0);
+        int co, dz;
+        if (C == 16) { co = lane < 16 ? lane : 64; dz = 2 - q; }
+        else if (C == 32) { co = lane; dz = 2 - q; }
+        else if (j < 6) { co = (q & 1) * 32 + lane; dz = 1 - (q >> 1); }
+        else { co = lane < 16 ? q * 16 + lane : 64; dz = 2; }
+        uint32_t r0[16], r1[16];                     // taps dx = 0, 1 and dx = 2 (upper half of r1 unused)
+        const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(j * 32);
+        tmem_ld16(at, r0);
+        tmem_ld16(at + 16, r1);
+        if (co >= cout || dz < 0) continue;
+        float* dst = st + co * ROW + dz * 9 + dy * 3;
 #pragma unroll
-          for (int i = 0; i < 16; i++)
-            atomicAdd(A.dw + ((size_t)(A.coOff + co) * cin + kk * 16 + i) * 27 + t, __uint_as_float(r[i]));
+        for (int i = 0; i < 8; i++) {
+          dst[i * 27] = __uint_as_float(r0[i]);
+          dst[i * 27 + 1] = __uint_as_float(r0[8 + i]);
+          dst[i * 27 + 2] = __uint_as_float(r1[i]);
         }
       }
+      __syncthreads();
+      for (int co = warp; co < cout; co += 8) {
+        float* dst = A.dw + ((size_t)(A.coOff + co) * cin + kk * 16 + half * 8) * 27;
+#pragma unroll
+        for (int r = 0; r < 7; r++)
+          if (r * 32 + lane < 8 * 27) atomicAdd(dst + r * 32 + lane, st[co * ROW + r * 32 + lane]);
+      }
+      __syncthreads();
     }
-    if (kk == 0 && (int)threadIdx.x < cout) atomicAdd(A.db + A.coOff + threadIdx.x, bsum);
+    if (kk == 0) {
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        float v = bs[e];
+        for (int o = 16; o >= D::CH; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane < D::CH) s_bias[warp][lane * 8 + e] = v;
+        bs[e] = 0.f;
+      }
+      __syncthreads();
+      if ((int)threadIdx.x < cout) {
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; w++) v += s_bias[w][threadIdx.x];
+        atomicAdd(A.db + A.coOff + threadIdx.x, v);
+      }
+    }
+    fresh = true;
     fence_before();
-    __syncthreads();                                 // accumulators and staged operands free for the next item
+    __syncthreads();                                 // accumulators free for the next run
   }
   if (s_abort && pending) mbar_wait(&mbar, phase);
   cp_async_wait_all();
   fence_before();
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"((uint32_t)D::TCOLS) : "memory");
 }
 cudaError_t launch_dw_tc(const ConvArgs& src, const bf16* dz, int cout, float* dw, float* db, int maxItems,
                          cudaStream_t s) {
   if (((src.c0 + src.c1) & 15) || (cout & 7) || cout > 128) return cudaErrorInvalidValue;
   static int smCount = 0;
   if (!smCount) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&smCount, cudaDevAttrMultiProcessorCount, dev); }
-  const unsigned grid = (unsigned)std::min(maxItems, smCount);     // one CTA per SM: 512 TMEM columns each
-  if (grid == 0) return cudaSuccess;
+  if (maxItems <= 0) return cudaSuccess;
   for (int off = 0; off < cout; off += 64) {       // the A operand holds 64 output channels per pass
     DwTcArgs A{src, dz, std::min(64, cout - off), cout, off, dw, db};
-    k_dw_tc<<<grid, 256, kDwTcSmem, s>>>(A);
+    // the narrowest shape that holds the pass's channels: fewer rows are fewer bytes per MMA
+    if (A.cout <= 16) k_dw_tc<16><<<std::min(maxItems, smCount * DwShape<16>::PERSM), 256, DwShape<16>::SMEM, s>>>(A);
+    else if (A.cout <= 32) k_dw_tc<32><<<std::min(maxItems, smCount), 256, DwShape<32>::SMEM, s>>>(A);
+    else k_dw_tc<64><<<std::min(maxItems, smCount), 256, DwShape<64>::SMEM, s>>>(A);
   }
   return cudaGetLastError();
 }
@@ -460,8 +584,9 @@ cudaError_t conv3_init() {
   if ((e = set_smem<96>()) != cudaSuccess) return e;
   if ((e = set_smem<128>()) != cudaSuccess) return e;
   if ((e = set_smem<192>()) != cudaSuccess) return e;
-  // the weight-gradient kernel holds more than half an SM's shared memory: one CTA per SM
-  return cudaFuncSetAttribute(k_dw_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kDwTcSmem);
+  if ((e = cudaFuncSetAttribute(k_dw_tc<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, DwShape<16>::SMEM)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(k_dw_tc<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, DwShape<32>::SMEM)) != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_dw_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, DwShape<64>::SMEM);
 }
 int conv3_zt(int cout) {
   switch (cout) {

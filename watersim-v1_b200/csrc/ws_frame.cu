@@ -655,9 +655,9 @@ __global__ void k_splat(Dims d, GridDev g, PartsDev P, double spacing) {
   long long sj = d.nx + 1, sk = (long long)(d.ny + 1) * sj;
   double X = P.px[p], Y = P.py[p], Z = P.pz[p];
   double fi = floor(over_dx(d, X)), fj = floor(over_dx(d, Y)), fk = floor(over_dx(d, Z));
-  int i0 = fi < 0 ? 0 : (fi > d.nx - 1 ? d.nx - 1 : (int)fi);
-  int j0 = fj < 0 ? 0 : (fj > d.ny - 1 ? d.ny - 1 : (int)fj);
-  int k0 = fk < 0 ? 0 : (fk > d.nz - 1 ? d.nz - 1 : (int)fk);
+  int i0 = !(fi >= 0) ? 0 : (fi > d.nx - 1 ? d.nx - 1 : (int)fi);
+  int j0 = !(fj >= 0) ? 0 : (fj > d.ny - 1 ? d.ny - 1 : (int)fj);
+  int k0 = !(fk >= 0) ? 0 : (fk > d.nz - 1 ? d.nz - 1 : (int)fk);
   double fx = X - i0 * dx, fy = Y - j0 * dx, fz = Z - k0 * dx;
   for (int kk = 0; kk < 2; kk++) {
     double czz = kk == 0 ? fz : fz - dx;

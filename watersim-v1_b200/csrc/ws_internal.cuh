@@ -238,7 +238,7 @@ __device__ __forceinline__ float sor_update(float qc, float pw, float rhs, float
 }
 __device__ __forceinline__ int jfloor_clamp(double v, int a, int b) {
   double f = floor(v);
-  if (f < a) return a;
+  if (!(f >= a)) return a;       // a NaN too: its conversion from double gives the most negative int
   if (f > b) return b;
   return (int)f;
 }
@@ -304,10 +304,10 @@ __device__ __forceinline__ void face_coords(const Dims& d, int comp, double x, d
   if (comp == 0) { a = X; b = Y - 0.5; c = Z - 0.5; }
   else if (comp == 1) { a = X - 0.5; b = Y; c = Z - 0.5; }
   else { a = X - 0.5; b = Y - 0.5; c = Z; }
-  double fi = floor(a), fj = floor(b), fk = floor(c);
-  if (fi < 0) { i0 = 0; tx = 0; } else if (fi > d.nx - 1) { i0 = d.nx - 1; tx = 1; } else { i0 = (int)fi; tx = a - fi; }
-  if (fj < 0) { j0 = 0; ty = 0; } else if (fj > d.ny - 2) { j0 = d.ny - 2; ty = 1; } else { j0 = (int)fj; ty = b - fj; }
-  if (fk < 0) { k0 = 0; tz = 0; } else if (fk > d.nz - 2) { k0 = d.nz - 2; tz = 1; } else { k0 = (int)fk; tz = c - fk; }
+  double fi = floor(a), fj = floor(b), fk = floor(c);   // a NaN takes index 0 (see jfloor_clamp)
+  if (!(fi >= 0)) { i0 = 0; tx = 0; } else if (fi > d.nx - 1) { i0 = d.nx - 1; tx = 1; } else { i0 = (int)fi; tx = a - fi; }
+  if (!(fj >= 0)) { j0 = 0; ty = 0; } else if (fj > d.ny - 2) { j0 = d.ny - 2; ty = 1; } else { j0 = (int)fj; ty = b - fj; }
+  if (!(fk >= 0)) { k0 = 0; tz = 0; } else if (fk > d.nz - 2) { k0 = d.nz - 2; tz = 1; } else { k0 = (int)fk; tz = c - fk; }
 }
 // flat offset into vel (u|v|w) and the j/k strides of component comp
 __device__ __forceinline__ void face_strides(const Dims& d, int comp, int i0, int j0, int k0,

@@ -16,11 +16,9 @@
  *    the next call that synchronises.
  *  - Host pointers are owned by the caller and read or written only during
  *    the call. Device memory is owned by the handle.
- *  - One CUDA stream per handle (ws_get_stream); with the learned warm start
- *    on, the pressure stage forks the SOR list build onto a second, internal
- *    stream and joins it back before the solve, so all of a call's work is
- *    still ordered after earlier work on the handle's stream and before later
- *    work on it. Calls on one handle must be serialised by
+ *  - One CUDA stream per handle (ws_get_stream): all of a call's work is
+ *    ordered after earlier work on it and before later work on it.
+ *    Calls on one handle must be serialised by
  *    the caller (a frame started by ws_step_async holds the handle until it
  *    is collected; other calls meanwhile return WS_ERR_BUSY). There is no
  *    global mutable state, so different handles may be used from different
@@ -113,8 +111,9 @@ typedef struct {
   int32_t nP, capacity;
   int32_t airborneCount, vaporCount, nightVaporCount, evapCount, substepsLast, nFluid;
   int32_t sorIters;        /* iterations run by the last solve */
-  int32_t sorPath;         /* solve path of the last solve: 1 grid-wide colour lists, 2 cluster-resident
-                              colour lists, 3 temporal-blocked on every SM (shared-memory regions),
+  int32_t sorPath;         /* solve path of the last solve: 1 grids above 160^3, every SM's lists in shared
+                              memory or (where they do not fit) grid-wide, 2 cluster-resident colour lists,
+                              3 temporal-blocked on every SM (shared-memory regions),
                               4 owned bricks in global memory on every SM (regions too large) */
 } ws_scalars;
 

@@ -24,8 +24,6 @@ struct MeshBuf {
 struct ws_handle {
   int device = 0;
   cudaStream_t stream = nullptr;
-  cudaStream_t side = nullptr;          // the SOR list build beside the learned warm start
-  cudaEvent_t evFork = nullptr, evJoin = nullptr;
   // host copies of the particle fields no substep kernel reads or writes
   // (ws_upload_state / ws_download_state) run on their own stream beside the
   // substep; every other entry point joins them into the main stream first
@@ -74,7 +72,6 @@ struct ws_handle {
   CellSort csort{};                     // the particles sorted by cell for P2G
   void* csortCub = nullptr;             // prefix-sum scratch
   size_t csortCubBytes = 0;
-  bool tbSetup = false;                 // the pressure setup may run over bricks (the solve needs no block counts)
   // substep graph: the kernel sequence of one substep captured once and
   // replayed while its launch parameters stay the same
   cudaGraphExec_t gexec = nullptr;
@@ -150,7 +147,7 @@ static GridDev grid_of(ws_handle* h) {
   g.omx = h->vort + 4 * N; g.omy = h->vort + 5 * N; g.omz = h->vort + 6 * N;
   g.dens = h->dens;
   g.sv = h->sv;
-  g.seed = h->bricks.seed; g.nbx = h->bricks.nbx; g.nby = h->bricks.nby;
+  g.seed = h->bricks.seed; g.nbx = h->bricks.nbx; g.nby = h->bricks.nby; g.fmask = h->bricks.fmask;
   return g;
 }
 // the next substep processes every brick (after a caller or a single stage wrote grid fields)
@@ -217,7 +214,7 @@ static void free_all(ws_handle* h) {
   if (h->mtScratch) cudaFree(h->mtScratch);
   if (h->queryBuf) cudaFree(h->queryBuf);
   {
-    void* bb[] = { h->bricks.seed, h->bricks.act, h->bricks.proc, h->bricks.list, h->bricks.count, h->bricks.forceAll,
+    void* bb[] = { h->bricks.seed, h->bricks.act, h->bricks.proc, h->bricks.list, h->bricks.count, h->bricks.forceAll, h->bricks.fmask,
                    h->csort.count, h->csort.start, h->csort.pcell, h->csort.pslot,
                    h->csort.perm, h->csortCub };
     for (void* b : bb) if (b) cudaFree(b);
@@ -235,12 +232,9 @@ static void free_all(ws_handle* h) {
   if (h->rdrScratch) cudaFree(h->rdrScratch);
   if (h->stHost) cudaFreeHost(h->stHost);
   if (h->redHost) cudaFreeHost(h->redHost);
-  if (h->evFork) cudaEventDestroy(h->evFork);
-  if (h->evJoin) cudaEventDestroy(h->evJoin);
   if (h->evCopy) cudaEventDestroy(h->evCopy);
   if (h->evMain) cudaEventDestroy(h->evMain);
   if (h->copyStream) cudaStreamDestroy(h->copyStream);
-  if (h->side) cudaStreamDestroy(h->side);
   if (h->stream) cudaStreamDestroy(h->stream);
 }
 
@@ -262,21 +256,15 @@ extern "C" ws_status ws_create(const ws_config* cfg, ws_handle** out) {
   cudaError_t e = cudaSetDevice(cfg->device);
   if (e != cudaSuccess) { ws_status r = fail_cuda(h, e, "cudaSetDevice"); delete h; return r; }
   e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->evFork, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->evJoin, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->copyStream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->evCopy, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->evMain, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     ws_status r = fail_cuda(h, e, "cudaStreamCreate");
-    if (h->evFork) cudaEventDestroy(h->evFork);
-    if (h->evJoin) cudaEventDestroy(h->evJoin);
     if (h->evCopy) cudaEventDestroy(h->evCopy);
     if (h->evMain) cudaEventDestroy(h->evMain);
     if (h->copyStream) cudaStreamDestroy(h->copyStream);
-    if (h->side) cudaStreamDestroy(h->side);
-    if (h->stream) cudaStreamDestroy(h->stream);
+      if (h->stream) cudaStreamDestroy(h->stream);
     delete h; return r;
   }
   Dims& d = h->d;
@@ -316,13 +304,12 @@ extern "C" ws_status ws_create(const ws_config* cfg, ws_handle** out) {
   AL(h->partials, partN)
   if ((e = sor_init(&h->sor, h->d, cfg->device)) != cudaSuccess) { ws_status r = fail_cuda(h, e, "SOR state"); free_all(h); delete h; return r; }
   h->partialsCap = (int)partN;
-  h->tbSetup = sor_uses_tb(h->sor);
   {
     BrickSet& B = h->bricks;
     B.nbx = (d.nx + 3) / 4; B.nby = (d.ny + 3) / 4; B.nbz = (d.nz + 3) / 4;
     B.dnbx = fastdiv_make((unsigned)B.nbx); B.dnby = fastdiv_make((unsigned)B.nby);
     const long long nB = (long long)B.nbx * B.nby * B.nbz;
-    AL(B.seed, nB) AL(B.act, nB) AL(B.proc, nB) AL(B.list, nB) AL(B.count, 1) AL(B.forceAll, 1)
+    AL(B.seed, nB) AL(B.act, nB) AL(B.proc, nB) AL(B.list, nB) AL(B.count, 1) AL(B.forceAll, 1) AL(B.fmask, nB)
     CellSort& cs = h->csort;
     AL(cs.count, 64 * nB + 1) AL(cs.start, 64 * nB + 1) AL(cs.pcell, P) AL(cs.pslot, P) AL(cs.perm, P)
     cs.cap = (int)P;
@@ -881,9 +868,7 @@ static ws_status stage_forces(ws_handle* h, double dt, double gsA, bool bricks =
 // FP64 residual land in the status word and are read at the next sync.
 static ws_status stage_pressure(ws_handle* h, bool bricks = false) {
   GridDev g = grid_of(h);
-  // the colour-list solves need the setup's per-block counts over the whole grid
-  if (bricks && h->tbSetup) launch_pressure_setup_bricks(h->d, g, h->diag8, h->P.omega, h->st, h->bricks, h->stream);
-  else launch_pressure_setup(h->d, g, h->diag8, h->P.omega, h->st, sor_block_counts(h->sor), h->stream);
+  launch_pressure_setup(h->d, g, h->diag8, h->P.omega, h->st, h->bricks, !bricks, h->stream);
   ws_status s = check_launch(h, 1); if (s) return s;
   bool tolMode = h->P.sorTol > 0;
   int iters = tolMode ? h->P.sorMaxIters : h->P.pressureIters;
@@ -895,31 +880,12 @@ static ws_status stage_pressure(ws_handle* h, bool bricks = false) {
       return fail_cuda(h, e, "warm-start pair (before the solve)");
   }
   if (h->net && h->unetOn) {
-    // the colour lists on the side stream while the network predicts q (they do not read q)
-    WS_TRY(cudaEventRecord(h->evFork, h->stream));
-    // From here on every exit joins the side stream back into the main one,
-    // so a capture in progress ends with no unjoined stream and reports the
-    // first error rather than an unjoined-capture one.
-    struct SideJoin {
-      ws_handle* h; bool armed;
-      ~SideJoin() {
-        if (armed && cudaEventRecord(h->evJoin, h->side) == cudaSuccess) cudaStreamWaitEvent(h->stream, h->evJoin, 0);
-      }
-    } join{ h, true };
-    WS_TRY(cudaStreamWaitEvent(h->side, h->evFork, 0));
-    if ((e = launch_sor_lists(h->sor, h->d, g, h->diag8, h->side)) != cudaSuccess) return fail_cuda(h, e, "SOR lists");
-    WS_TRY(cudaEventRecord(h->evJoin, h->side));
     if ((e = h->net->predict(h->q, h->rhs, h->diag8, h->type, h->stream)) != cudaSuccess)
       return fail_cuda(h, e, "learned warm start");
     h->launches += 23;
-    join.armed = false;
-    WS_TRY(cudaStreamWaitEvent(h->stream, h->evJoin, 0));
-    e = launch_sor_run(h->sor, h->d, g, h->diag8, h->P.omega, iters, check, h->P.sorTol, &h->st->err, &dIters, &dRel,
-                       &dPath, h->stream);
-  } else {
-    e = launch_sor_solve(h->sor, h->d, g, h->diag8, h->P.omega, iters, check, h->P.sorTol,
-                         &h->st->err, &dIters, &dRel, &dPath, h->stream);
   }
+  e = launch_sor_solve(h->sor, h->d, g, h->diag8, h->P.omega, iters, check, h->P.sorTol, h->st, &dIters, &dRel, &dPath,
+                       h->stream);
   if (e != cudaSuccess) return fail_cuda(h, e, "SOR solve launch");
   s = check_launch(h, sor_solve_launches(h->sor)); if (s) return s;
   WS_TRY(cudaMemcpyAsync(&h->st->sorIters, dIters, sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
@@ -1574,7 +1540,7 @@ extern "C" ws_status ws_time_kernel(ws_handle* h, int32_t kernel, int32_t reps, 
       case 5: launch_project(h->d, g, 1, h->P.maxSpeed, h->st, h->stream); break;
       case 6: { int* di; double* dr; int* dp;
                 cudaError_t e6 = launch_sor_solve(h->sor, h->d, g, h->diag8, h->P.omega, h->P.pressureIters, 0, 0,
-                                                  &h->st->err, &di, &dr, &dp, h->stream);
+                                                  h->st, &di, &dr, &dp, h->stream);
                 if (e6 != cudaSuccess) { cudaEventDestroy(e0); cudaEventDestroy(e1); return fail_cuda(h, e6, "SOR solve"); }
                 h->launches += sor_solve_launches(h->sor) - 1; } break;   // list build; timed per whole solve
       case 8: launch_faces_normalize_bc_bricks(h->d, g, h->bricks, h->stream); break;
@@ -1587,7 +1553,7 @@ extern "C" ws_status ws_time_kernel(ws_handle* h, int32_t kernel, int32_t reps, 
                  h->launches += n12 - 1; } break;
       case 7: { int* di; double* dr; int* dp;
                 cudaError_t e7 = launch_sor_solve_lists(h->sor, h->d, g, h->diag8, h->P.omega, h->P.pressureIters, 0, 0,
-                                                        &h->st->err, &di, &dr, &dp, h->stream);
+                                                        h->st, &di, &dr, &dp, h->stream);
                 if (e7 != cudaSuccess) { cudaEventDestroy(e0); cudaEventDestroy(e1); return fail_cuda(h, e7, "SOR solve"); }
                 h->launches += sor_list_solve_launches(h->sor) - 1; } break;
       default: cudaEventDestroy(e0); cudaEventDestroy(e1); return fail(h, WS_ERR_INVALID, "unknown kernel id");
@@ -1748,7 +1714,7 @@ extern "C" ws_status ws_unet_probe(ws_handle* h, double* relres_prev, double* re
   ws_status s = net_ready(h); if (s) return s;
   if (!(h->net->gain > 0)) return fail(h, WS_ERR_STATE, "network has no output gain");
   GridDev g = grid_of(h);
-  launch_pressure_setup(h->d, g, h->diag8, h->P.omega, h->st, sor_block_counts(h->sor), h->stream);
+  launch_pressure_setup(h->d, g, h->diag8, h->P.omega, h->st, h->bricks, true, h->stream);
   if ((s = check_launch(h, 1))) return s;
   launch_residual(h->d, g, h->diag8, h->partials, h->st, nullptr, h->stream);
   if ((s = check_launch(h, 2))) return s;

@@ -105,7 +105,7 @@ __global__ void k_clear_raster(Dims d, GridDev g, DevStatus* st, int clearAcc) {
   }
   if (t < n16) reinterpret_cast<uint4*>(g.type)[t] = reinterpret_cast<const uint4*>(g.staticTypes)[t];
   else if (t < n16 + (d.nCells & 15)) { const long long c = (n16 << 4) + (t - n16); g.type[c] = g.staticTypes[c]; }
-  if (t == 0) { st->umaxBits = 0u; st->airborne = 0; st->nFluid = 0; }
+  if (t == 0) { st->umaxBits = 0u; st->airborne = 0; st->nFluid = 0; st->oddFluid = 0; }
 }
 void launch_clear_raster(const Dims& d, const GridDev& g, DevStatus* st, bool clearAcc, cudaStream_t s) {
   const long long a = clearAcc ? (d.F >> 1) + 1 : 0, b = (d.nCells >> 4) + 16;
@@ -583,10 +583,9 @@ void launch_faces_forces(const Dims& d, const GridDev& g, double coef, int viscO
 // ------------------------------------------------------------ 6. pressure setup
 // _pressureSolve passes 1-2, js/solver.js:1321-1366: q = 0 off the fluid,
 // diag = Nf + Na, rhs = -dx^2 div, relaxation weight pw = omega/diag
-// (float32, as the reference's pW). pw < 0 marks a non-fluid cell. Each
-// 256-cell block also counts its interior fluid cells per colour for the SOR
-// list build (sorCounts[2 b], [2 b + 1]; null skips) and adds its fluid
-// cells to the fluid count with one atomic.
+// (float32, as the reference's pW). pw < 0 marks a non-fluid cell. The pass
+// (k_pressure_setup, below the brick list) also leaves each 4^3 brick's mask
+// of interior fluid cells, from which the solve builds its plan.
 // one cell of the setup: returns whether it is fluid and its SOR colour (-1 off the lists)
 __device__ __forceinline__ bool cell_pressure_setup(const Dims& d, const GridDev& g, uint8_t* __restrict__ diag8,
                                                     double omega, long long c, int i, int j, int k, int& col) {
@@ -610,32 +609,6 @@ __device__ __forceinline__ bool cell_pressure_setup(const Dims& d, const GridDev
   if (i >= 1 && j >= 1 && k >= 1 && i + 2 <= nx && j + 2 <= ny && k + 2 <= nz) col = (i + j + k) & 1;
   return true;
 }
-__global__ void __launch_bounds__(256) k_pressure_setup(Dims d, GridDev g, uint8_t* __restrict__ diag8, double omega,
-                                                        DevStatus* st, int* __restrict__ sorCounts) {
-  __shared__ int wc[3][8];                           // per warp: colour-0 and colour-1 list cells, fluid cells
-  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  int col = -1, fluid = 0;
-  if (c < d.nCells) {
-    int i, j, k; decode_cell(d, c, i, j, k);
-    fluid = cell_pressure_setup(d, g, diag8, omega, c, i, j, k, col) ? 1 : 0;
-  }
-  const unsigned full = 0xffffffffu;
-  const unsigned m0 = __ballot_sync(full, col == 0), m1 = __ballot_sync(full, col == 1), mf = __ballot_sync(full, fluid);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) { wc[0][wid] = __popc(m0); wc[1][wid] = __popc(m1); wc[2][wid] = __popc(mf); }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int a = 0, b = 0, f = 0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); q++) { a += wc[0][q]; b += wc[1][q]; f += wc[2][q]; }
-    if (sorCounts) { sorCounts[2 * blockIdx.x] = a; sorCounts[2 * blockIdx.x + 1] = b; }
-    if (f) atomicAdd(&st->nFluid, f);
-  }
-}
-void launch_pressure_setup(const Dims& d, const GridDev& g, uint8_t* diag8, double omega, DevStatus* st, int* sorCounts,
-                           cudaStream_t s) {
-  k_pressure_setup<<<grid_for(d.nCells, 256), 256, 0, s>>>(d, g, diag8, omega, st, sorCounts);
-}
-
 // ------------------------------------------------------------ 7. red-black SOR
 // One colour of the SOR sweep, js/solver.js:1397-1404 in red-black order:
 // q <- q (1 - omega) + pw (rhs + sum of the six neighbour q), FP64 arithmetic
@@ -1062,28 +1035,37 @@ void launch_extrapolate_bricks(const Dims& d, const GridDev& g, const BrickSet& 
 void launch_clear_acc_bricks(const Dims& d, const GridDev& g, const BrickSet& B, cudaStream_t s) {
   k_faces_bricks<4><<<brick_grid(B), 256, 0, s>>>(d, g, B, FacePassArgs{}, nullptr);
 }
-// the pressure setup over the brick list: four bricks per 256-thread block
-__global__ void __launch_bounds__(256) k_pressure_setup_bricks(Dims d, GridDev g, uint8_t* __restrict__ diag8,
-                                                               double omega, DevStatus* st, BrickSet B) {
-  const int n = *B.count;
-  int fluid = 0;
+// the pressure setup over the brick list (or every brick): four bricks per
+// 256-thread block, a brick's two warps ballot its mask
+__global__ void __launch_bounds__(256) k_pressure_setup(Dims d, GridDev g, uint8_t* __restrict__ diag8, double omega,
+                                                        DevStatus* st, BrickSet B, int allBricks) {
+  const int n = allBricks ? B.nbx * B.nby * B.nbz : *B.count;
+  unsigned* mask = reinterpret_cast<unsigned*>(g.fmask);
+  int fluid = 0, odd = 0;
   for (int it = blockIdx.x * 4; it < n; it += gridDim.x * 4) {
     const int e = it + (threadIdx.x >> 6);
-    if (e >= n) continue;
-    const int b = B.list[e], c = threadIdx.x & 63;
+    if (e >= n) continue;                              // uniform over the warp
+    const int b = allBricks ? e : B.list[e], c = threadIdx.x & 63;
     int bx, by, bz;
     brick_coords(B, b, bx, by, bz);
     const int i = bx * 4 + (c & 3), j = by * 4 + ((c >> 2) & 3), k = bz * 4 + (c >> 4);
-    if (i >= d.nx || j >= d.ny || k >= d.nz) continue;
-    int col;
-    if (cell_pressure_setup(d, g, diag8, omega, ((long long)k * d.ny + j) * d.nx + i, i, j, k, col)) fluid++;
+    int col = -1;
+    if (i < d.nx && j < d.ny && k < d.nz &&
+        cell_pressure_setup(d, g, diag8, omega, ((long long)k * d.ny + j) * d.nx + i, i, j, k, col)) {
+      fluid++;
+      odd |= col < 0;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, col >= 0);
+    if ((threadIdx.x & 31) == 0) mask[2 * b + (c >> 5)] = m;
   }
   fluid = warp_sum(fluid);
   if ((threadIdx.x & 31) == 0 && fluid) atomicAdd(&st->nFluid, fluid);
+  if (odd) atomicOr(&st->oddFluid, 1);
+  if (blockIdx.x == 0 && threadIdx.x == 0) st->sorOmega = omega;
 }
-void launch_pressure_setup_bricks(const Dims& d, const GridDev& g, uint8_t* diag8, double omega, DevStatus* st,
-                                  const BrickSet& B, cudaStream_t s) {
-  k_pressure_setup_bricks<<<brick_grid(B), 256, 0, s>>>(d, g, diag8, omega, st, B);
+void launch_pressure_setup(const Dims& d, const GridDev& g, uint8_t* diag8, double omega, DevStatus* st,
+                           const BrickSet& B, bool allBricks, cudaStream_t s) {
+  k_pressure_setup<<<brick_grid(B), 256, 0, s>>>(d, g, diag8, omega, st, B, allBricks ? 1 : 0);
 }
 
 // ------------------------------------------------------------ field helpers

@@ -129,7 +129,9 @@ struct DevStatus {
   double rr, bb;
   unsigned long long evIrr;   // evaporation pass: (ejection << 32 | candidate) of the first irregular kick
   int evNEj, evNC, evKeff;    // ejections in the pass, candidates, tabulated band width
-  unsigned int evSEnd, evSStart, pad3;   // stream after the pass; start state of a restarted pass
+  unsigned int evSEnd, evSStart;   // stream after the pass; start state of a restarted pass
+  int oddFluid;            // the pressure setup met a fluid cell on the domain's outermost layer (zeroed by the raster)
+  double sorOmega;         // omega of the last pressure setup (pw = omega / diag)
 };
 
 struct GridDev {
@@ -146,6 +148,7 @@ struct GridDev {
   const float* sv;          // solid velocity (3 x nCells: x, y, z) of moving solids, or null
   uint8_t* seed;            // 4^3 bricks holding a particle or a moving solid this substep (or null)
   int nbx, nby;             // bricks per axis (x, y) of the seed map
+  unsigned long long* fmask;   // per 4^3 brick: its interior fluid cells (bit 16 z + 4 y + x), written by the pressure setup
 };
 // The 4^3-brick work list of the substep's face and cell passes (ws_grid.cu)
 struct BrickSet {
@@ -157,6 +160,7 @@ struct BrickSet {
   int* count;
   int* forceAll;            // device flag: process every brick once
   FastDiv dnbx, dnby;       // division by nbx and nby (brick coordinates of a linear brick index)
+  unsigned long long* fmask;   // per brick: its interior fluid cells as of the last pressure setup
 };
 // (bx, by, bz) of linear brick b = (bz * nby + by) * nbx + bx
 __device__ __forceinline__ void brick_coords(const BrickSet& B, int b, int& bx, int& by, int& bz) {

@@ -34,8 +34,6 @@ void launch_faces_forces_bricks(const Dims& d, const GridDev& g, const BrickSet&
 void launch_project_bricks(const Dims& d, const GridDev& g, const BrickSet& B, int doClamp, double maxSpeed,
                            DevStatus* st, cudaStream_t s);
 void launch_extrapolate_bricks(const Dims& d, const GridDev& g, const BrickSet& B, cudaStream_t s);
-void launch_pressure_setup_bricks(const Dims& d, const GridDev& g, uint8_t* diag8, double omega, DevStatus* st,
-                                  const BrickSet& B, cudaStream_t s);
 // cs: count every particle P2G will scatter in its cell (null: mark only)
 void launch_mark_fluid(const Dims& d, const GridDev& g, const PartsDev& P, const TerrainDev& t,
                        double oceanR, double coreR, const CellSort* cs, DevStatus* st, cudaStream_t s);
@@ -45,8 +43,9 @@ int launch_p2g_sorted(const Dims& d, const GridDev& g, const PartsDev& P, const 
                       bool binned, void* scratch, size_t scratchBytes, DevStatus* st, cudaStream_t s);
 void launch_faces_normalize_bc(const Dims& d, const GridDev& g, cudaStream_t s);
 void launch_faces_forces(const Dims& d, const GridDev& g, double coef, int viscOn, double dt, double gs, cudaStream_t s);
-void launch_pressure_setup(const Dims& d, const GridDev& g, uint8_t* diag8, double omega, DevStatus* st, int* sorCounts,
-                           cudaStream_t s);
+// over the brick list, or every brick of the grid (allBricks)
+void launch_pressure_setup(const Dims& d, const GridDev& g, uint8_t* diag8, double omega, DevStatus* st,
+                           const BrickSet& B, bool allBricks, cudaStream_t s);
 void launch_sor_color(const Dims& d, const GridDev& g, int color, double om1, cudaStream_t s);
 int residual_blocks(const Dims& d);
 void launch_residual(const Dims& d, const GridDev& g, const uint8_t* diag8, double2* partials,
@@ -127,27 +126,19 @@ void launch_terrain_radius(const TerrainDev& t, double coreR, const double* xyz,
 void launch_ocean_point(const Dims& d, const TerrainDev& t, double coreR, double oceanR, double need, uint32_t s0,
                         double* out, cudaStream_t s);
 
-// ---- ws_sor.cu (colour lists) and ws_sor_tb.cu (temporal blocking on every SM)
+// ---- ws_sor_tb.cu (regions in shared memory on every SM) and ws_sor.cu (colour lists)
 cudaError_t sor_init(void** statePtr, const Dims& d, int device);
 void sor_free(void* statePtr);
-// the colour lists the list paths need (nothing when the temporal-blocked
-// solve is the default: it builds its own plan)
-cudaError_t launch_sor_lists(void* state, const Dims& d, const GridDev& g, const uint8_t* diag8, cudaStream_t s);
-cudaError_t launch_sor_run(void* state, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                           int iters, int check, double tol, int* err, int** outIters, double** outRel, int** outPath,
-                           cudaStream_t s);
+// the whole solve of the last pressure setup's system; iterations, residual
+// and path land in device memory
 cudaError_t launch_sor_solve(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                             int iters, int check, double tol, int* err, int** outIters, double** outRel,
+                             int iters, int check, double tol, DevStatus* st, int** outIters, double** outRel,
                              int** outPath, cudaStream_t s);
 cudaError_t launch_sor_solve_lists(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                                   int iters, int check, double tol, int* err, int** outIters, double** outRel,
+                                   int iters, int check, double tol, DevStatus* st, int** outIters, double** outRel,
                                    int** outPath, cudaStream_t s);
-// per-256-cell-block colour counts the pressure setup fills for the list build
-int* sor_block_counts(void* state);
 int sor_solve_launches(void* state);
 int sor_list_solve_launches(void* state);
-// whether the default solve is the temporal-blocked one (it needs no per-block colour counts)
-bool sor_uses_tb(void* state);
 
 // ---- ws_contacts.cu
 void launch_vapor_collisions(const Dims& d, const PartsDev& P, double spacing, double oceanR, int spinOn,

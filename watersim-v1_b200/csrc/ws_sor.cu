@@ -49,14 +49,26 @@ __device__ __forceinline__ int sor_colour(const Dims& d, const float* __restrict
   if (i < 1 || j < 1 || k < 1 || i + 2 > nx || j + 2 > ny || (int)k + 2 > d.nz) return -1;
   return (int)((i + j + k) & 1u);
 }
+// interior fluid cells per colour of each 256-cell chunk. Like the other list
+// kernels it leaves at once when the region solve before it solved the system
+// (solved null: always runs).
+__global__ void __launch_bounds__(256) k_sor_count(Dims d, const float* __restrict__ pw, int* __restrict__ blockCounts,
+                                                   int nChunks, const int* __restrict__ solved) {
+  if (solved && *solved) return;
+  for (int b = blockIdx.x; b < nChunks; b += gridDim.x) {
+    const int col = sor_colour(d, pw, (unsigned)b * 256u + threadIdx.x);
+    const int n0 = __syncthreads_count(col == 0), n1 = __syncthreads_count(col == 1);
+    if (threadIdx.x == 0) { blockCounts[2 * b] = n0; blockCounts[2 * b + 1] = n1; }
+  }
+}
 // exclusive scan of the (colour 0, colour 1) block counts into offs, one
 // block of 32 warps: each warp owns a contiguous segment and reads it 32 pairs
 // at a time (coalesced); pass 1 sums the segments, the block scans the 32
 // sums, pass 2 rescans each segment from its carry and writes the offsets.
-// total = the two list lengths. The counts stay as the pressure setup wrote
-// them, so the solve can be repeated on the same system.
+// total = the two list lengths.
 __global__ void __launch_bounds__(1024) k_sor_scan(const int* __restrict__ blockCounts, int nb, int* __restrict__ offs,
-                                                   int* __restrict__ total) {
+                                                   int* __restrict__ total, const int* __restrict__ solved) {
+  if (solved && *solved) return;
   __shared__ int w0[32], w1[32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int2* cnt = reinterpret_cast<const int2*>(blockCounts);
@@ -90,13 +102,14 @@ __global__ void __launch_bounds__(1024) k_sor_scan(const int* __restrict__ block
   }
   if (threadIdx.x == 0) { total[0] = w0[nw - 1]; total[1] = w1[nw - 1]; }
 }
-// Persistent over the 256-cell chunks the pressure setup counted (chunk b
+// Persistent over the 256-cell chunks k_sor_count counted (chunk b
 // holds cells 256 b .. 256 b + 255 and its list offsets are offs[2 b], offs[2 b
 // + 1]); the next chunk's colours and offsets are fetched before this chunk's
 // ranks are formed. Warp totals are double-buffered: one barrier per chunk.
 __global__ void __launch_bounds__(256) k_sor_scatter(Dims d, const float* __restrict__ pw, const float* __restrict__ rhs,
                                                      const uint8_t* __restrict__ diag8, const int* __restrict__ offs,
-                                                     SorLists L, int nChunks) {
+                                                     SorLists L, int nChunks, const int* __restrict__ solved) {
+  if (solved && *solved) return;
   __shared__ int wt[2][2][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int b = blockIdx.x;
@@ -202,6 +215,7 @@ struct SorArgs {
   int clusterCap;      // lists up to this size per colour were solved by k_sor_cluster
   const int* offs;     // per 256-cell chunk b: its first list entry of colour 0 and 1 (offs[2 b], offs[2 b + 1])
   int nChunks;
+  const int* solved;   // the region solve's flag (null: none ran)
 };
 
 // One colour's half-sweep over the lists in global memory, three cells per
@@ -425,6 +439,7 @@ __device__ __forceinline__ void persistent_loop(const SorArgs& a, unsigned tid, 
   if (blockIdx.x == 0 && threadIdx.x == 0) { *a.outIters = it; *a.outRel = rel; *a.outPath = 1; }
 }
 __global__ void __launch_bounds__(1024, 1) k_sor_persistent(SorArgs a) {
+  if (a.solved && *a.solved) return;
   const unsigned T = gridDim.x * blockDim.x;
   const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int n0 = a.L.count[0], n1 = a.L.count[1];
@@ -595,7 +610,7 @@ static size_t cluster_smem_bytes() { return (size_t)(kSmax + 1) * 2 * 4 + (size_
 // ---------------------------------------------------------------- host side
 struct SorState {
   SorLists L{};
-  int* blockCounts = nullptr;  // per 256-cell block: interior fluid cells of colour 0, 1 (pressure setup)
+  int* blockCounts = nullptr;  // per 256-cell block: interior fluid cells of colour 0, 1
   int* blockOffs = nullptr;    // their exclusive scan: each block's first list slot per colour
   GridBar* bar = nullptr;
   double2* partials = nullptr;
@@ -605,17 +620,19 @@ struct SorState {
   int grid = 0, block = 1024;
   long long cap = 0;
   int clusterSize = 0;       // 0: cluster path unavailable on this device
-  void* tb = nullptr;        // temporal-blocked solve (ws_sor_tb.cu); null: the colour-list paths
+  void* tb = nullptr;        // region solve (ws_sor_tb.cu); null: the colour-list paths
+  bool big = false;          // grid above kTbMaxCells: a system whose regions do not fit goes to the lists
 };
 
-// the temporal-blocked solve (ws_sor_tb.cu)
+// the region solve (ws_sor_tb.cu)
 cudaError_t sor_tb_init(void** statePtr, const Dims& d, int device);
 void sor_tb_free(void* statePtr);
+const int* sor_tb_solved(void* statePtr);
 cudaError_t launch_sor_tb(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                          int iters, int check, double tol, int* err, int* outIters, double* outRel, int* outPath,
-                          cudaStream_t s);
-// grids up to this many cells solve on every SM with temporal blocking (at
-// 128^3 every region fits in shared memory); larger ones on the colour lists
+                          int iters, int check, double tol, DevStatus* st, bool listFallback, int* outIters,
+                          double* outRel, int* outPath, cudaStream_t s);
+// grids up to this many cells sweep a system whose regions do not fit shared
+// memory from the region kernel itself; larger ones on the colour lists
 static const long long kTbMaxCells = 160LL * 160 * 160;
 
 cudaError_t sor_init(void** statePtr, const Dims& d, int device) {
@@ -623,7 +640,13 @@ cudaError_t sor_init(void** statePtr, const Dims& d, int device) {
   *statePtr = S;
   const long long nCells = d.nCells;
   cudaError_t e;
-  if (nCells <= kTbMaxCells && (e = sor_tb_init(&S->tb, d, device)) != cudaSuccess) return e;
+  S->big = nCells > kTbMaxCells;
+  if ((e = sor_tb_init(&S->tb, d, device)) != cudaSuccess) {
+    if (!S->big) return e;
+    cudaGetLastError();                                 // a large grid does without the exchange buffers
+    sor_tb_free(S->tb);
+    S->tb = nullptr;
+  }
   int smCount = 0, perSM = 0;
   cudaDeviceGetAttribute(&smCount, cudaDevAttrMultiProcessorCount, device);
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_sor_persistent, S->block, 0)) != cudaSuccess) return e;
@@ -660,8 +683,6 @@ cudaError_t sor_init(void** statePtr, const Dims& d, int device) {
   }
   cudaGetLastError();                                   // a refused probe is not an error
   if ((e = cudaMalloc(&S->blockCounts, sizeof(int) * 2 * nb)) != cudaSuccess) return e;
-  // zero until the first pressure setup fills them: a solve before it lists no cell
-  if ((e = cudaMemset(S->blockCounts, 0, sizeof(int) * 2 * nb)) != cudaSuccess) return e;
   if ((e = cudaMalloc(&S->blockOffs, sizeof(int) * 2 * nb)) != cudaSuccess) return e;
   if ((e = cudaMalloc(&S->bar, sizeof(GridBar))) != cudaSuccess) return e;
   if ((e = cudaMemset(S->bar, 0, sizeof(GridBar))) != cudaSuccess) return e;
@@ -672,15 +693,15 @@ cudaError_t sor_init(void** statePtr, const Dims& d, int device) {
   return cudaSuccess;
 }
 
-int* sor_block_counts(void* statePtr) { return statePtr ? ((SorState*)statePtr)->blockCounts : nullptr; }
-// kernels one launch_sor_solve issues: scan, scatter, [codes, cluster solve,] grid solve
+// kernels one launch_sor_solve issues: the region solve [and, above
+// kTbMaxCells, count, scan, scatter, grid solve, which leave at once when it
+// solved the system]; or count, scan, scatter, [codes, cluster solve,] grid solve
+int sor_list_solve_launches(void* statePtr) { return statePtr && ((SorState*)statePtr)->clusterSize ? 6 : 4; }
 int sor_solve_launches(void* statePtr) {
   SorState* S = (SorState*)statePtr;
-  if (S && S->tb) return 1;
-  return S && S->clusterSize ? 5 : 3;
+  if (S && S->tb) return S->big ? 5 : 1;
+  return sor_list_solve_launches(statePtr);
 }
-bool sor_uses_tb(void* statePtr) { return statePtr && ((SorState*)statePtr)->tb; }
-int sor_list_solve_launches(void* statePtr) { return statePtr && ((SorState*)statePtr)->clusterSize ? 5 : 3; }
 void sor_free(void* statePtr) {
   SorState* S = (SorState*)statePtr;
   if (!S) return;
@@ -692,48 +713,26 @@ void sor_free(void* statePtr) {
   delete S;
 }
 
-// Builds the colour lists from the pressure setup (pw, rhs, diag8) and runs
-// the whole solve. Results land in device memory (iterations, residual);
-// the caller reads them with its next status synchronisation.
-// The colour lists (scan of the setup's block counts, scatter, neighbour
-// codes) and the barrier reset. They read the pressure setup's rhs, pw and
-// stencil bytes, never q, so they may run beside anything that only writes q
-// (the learned warm start).
-static cudaError_t build_lists(SorState* S, const Dims& d, const GridDev& g, const uint8_t* diag8, cudaStream_t s);
-cudaError_t launch_sor_lists(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, cudaStream_t s) {
-  SorState* S = (SorState*)statePtr;
-  if (S->tb) return cudaSuccess;          // the temporal-blocked solve builds its own plan
-  return build_lists(S, d, g, diag8, s);
-}
-static cudaError_t build_lists(SorState* S, const Dims& d, const GridDev& g, const uint8_t* diag8, cudaStream_t s) {
-  // the per-block colour counts come from the pressure setup (k_pressure_setup)
-  int nb = (int)grid_for(d.nCells, 256);
-  k_sor_scan<<<1, 1024, 0, s>>>(S->blockCounts, nb, S->blockOffs, S->L.count);
-  k_sor_scatter<<<std::min(nb, 148 * 8), 256, 0, s>>>(d, g.pw, g.rhs, diag8, S->blockOffs, S->L, nb);
+// The colour lists of the pressure setup's pw, rhs and diag8 (counts, scan,
+// scatter, neighbour codes of the cluster solve) and the barrier reset.
+static cudaError_t build_lists(SorState* S, const Dims& d, const GridDev& g, const uint8_t* diag8, bool cluster,
+                               const int* solved, cudaStream_t s) {
+  const int nb = (int)grid_for(d.nCells, 256), grid = std::min(nb, 148 * 8);
+  k_sor_count<<<grid, 256, 0, s>>>(d, g.pw, S->blockCounts, nb, solved);
+  k_sor_scan<<<1, 1024, 0, s>>>(S->blockCounts, nb, S->blockOffs, S->L.count, solved);
+  k_sor_scatter<<<grid, 256, 0, s>>>(d, g.pw, g.rhs, diag8, S->blockOffs, S->L, nb, solved);
   cudaMemsetAsync(S->bar, 0, sizeof(GridBar), s);     // a solve that timed out leaves no stale arrivals
-  if (S->clusterSize)
+  if (cluster)
     k_sor_codes<<<dim3((unsigned)std::min<long long>(grid_for(6 * S->cap, 256), 148 * 8), 2), 256, 0, s>>>(d, g.pw,
                                                                                                       S->L, S->clusterSize);
   return cudaGetLastError();
 }
-// The solve on the lists of launch_sor_lists: cluster-resident when they fit
-// one cluster, else the grid-wide persistent kernel (each returns at once when
+// The solve on the lists: with `cluster` cluster-resident when they fit one
+// cluster, else the grid-wide persistent kernel (each returns at once when
 // the other path applies).
 static cudaError_t run_lists(SorState* S, const Dims& d, const GridDev& g, double omega, int iters, int check,
-                             double tol, int* err, int** outIters, double** outRel, int** outPath, cudaStream_t s);
-cudaError_t launch_sor_run(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                           int iters, int check, double tol, int* err, int** outIters, double** outRel, int** outPath,
-                           cudaStream_t s) {
-  SorState* S = (SorState*)statePtr;
-  *outPath = S->outPath; *outIters = S->outIters; *outRel = S->outRel;
-  if (S->tb)
-    return launch_sor_tb(S->tb, d, g, diag8, omega, iters, check, tol, err, S->outIters, S->outRel, S->outPath, s);
-  return run_lists(S, d, g, omega, iters, check, tol, err, outIters, outRel, outPath, s);
-}
-static cudaError_t run_lists(SorState* S, const Dims& d, const GridDev& g, double omega, int iters, int check,
-                             double tol, int* err, int** outIters, double** outRel, int** outPath, cudaStream_t s) {
-  *outPath = S->outPath;
-  int C = S->clusterSize;
+                             double tol, int* err, bool cluster, const int* solved, cudaStream_t s) {
+  const int C = cluster ? S->clusterSize : 0;
   if (C) {
     ClusterArgs ca;
     ca.d = d; ca.q = g.q; ca.L = S->L; ca.om1 = 1 - omega; ca.iters = iters; ca.check = check; ca.tol = tol;
@@ -753,25 +752,35 @@ static cudaError_t run_lists(SorState* S, const Dims& d, const GridDev& g, doubl
   a.outPath = S->outPath;
   a.clusterCap = C ? C * kSmax : -1;
   a.offs = S->blockOffs; a.nChunks = (int)grid_for(d.nCells, 256);
+  a.solved = solved;
   void* args[] = { &a };
-  cudaError_t e = cudaLaunchCooperativeKernel((void*)k_sor_persistent, dim3(S->grid), dim3(S->block), args, 0, s);
-  *outIters = S->outIters; *outRel = S->outRel;
-  return e;
+  return cudaLaunchCooperativeKernel((void*)k_sor_persistent, dim3(S->grid), dim3(S->block), args, 0, s);
 }
+// The default solve: the regions in shared memory; where the state says the
+// device or grid cannot hold them, the lists. Above kTbMaxCells the list
+// kernels follow and leave at once when the regions fitted: four launches of
+// about 1.5 us against a list solve of 15-20 us an iteration where they did not.
 cudaError_t launch_sor_solve(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                             int iters, int check, double tol, int* err, int** outIters, double** outRel,
+                             int iters, int check, double tol, DevStatus* st, int** outIters, double** outRel,
                              int** outPath, cudaStream_t s) {
-  cudaError_t e = launch_sor_lists(statePtr, d, g, diag8, s);
-  if (e != cudaSuccess) return e;
-  return launch_sor_run(statePtr, d, g, diag8, omega, iters, check, tol, err, outIters, outRel, outPath, s);
+  SorState* S = (SorState*)statePtr;
+  if (!S->tb) return launch_sor_solve_lists(statePtr, d, g, diag8, omega, iters, check, tol, st, outIters, outRel, outPath, s);
+  *outPath = S->outPath; *outIters = S->outIters; *outRel = S->outRel;
+  cudaError_t e = launch_sor_tb(S->tb, d, g, diag8, omega, iters, check, tol, st, S->big, S->outIters, S->outRel,
+                                S->outPath, s);
+  if (e != cudaSuccess || !S->big) return e;
+  const int* solved = sor_tb_solved(S->tb);
+  if ((e = build_lists(S, d, g, diag8, false, solved, s)) != cudaSuccess) return e;
+  return run_lists(S, d, g, omega, iters, check, tol, &st->err, false, solved, s);
 }
 // the same solve on the colour lists (cluster-resident or grid-wide), whatever
 // the default path; for comparisons of the two paths
 cudaError_t launch_sor_solve_lists(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                                   int iters, int check, double tol, int* err, int** outIters, double** outRel,
+                                   int iters, int check, double tol, DevStatus* st, int** outIters, double** outRel,
                                    int** outPath, cudaStream_t s) {
   SorState* S = (SorState*)statePtr;
-  cudaError_t e = build_lists(S, d, g, diag8, s);
+  *outPath = S->outPath; *outIters = S->outIters; *outRel = S->outRel;
+  cudaError_t e = build_lists(S, d, g, diag8, S->clusterSize > 0, nullptr, s);
   if (e != cudaSuccess) return e;
-  return run_lists(S, d, g, omega, iters, check, tol, err, outIters, outRel, outPath, s);
+  return run_lists(S, d, g, omega, iters, check, tol, &st->err, true, nullptr, s);
 }

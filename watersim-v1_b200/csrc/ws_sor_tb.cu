@@ -1,37 +1,57 @@
 // ws_sor_tb.cu — the pressure solve of _pressureSolve (js/solver.js:1368-1404)
-// on every SM at once: red-black SOR with temporal blocking.
+// on every SM at once: red-black SOR over shared-memory regions.
 //
-// Partition. The grid is cut into 4x4x4-cell bricks. Bricks holding a fluid
-// cell are taken in Morton order and split into one contiguous chunk per CTA
-// with equal shares of weight (interior fluid cells plus kBrickWeight per
-// brick), so each CTA owns a compact patch of the ocean shell (about 700
-// cells at 128^3).
+// Partition. The grid is cut into 4x4x4-cell bricks; the pressure setup
+// leaves one 64-bit mask of interior fluid cells per brick. Bricks holding a
+// fluid cell are taken in Morton order and split into one contiguous chunk
+// per CTA with equal shares of weight (fluid cells plus kBrickWeight per
+// brick), so each CTA owns a compact patch of the ocean shell.
 //
-// Region. A CTA keeps in shared memory its owned bricks plus every active
-// brick among their 26 neighbours, densely (64 q values per brick). The
-// interior fluid cells of the region are labelled with d, their L1 distance
-// in cells to the boxes of the owned bricks (d = 0 owned). d changes by at
-// most one between neighbouring cells, and a red-black half-sweep only
-// propagates information one cell, so after loading exact values for d <= 4,
-// the CTA can run four half-sweeps (two iterations) on its own: half-sweep t
-// updates the cells with d <= 4 - t, and after the fourth the owned cells
-// hold exactly the values of the global sweep. Each cell's update reads the same six neighbours in
-// the same order with the same arithmetic as the reference's sweep, so the
-// iterates are bitwise those of the plain red-black solve.
+// Region. A CTA works on the fluid cells of its owned bricks (d = 0) and on
+// those of the surrounding bricks by their L1 distance d in cells to the
+// owned bricks' boxes. d changes by at most one between neighbouring cells
+// and a red-black half-sweep moves information one cell, so after loading
+// exact values for d <= H the CTA can run H half-sweeps (H / 2 iterations) on
+// its own: half-sweep t updates the cells with d <= H - t, and after the last
+// one the owned cells hold exactly the values of the global sweep. Each
+// update reads the same six neighbours in the same order with the same
+// arithmetic as the reference's sweep (sor_update), so the iterates are
+// bitwise those of the plain red-black solve. H is 4 where every CTA's region
+// fits shared memory with it, else 2: a larger H halves the exchanges, and
+// costs the cells of two more layers.
 //
-// Exchange. After each such epoch e a CTA writes its owned cells into one of
-// two global exchange buffers (e & 1) as 64-bit words (q's bits | e << 32),
-// one single-copy-atomic relaxed store per cell and no fence or flag; before
-// the next epoch every thread loads its halo cells from that buffer and
-// polls a word again until its tag reads e. The tag travels in the same word
-// as the value, so a matching tag proves the value, and a CTA waits only for
-// the values it needs. Double buffering makes the write of epoch e + 2 safe
-// against neighbours still reading epoch e: a CTA computes epoch e + 2 only
-// after reading its neighbours' epoch e + 1 values, which each neighbour
-// wrote after it had read this CTA's epoch e values (halo adjacency is
-// symmetric). The plan phase clears the tags of every owned cell in both
-// buffers before the first epoch, so stale words of an earlier solve never
-// match.
+// Storage. Only fluid cells are stored, colour by colour and by d inside a
+// colour (colour 0 d = 0 .. H - 1, then colour 1 d = 0 .. H): a half-sweep
+// updates a prefix of its colour, an update entry's own q has the entry's
+// index, and neighbours of neighbouring entries sit mostly in neighbouring
+// banks. A cell's index is its brick's base in its (colour, d) class plus the
+// set bits below it in the class mask. An entry is one 16-byte record (the
+// byte offsets of its six neighbours, 16 bits each, the right-hand side, and
+// the stencil count in the offsets' unused low bits; omega / count comes from a
+// table), a cell 4 bytes: about 10,000 entries fit one SM, 1.3M fluid cells of
+// a thin ocean the chip. (Before, q was dense over the region's bricks with 24
+// bytes an entry; that held 4096 entries, and grids above 160^3 read lists
+// from L2 in every half-sweep.)
+//
+// Exchange. After each epoch of H half-sweeps a CTA writes the owned cells
+// that some other CTA's halo holds into its own packed list (two of them, by
+// epoch parity) as 64-bit words (q's bits | tag << 32), one single-copy-atomic
+// relaxed store per cell and no fence or flag; before the next epoch every
+// thread loads its halo words and polls a word again until its tag is the
+// epoch's. The tag travels in the same word as the value, so a matching tag
+// proves the value, and a CTA waits only for the values it needs. The lists
+// are in brick order on both sides, so a warp's words share sectors: words
+// scattered over a grid-sized array took half of the solve in L2 traffic and
+// polls. Double buffering makes the write of epoch e + 2 safe against
+// neighbours still reading epoch e: a CTA computes epoch e + 2 only after
+// reading its neighbours' epoch e + 1 values, which each neighbour wrote
+// after it had read this CTA's epoch e values (halo adjacency is symmetric).
+// Tags count on from solve to solve (tagBase), so a word left by an earlier
+// solve never matches and nothing has to be cleared.
+//
+// Overlap. Colour 0's owned cells are stored with those first that touch no
+// foreign brick: their part of an epoch's first half-sweep reads no halo, so
+// it runs between the publication and the wait.
 //
 // Residual check. Every sorCheckEvery iterations (epochs end on check
 // iterations) the FP64 partial ||b - A q||^2 and ||b||^2 of the owned cells
@@ -40,11 +60,15 @@
 // between two buffers so a CTA running ahead cannot overwrite one that a
 // slower CTA still sums.
 //
-// The plan (brick counts, Morton scan, chunks, regions) is built inside the
-// same cooperative launch, separated by three grid barriers. When a region
-// does not fit in shared memory, every CTA takes the same fallback: the
-// red-black sweep over its owned bricks in global memory with a grid barrier
-// per half-sweep (same arithmetic, same iterates).
+// The plan (brick weights, Morton scan, chunks, regions) is built inside the
+// same cooperative launch, separated by three grid barriers. When some
+// region does not fit even with H = 2, or a fluid cell lies on the domain's
+// outermost layer (only by a caller's upload), every CTA leaves the solve to
+// a fallback: grids up to 160^3 sweep the owned bricks in global memory with
+// a grid barrier per half-sweep, larger ones leave the solved flag clear for
+// the list kernels that follow (ws_sor.cu). Same arithmetic, same iterates.
+//
+// What bounds it and what it measured stands at k_sor_tb.
 //
 // Every wait is bounded: after kTbSpinLimit polls the CTA latches
 // WS_DERR_TIMEOUT, stops, and the waits of the others run out in turn. The
@@ -52,18 +76,22 @@
 // run never reaches the limit.
 #include "ws_kernels.cuh"
 #include <algorithm>
+#include <cstddef>
 
 namespace {
 
+typedef unsigned long long u64;
+
 constexpr int kTbThreads = 1024;
-constexpr int kRbMax = 256;                 // region bricks per CTA
-constexpr int kEMax = 4096;                 // update entries (d <= 3) per CTA
-constexpr int kLMax = 4096;                 // halo reload cells (1 <= d <= 4) per CTA
-constexpr int kOMax = 2048;                 // owned interior fluid cells per CTA
-constexpr int kHashSlots = 1024;            // open-addressing table of region bricks
-constexpr int kZero = kRbMax * 64;          // dense index of the always-zero cell
+constexpr int kRbMax = 896;                 // region bricks per CTA
+constexpr int kHMax = 4;                    // half-sweeps per epoch where the regions fit
+constexpr int kHashSlots = 2048;            // open-addressing table of region bricks
+constexpr int kQMax = 16384;                // stored cells per CTA (the neighbour indices hold 16 bits)
+constexpr int kPubMax = 8192;               // published cells per CTA
+constexpr int kFetchMax = 8192;             // halo cells per CTA
 constexpr long long kTbSpinLimit = 4000000LL;
 constexpr int kMaxCtas = 1024;
+constexpr int kTbSmem = 229376;             // dynamic shared memory: the 227 KB of a block less the static part
 // Chunk weight of an active brick: its interior fluid cells plus this much.
 // Equal shares of fluid alone gave CTAs 13-55 owned bricks at 128^3 (bricks
 // at the shell's edges hold few fluid cells), and the CTA with the most
@@ -71,32 +99,39 @@ constexpr int kMaxCtas = 1024;
 // of the plan; the per-brick term evens out the brick counts too.
 constexpr int kBrickWeight = 16;
 
-// device control block, zeroed before every solve
+// device control block; all but tagBase zeroed before every solve
 struct TbCtl {
-  unsigned barCount, barGen;     // grid barrier
+  unsigned barCount;             // arrivals at the grid barriers of this solve
   unsigned resCount;             // residual partials published so far (all checks)
-  int overflow;                  // some region did not fit: every CTA takes the fallback
-  int pad[12];
+  int over4, over2;              // some region does not fit with H = 4, with H = 2
+  int solved;                    // 1: this launch solved the system (the list kernels leave at once)
+  int pad[11];
+  unsigned tagBase;              // exchange tags of this solve start after it
 };
 
 struct TbArgs {
   Dims d;
-  float* q;                      // the solve's q (epochs 0, 2, 4, ... end here)
-  unsigned long long* xq;        // exchange: two buffers of nCells words (q bits | epoch << 32)
+  float* q;
+  u64* xq;                       // exchange: per CTA two lists of kPubMax words (q bits | tag << 32)
+  unsigned* xmap;                // [2][nCells]: place of a published cell (owner * 2 * kPubMax + position), H = 2 and 4
   const float* rhs;
   const float* pw;               // omega/diag, negative off the fluid
   const uint8_t* diag8;
+  const u64* fmask;              // per linear brick: its interior fluid cells (bit 16 z + 4 y + x)
+  const DevStatus* st;           // the setup's omega and odd-fluid flag
   int nbx, nby, nbz, mbits;      // bricks per axis; Morton cube side 2^mbits
-  int* brickW;                   // per Morton code: chunk weight (interior fluid + kBrickWeight) | any-fluid << 8
-  int2* cntPart;                 // per CTA: (active bricks, interior fluid cells) of its Morton chunk
+  int2* cntPart;                 // per CTA: (active bricks, chunk weight) of its Morton chunk
   int* actLin;                   // active brick t -> linear brick index
-  int* actWPre;                  // active brick t -> chunk weight before it
-  int* brickOrd;                 // linear brick -> active ordinal, -1 inactive
+  int* wPre;                     // linear (active) brick -> chunk weight before it
   int* chunkStart;               // CTA -> first owned active brick ([P] = number of active bricks)
+  unsigned* glist;               // per CTA: global cell of each owned cell by its stored index (kQMax)
+  unsigned short* dense;         // per CTA: stored index of each region cell (64 kRbMax), where shared memory has no room
+  unsigned short* plist;         // per CTA: stored index of each published cell (kPubMax)
+  uint2* flist;                  // per CTA: (place in xq, stored index) of each halo cell (kFetchMax)
   double2* resPart;              // 2 x P residual partials
   TbCtl* ctl;
   double om1;
-  int iters, check;
+  int iters, check, listFallback;
   double tol;
   int* err;
   int* outIters;
@@ -104,24 +139,47 @@ struct TbArgs {
   int* outPath;
 };
 
-// shared-memory layout (dynamic)
-struct TbSmem {
-  float q[kRbMax * 64 + 4];               // dense region q; [kZero] = 0
-  uint8_t dist[kRbMax * 64];              // 0..4 distance d, 5 farther, 254 constant
+// Plan-time tables in shared memory. The first lie where the solve's values
+// and records go: they are read for the last time when the dense index table
+// is filled. The second lie at the end of the block's shared memory, the dense
+// table before them where it clears both the first tables and the records,
+// else in global memory.
+struct TbPlan {
+  u64 mask[kRbMax];                       // interior fluid cells of each region brick
+  u64 cm[kHMax][kRbMax];                  // halo brick: its cells at d = 1 .. 4; owned brick: [0], [1] its cells to publish
+                                          // with H = 2, 4, [2] its cells with a foreign face neighbour
   int hkey[kHashSlots];
   short hval[kHashSlots];
-  int rbLin[kRbMax];
-  short rbX[kRbMax], rbY[kRbMax], rbZ[kRbMax];   // brick coordinates of each slot
-  short rbOwn[kRbMax];
-  short rbNb[kRbMax][6];
-  unsigned rbOwnMask[kRbMax];             // which of the 27 bricks around a slot (itself included) this CTA owns
-  unsigned short eSelf[kEMax];
-  unsigned eNb[kEMax][3];                 // six neighbour dense indices, two per word
-  float eRhs[kEMax], ePw[kEMax];
-  unsigned short lDense[kLMax];
-  unsigned lGlob[kLMax];
-  unsigned oGlob[kOMax];                  // global index of each owned entry (buckets 0 and 4, in order)
+  unsigned dirs[kRbMax];                  // halo brick: which of the 27 bricks around it this CTA owns; owned: which are foreign
+  // bases of a brick's cells in the lists. Owned: [0] colour 0 without, [4] with
+  // a foreign face neighbour, [1] colour 1, [2], [3] published cells; halo:
+  // [2 (d - 1) + colour], [8], [9] fetched cells with H = 2, 4
+  unsigned short base[2 * kHMax + 2][kRbMax];
 };
+struct TbPlan2 {
+  uchar4 rbXYZ[kRbMax];                   // brick coordinates
+  unsigned short rbNb[6][kRbMax];         // face neighbours' slots (kNone: not in the region)
+};
+constexpr unsigned short kNone = 0xffffu;
+static_assert(sizeof(TbPlan) + sizeof(TbPlan2) <= (size_t)kTbSmem, "plan tables");
+
+// bits of the cells with x + y + z odd
+constexpr u64 kOdd = 0xa5a55a5aa5a55a5aull;
+// cells of a brick within L1 distance d of the box of the brick in direction
+// n27 = (ox + 1) + 3 (oy + 1) + 9 (oz + 1)
+constexpr int axis_dist(int o, int c) { return o < 0 ? c + 1 : o > 0 ? 4 - c : 0; }
+struct NearTable { u64 m[27][kHMax]; };
+constexpr NearTable make_near() {
+  NearTable t{};
+  for (int n = 0; n < 27; n++)
+    for (int c = 0; c < 64; c++) {
+      const int dd = axis_dist(n % 3 - 1, c & 3) + axis_dist((n / 3) % 3 - 1, (c >> 2) & 3) + axis_dist(n / 9 - 1, c >> 4);
+      for (int d = 1; d <= kHMax; d++)
+        if (dd <= d) t.m[n][d - 1] |= 1ull << c;
+    }
+  return t;
+}
+__device__ const NearTable kNear = make_near();
 
 __device__ __forceinline__ unsigned compact1by2(unsigned x) {
   x &= 0x09249249u;
@@ -146,24 +204,18 @@ __device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned l
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
 }
 
-// bounded grid barrier on ctl->barCount/barGen; false when a wait timed out
-__device__ bool tb_grid_barrier(TbCtl* ctl, int* err, int* sAbort) {
+// Bounded grid barrier number n (counted from 1) on the arrivals of this
+// solve: one reduction to arrive and a poll until all have. (An arrival that
+// read the count back and a last CTA that reset it and raised a generation
+// word took three round trips to L2 in a row, about 2 us more.) false when a
+// wait timed out.
+__device__ bool tb_grid_barrier(TbCtl* ctl, unsigned n, int* err, int* sAbort) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    volatile unsigned* vgen = &ctl->barGen;
-    unsigned g = *vgen;
-    __threadfence();
-    if (atomicAdd(&ctl->barCount, 1u) == gridDim.x - 1) {
-      atomicExch(&ctl->barCount, 0u);
-      __threadfence();
-      atomicAdd(&ctl->barGen, 1u);
-    } else {
-      long long n = 0;
-      while (*vgen == g) {
-        if (++n > kTbSpinLimit) { atomicOr(err, WS_DERR_TIMEOUT); *sAbort = 1; break; }
-      }
-    }
-    __threadfence();
+    fence_acq_rel_gpu();
+    atomicAdd(&ctl->barCount, 1u);
+    if (!bounded_wait_geq(&ctl->barCount, n * gridDim.x, kTbSpinLimit, err)) *sAbort = 1;
+    fence_acq_rel_gpu();
     if (*(volatile int*)err & WS_DERR_TIMEOUT) *sAbort = 1;
   }
   __syncthreads();
@@ -180,43 +232,24 @@ __device__ __forceinline__ int owner_of(long long wpre, int P, long long NF) {
 __device__ __forceinline__ bool interior(const Dims& d, int i, int j, int k) {
   return i >= 1 && j >= 1 && k >= 1 && i + 2 <= d.nx && j + 2 <= d.ny && k + 2 <= d.nz;
 }
-
-// dense neighbour (direction 0..5 = -x, +x, -y, +y, -z, +z) of dense cell x
-__device__ __forceinline__ int dense_nb(const TbSmem& S, int x, int dir) {
-  const int s = x >> 6, c = x & 63, cx = c & 3, cy = (c >> 2) & 3, cz = c >> 4;
-  int nbS;
-  switch (dir) {
-    case 0: if (cx > 0) return x - 1; nbS = S.rbNb[s][0]; return nbS < 0 ? kZero : (nbS << 6) | (c + 3);
-    case 1: if (cx < 3) return x + 1; nbS = S.rbNb[s][1]; return nbS < 0 ? kZero : (nbS << 6) | (c - 3);
-    case 2: if (cy > 0) return x - 4; nbS = S.rbNb[s][2]; return nbS < 0 ? kZero : (nbS << 6) | (c + 12);
-    case 3: if (cy < 3) return x + 4; nbS = S.rbNb[s][3]; return nbS < 0 ? kZero : (nbS << 6) | (c - 12);
-    case 4: if (cz > 0) return x - 16; nbS = S.rbNb[s][4]; return nbS < 0 ? kZero : (nbS << 6) | (c + 48);
-    default: if (cz < 3) return x + 16; nbS = S.rbNb[s][5]; return nbS < 0 ? kZero : (nbS << 6) | (c - 48);
-  }
-}
-// global cell index of dense cell x (region brick s holds linear brick rbLin[s]);
-// false outside the domain
-__device__ __forceinline__ bool dense_global(const TbArgs& a, const TbSmem& S, int x, unsigned& g, int& i, int& j,
-                                             int& k) {
-  const int s = x >> 6, c = x & 63;
-  i = S.rbX[s] * 4 + (c & 3); j = S.rbY[s] * 4 + ((c >> 2) & 3); k = S.rbZ[s] * 4 + (c >> 4);
-  if (i >= a.d.nx || j >= a.d.ny || k >= a.d.nz) return false;
-  g = ((unsigned)k * (unsigned)a.d.ny + (unsigned)j) * (unsigned)a.d.nx + (unsigned)i;
-  return true;
+// linear brick of Morton code m, -1 outside the grid
+__device__ __forceinline__ int morton_brick(const TbArgs& a, long long m) {
+  const int bx = (int)compact1by2((unsigned)m), by = (int)compact1by2((unsigned)(m >> 1)), bz = (int)compact1by2((unsigned)(m >> 2));
+  return bx < a.nbx && by < a.nby && bz < a.nbz ? (bz * a.nby + by) * a.nbx + bx : -1;
 }
 
-__device__ __forceinline__ bool hash_insert(TbSmem& S, int key, int* nRegion, int* sOverflow, int fixedSlot,
-                                            short owner, int nbx, int nby) {
-  unsigned h = ((unsigned)key * 2654435761u) >> 22;          // 10 bits
+__device__ __forceinline__ bool hash_insert(TbPlan& S, TbPlan2& S2, int key, u64 mask, int* nRegion, int* sOverflow, int fixedSlot,
+                                            int nbx, int nby) {
+  unsigned h = ((unsigned)key * 2654435761u) >> 21;          // 11 bits
   for (int probe = 0; probe < kHashSlots; probe++, h = (h + 1) & (kHashSlots - 1)) {
     int prev = atomicCAS(&S.hkey[h], -1, key);
     if (prev == -1) {
       int slot = fixedSlot >= 0 ? fixedSlot : atomicAdd(nRegion, 1);
       S.hval[h] = (short)(slot < kRbMax ? slot : -1);
       if (slot < kRbMax) {
-        S.rbLin[slot] = key; S.rbOwn[slot] = owner;
         const int t = key / nbx;
-        S.rbX[slot] = (short)(key - t * nbx); S.rbY[slot] = (short)(t % nby); S.rbZ[slot] = (short)(t / nby);
+        S.mask[slot] = mask; S.dirs[slot] = 0u;
+        S2.rbXYZ[slot] = make_uchar4((unsigned char)(key - t * nbx), (unsigned char)(t % nby), (unsigned char)(t / nby), 0);
       }
       else *sOverflow = 1;
       return true;
@@ -226,8 +259,8 @@ __device__ __forceinline__ bool hash_insert(TbSmem& S, int key, int* nRegion, in
   *sOverflow = 1;
   return false;
 }
-__device__ __forceinline__ int hash_find(const TbSmem& S, int key) {
-  unsigned h = ((unsigned)key * 2654435761u) >> 22;
+__device__ __forceinline__ int hash_find(const TbPlan& S, int key) {
+  unsigned h = ((unsigned)key * 2654435761u) >> 21;
   for (int probe = 0; probe < kHashSlots; probe++, h = (h + 1) & (kHashSlots - 1)) {
     int k = S.hkey[h];
     if (k == key) return S.hval[h];
@@ -235,6 +268,19 @@ __device__ __forceinline__ int hash_find(const TbSmem& S, int key) {
   }
   return -1;
 }
+// slot of the brick (ox, oy, oz) bricks away from slot s, -1 when not in the region
+__device__ __forceinline__ int slot_at(const TbArgs& a, const TbPlan& S, const TbPlan2& S2, int s, int ox, int oy, int oz) {
+  const uchar4 b = S2.rbXYZ[s];
+  const int x = (int)b.x + ox, y = (int)b.y + oy, z = (int)b.z + oz;
+  if (x < 0 || y < 0 || z < 0 || x >= a.nbx || y >= a.nby || z >= a.nbz) return -1;
+  return hash_find(S, (z * a.nby + y) * a.nbx + x);
+}
+__device__ __forceinline__ unsigned cell_global(const TbArgs& a, const TbPlan2& S, int s, int c) {
+  const uchar4 b = S.rbXYZ[s];
+  const unsigned i = b.x * 4u + (c & 3), j = b.y * 4u + ((c >> 2) & 3), k = b.z * 4u + (c >> 4);
+  return (k * (unsigned)a.d.ny + j) * (unsigned)a.d.nx + i;
+}
+__device__ __forceinline__ int bits_below(u64 m, int c) { return __popcll(m & ((1ull << c) - 1ull)); }
 
 // block-wide exclusive scan of two ints (1024 threads); totals returned
 __device__ __forceinline__ int2 block_scan2(int a, int b, int2& total, int2* sw) {
@@ -269,37 +315,6 @@ __device__ __forceinline__ float relax(float qc, float pw, float rhs, const floa
   return sor_update(qc, pw, rhs, v[0], v[1], v[2], v[3], v[4], v[5], om1);
 }
 
-// residual partial of the owned cells (dense order, deterministic) of the
-// state in S.q; block total returned on thread 0
-__device__ double2 owned_residual(const TbArgs& a, const TbSmem& S, int O, double2* sred) {
-  double rr = 0, bb = 0;
-  for (int x = threadIdx.x; x < O * 64; x += blockDim.x) {
-    if (S.dist[x] != 0) continue;
-    unsigned g; int i, j, k;
-    dense_global(a, S, x, g, i, j, k);
-    float v[6];
-#pragma unroll
-    for (int dir = 0; dir < 6; dir++) v[dir] = S.q[dense_nb(S, x, dir)];
-    double sum = (double)v[0];
-    sum += (double)v[1]; sum += (double)v[2]; sum += (double)v[3]; sum += (double)v[4]; sum += (double)v[5];
-    double b = a.rhs[g];
-    double r = b + sum - (double)a.diag8[g] * (double)S.q[x];
-    rr += r * r; bb += b * b;
-  }
-  rr = warp_sum(rr); bb = warp_sum(bb);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sred[wid] = make_double2(rr, bb);
-  __syncthreads();
-  double2 out = make_double2(0, 0);
-  if (wid == 0) {
-    double2 v = lane < (int)(blockDim.x >> 5) ? sred[lane] : make_double2(0, 0);
-    rr = warp_sum(v.x); bb = warp_sum(v.y);
-    out = make_double2(rr, bb);
-  }
-  __syncthreads();
-  return out;
-}
-
 // publish this CTA's partial for check number k, wait for all, sum in a
 // fixed order (lane l adds partials l, l + 32, ..., then a fixed butterfly);
 // every CTA gets the same value. false when the wait timed out.
@@ -327,30 +342,76 @@ __device__ bool global_residual(const TbArgs& a, double2 part, int k, double* sR
   return *(volatile int*)sAbort == 0;
 }
 
-}  // namespace
+// Offsets of the (colour, d) classes for epochs of H half-sweeps: colour 0
+// stores d = 0 .. H - 1 (all of them update entries), colour 1 d = 0 .. H (the
+// entries d <= H - 2 first).
+struct TbLayout {
+  int H, NE, NQ, c1;             // entries, stored cells, first cell of colour 1
+  int off[2][kHMax + 1];         // first cell of a class
+  int n[2][kHMax + 1];           // its cells
+  int nA;                        // colour 0, d = 0: cells without a foreign face neighbour (stored first)
+  int cum[2][kHMax];             // cells of a colour with d <= index
+  int pub, fetch;                // published and fetched cells
+};
+// bytes of the solve's values and records: the cells and the zero cell, then the entries
+__device__ __forceinline__ int record_at(int NQ) { return (4 * (NQ + 1) + 15) & ~15; }
+// whether the solve's values and records fit with epochs of H half-sweeps
+__device__ __forceinline__ bool make_layout(TbLayout& L, int H, int pub, int fetch) {
+  L.H = H; L.pub = pub; L.fetch = fetch;
+  int at = 0;
+  for (int d = 0; d < H; d++) { L.off[0][d] = at; at += L.n[0][d]; }
+  L.c1 = at;
+  for (int d = 0; d <= H; d++) {
+    if (d == H - 1) L.NE = at;
+    L.off[1][d] = at; at += L.n[1][d];
+  }
+  L.NQ = at;
+  for (int c = 0; c < 2; c++) {
+    int sum = 0;
+    for (int d = 0; d < kHMax; d++) { sum += L.n[c][d]; L.cum[c][d] = sum; }
+  }
+  return L.NQ < kQMax && pub <= kPubMax && fetch <= kFetchMax &&
+         record_at(L.NQ) + 16 * L.NE <= (kTbSmem - (int)sizeof(TbPlan2)) / 16 * 16;
+}
 
+}  // namespace
 
 extern __shared__ __align__(16) unsigned char tb_smem_raw[];
 
 // The whole solve in one cooperative launch of one 1024-thread CTA per SM.
+//
+// What bounds it: not bytes (DRAM under 1%), but latency and shared memory.
+// A half-sweep costs about 600 cycles whatever its length (record, gathers,
+// FP64 chain, store, barrier) plus about 28 cycles per 32 entries of an SM
+// (4 wavefronts of the record, six gathers at 1.8 ways, FP64 conversions); an
+// exchange about 1.2 us, partly behind the first half-sweep. 1024 threads with
+// two entries each in flight: 512 with four were a third slower. Measured
+// (fixed-iteration fits, before -> now, us): 32^3 (2.9k fluid cells) plan
+// 32 -> 29, iteration 1.36 -> 1.15; 97^3 (75k) 67 -> 52, 4.05 -> 1.77; 128^3
+// (160k) 65 -> 55, 4.17 -> 2.18; 256^3 (1.09M, lists before) 143 -> 141,
+// 17.6 -> 5.9.
 __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
-  TbSmem& S = *reinterpret_cast<TbSmem*>(tb_smem_raw);
-  __shared__ int sAbort, sOverflow, nRegion, nReload, sT0, sT1, sA;
-  __shared__ int bucket[8], bstart[8], bcur[8];
+  __shared__ int sAbort, sOverflow, nRegion, sT0, sT1, sA;
+  __shared__ TbLayout sL;
+  __shared__ int sCnt[16];
+  __shared__ float sPw[8];
   __shared__ int2 sScan[33];
   __shared__ double2 sRed[32];
   __shared__ double sRel;
   __shared__ long long sNF;
-  const int P = gridDim.x, p = blockIdx.x, tid = threadIdx.x, T = blockDim.x;
-  const int lane = tid & 31;
+  const int P = gridDim.x, p = blockIdx.x, tid = threadIdx.x, T = kTbThreads;
+  const int lane = tid & 31, warp = tid >> 5;
   const Dims& d = a.d;
-  int it = 0, O = 0, R = 0, path = 3;
+  int it = 0, path = a.listFallback ? 1 : 3;
+  unsigned epoch = 0, nBar = 0;
   double rel = -1;
-  if (tid == 0) { sAbort = 0; sOverflow = 0; nRegion = 0; nReload = 0; }
-  if (tid < 8) bucket[tid] = 0;
+  bool solved = false;
+  const unsigned tag0 = *(volatile const unsigned*)&a.ctl->tagBase;
+  if (tid == 0) { sAbort = 0; sOverflow = 0; nRegion = 0; }
+  if (tid < 8) sPw[tid] = tid ? (float)(a.st->sorOmega / (double)tid) : 0.f;   // as the setup rounds pw
   __syncthreads();
 
-  // ---- phase 0: interior fluid cells per brick, Morton order, one chunk of codes per CTA
+  // ---- phase 0: weight of a chunk of Morton codes per CTA
   const long long MC = 1LL << (3 * a.mbits);
   const long long per = (MC + P - 1) / P;
   const long long c0 = std::min(MC, (long long)p * per), c1 = std::min(MC, c0 + per);
@@ -359,55 +420,24 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
   }
   {
     int actSum = 0, wSum = 0;
-    const bool vec = (d.nx & 3) == 0;
-    for (long long base = c0 * 16; base < c1 * 16; base += T) {
-      // 16 consecutive threads share one brick: one row of 4 cells each
-      const long long item = base + tid, m = item >> 4;
-      int w = 0, act = 0;
-      if (m < c1) {
-        const int row = (int)(item & 15);
-        const unsigned bx = compact1by2((unsigned)m), by = compact1by2((unsigned)(m >> 1)),
-                       bz = compact1by2((unsigned)(m >> 2));
-        const int j = (int)by * 4 + (row & 3), k = (int)bz * 4 + (row >> 2), i0 = (int)bx * 4;
-        if ((int)bx < a.nbx && (int)by < a.nby && (int)bz < a.nbz && j < d.ny && k < d.nz) {
-          const long long g = ((long long)k * d.ny + j) * d.nx + i0;
-          float v[4];
-          if (vec) {
-            const float4 f = __ldcg(reinterpret_cast<const float4*>(a.pw + g));
-            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-          } else {
-#pragma unroll
-            for (int c = 0; c < 4; c++) v[c] = i0 + c < d.nx ? __ldcg(a.pw + g + c) : -1.f;
-          }
-#pragma unroll
-          for (int c = 0; c < 4; c++)
-            if (v[c] >= 0.f) { act = 1; if (interior(d, i0 + c, j, k)) w++; }
-        }
-      }
-      // the 16 rows of a brick sit in one half-warp
-      for (int o = 8; o > 0; o >>= 1) {
-        w += __shfl_down_sync(0xffffffffu, w, o, 16);
-        act |= __shfl_down_sync(0xffffffffu, act, o, 16);
-      }
-      if ((tid & 15) == 0 && m < c1) {
-        w += act * kBrickWeight;
-        a.brickW[m] = w | (act << 8);
-        actSum += act; wSum += w;
-      }
+    for (long long m = c0 + tid; m < c1; m += T) {
+      const int lin = morton_brick(a, m);
+      const int cnt = lin >= 0 ? __popcll(__ldcg(a.fmask + lin)) : 0;
+      if (cnt) { actSum++; wSum += cnt + kBrickWeight; }
     }
     actSum = warp_sum(actSum); wSum = warp_sum(wSum);
-    if (lane == 0) sScan[tid >> 5] = make_int2(actSum, wSum);
+    if (lane == 0) sScan[warp] = make_int2(actSum, wSum);
     __syncthreads();
     if (tid < 32) {
-      int2 v = tid < (T >> 5) ? sScan[tid] : make_int2(0, 0);
+      int2 v = sScan[tid];
       v.x = warp_sum(v.x); v.y = warp_sum(v.y);
       if (tid == 0) __stcg(&a.cntPart[p], v);
     }
   }
-  if (!tb_grid_barrier(a.ctl, a.err, &sAbort)) goto done;
+  if (!tb_grid_barrier(a.ctl, ++nBar, a.err, &sAbort)) goto done;
 
-  // ---- phase 1: ordinals and fluid prefixes of this chunk's active bricks,
-  // the dense brick -> ordinal map, and the CTA chunk starts
+  // ---- phase 1: this chunk's active bricks in order, the weight before each,
+  // and the CTA chunk starts
   {
     if (tid < 32) {
       long long bA = 0, bW = 0, tA = 0, tW = 0;
@@ -425,41 +455,33 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
     const long long NF = sNF;
     for (long long m0 = c0; m0 < c1; m0 += T) {
       const long long m = m0 + tid;
-      const int v = m < c1 ? __ldcg(&a.brickW[m]) : 0;
-      const int act = (v >> 8) & 1, w = v & 255;
+      const int lin = m < c1 ? morton_brick(a, m) : -1;
+      const int cnt = lin >= 0 ? __popcll(__ldcg(a.fmask + lin)) : 0;
+      const int act = cnt > 0, w = act ? cnt + kBrickWeight : 0;
       int2 tot;
       const int2 ex = block_scan2(act, w, tot, sScan);
-      if (m < c1) {
-        const unsigned bx = compact1by2((unsigned)m), by = compact1by2((unsigned)(m >> 1)),
-                       bz = compact1by2((unsigned)(m >> 2));
-        if ((int)bx < a.nbx && (int)by < a.nby && (int)bz < a.nbz) {
-          const int lin = ((int)bz * a.nby + (int)by) * a.nbx + (int)bx;
-          if (act) {
-            const int t = baseA + ex.x;
-            const long long wpre = baseW + ex.y;
-            a.actLin[t] = lin; a.actWPre[t] = (int)wpre; a.brickOrd[lin] = t;
-            // the next active brick starts every CTA q whose first fluid cell
-            // (prefix ceil(q NF / P)) lies in (wpre, wpre + w]
-            if (w > 0) {
-              const long long qlo = wpre * P / NF + 1, qhi = std::min((long long)P - 1, (wpre + w) * P / NF);
-              for (long long q = qlo; q <= qhi; q++) a.chunkStart[q] = t + 1;
-            }
-            if (t == A - 1) a.chunkStart[P] = A;
-          } else {
-            a.brickOrd[lin] = -1;
-          }
-        }
+      if (act) {
+        const int t = baseA + ex.x;
+        const long long wpre = baseW + ex.y;
+        a.actLin[t] = lin; a.wPre[lin] = (int)wpre;
+        // the next active brick starts every CTA q whose first unit of weight
+        // (prefix ceil(q NF / P)) lies in (wpre, wpre + w]
+        const long long qlo = wpre * P / NF + 1, qhi = std::min((long long)P - 1, (wpre + w) * P / NF);
+        for (long long q = qlo; q <= qhi; q++) a.chunkStart[q] = t + 1;
+        if (t == A - 1) a.chunkStart[P] = A;
       }
       baseA += tot.x; baseW += tot.y;
     }
   }
-  if (!tb_grid_barrier(a.ctl, a.err, &sAbort)) goto done;
-  // no fluid cell: the reference returns before its first sweep
+  if (!tb_grid_barrier(a.ctl, ++nBar, a.err, &sAbort)) goto done;
+  // no interior fluid cell: the reference returns before its first sweep
   // (js/solver.js:1330); every CTA read the same total, so all leave here
-  if (sA == 0) { rel = 0; goto done; }
+  if (sA == 0 && !a.st->oddFluid) { rel = 0; solved = true; goto done; }
 
   // ---- phase 2: this CTA's region
   {
+    TbPlan& S = *reinterpret_cast<TbPlan*>(tb_smem_raw);
+    TbPlan2& S2 = *reinterpret_cast<TbPlan2*>(tb_smem_raw + (kTbSmem - sizeof(TbPlan2)) / 16 * 16);
     const int A = sA;
     const long long NF = sNF;
     if (tid == 0) {
@@ -472,320 +494,327 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
     }
     for (int h = tid; h < kHashSlots; h += T) S.hkey[h] = -1;
     __syncthreads();
-    const int t0 = sT0;
-    O = sT1 - sT0;
+    const int t0 = sT0, O = sT1 - sT0;
     if (!sOverflow) {
-      for (int s = tid; s < O; s += T)
-        hash_insert(S, __ldcg(&a.actLin[t0 + s]), &nRegion, &sOverflow, s, (short)p, a.nbx, a.nby);
+      for (int s = tid; s < O; s += T) {
+        const int lin = __ldcg(&a.actLin[t0 + s]);
+        hash_insert(S, S2, lin, __ldcg(a.fmask + lin), &nRegion, &sOverflow, s, a.nbx, a.nby);
+      }
       __syncthreads();
       // the active bricks among the owned bricks' 26 neighbours that other CTAs own
       for (int item = tid; item < O * 26; item += T) {
-        const int s = item / 26, n27 = item % 26 < 13 ? item % 26 : item % 26 + 1;
-        const int bx = S.rbX[s], by = S.rbY[s], bz = S.rbZ[s];
-        const int nx_ = bx + n27 % 3 - 1, ny_ = by + (n27 / 3) % 3 - 1, nz_ = bz + n27 / 9 - 1;
-        if (nx_ < 0 || ny_ < 0 || nz_ < 0 || nx_ >= a.nbx || ny_ >= a.nby || nz_ >= a.nbz) continue;
-        const int lin2 = (nz_ * a.nby + ny_) * a.nbx + nx_;
-        const int ord = __ldcg(&a.brickOrd[lin2]);
-        if (ord < 0) continue;
-        const int ow = owner_of(__ldcg(&a.actWPre[ord]), P, NF);
-        if (ow != p) hash_insert(S, lin2, &nRegion, &sOverflow, -1, (short)ow, a.nbx, a.nby);
+        const int s = item / 26, n26 = item - s * 26, n27 = n26 < 13 ? n26 : n26 + 1;
+        const uchar4 b = S2.rbXYZ[s];
+        const int x = (int)b.x + n27 % 3 - 1, y = (int)b.y + (n27 / 3) % 3 - 1, z = (int)b.z + n27 / 9 - 1;
+        if (x < 0 || y < 0 || z < 0 || x >= a.nbx || y >= a.nby || z >= a.nbz) continue;
+        const int lin2 = (z * a.nby + y) * a.nbx + x;
+        const u64 m = __ldcg(a.fmask + lin2);
+        const int wp = __ldcg(&a.wPre[lin2]);
+        if (m && owner_of(wp, P, NF) != p) hash_insert(S, S2, lin2, m, &nRegion, &sOverflow, -1, a.nbx, a.nby);
       }
       __syncthreads();
-      if (tid == 0 && nRegion > kRbMax) sOverflow = 1;
-      __syncthreads();
     }
-    R = sOverflow ? 0 : nRegion;
-    // face neighbours of each region brick (slot, or -1: outside the region),
-    // and which of its 27 surrounding bricks this CTA owns
-    for (int item = tid; item < R * 6; item += T) {
-      const int s = item / 6, dir = item % 6;
-      int bx = S.rbX[s], by = S.rbY[s], bz = S.rbZ[s];
-      if (dir == 0) bx--; else if (dir == 1) bx++; else if (dir == 2) by--; else if (dir == 3) by++;
-      else if (dir == 4) bz--; else bz++;
-      int slot = -1;
-      if (bx >= 0 && by >= 0 && bz >= 0 && bx < a.nbx && by < a.nby && bz < a.nbz)
-        slot = hash_find(S, (bz * a.nby + by) * a.nbx + bx);
-      S.rbNb[s][dir] = (short)slot;
-    }
-    for (int s = tid; s < R; s += T) S.rbOwnMask[s] = 0;
+    if (tid == 0 && nRegion > kRbMax) sOverflow = 1;
     __syncthreads();
-    for (int item = tid; item < (R - O) * 27; item += T) {
-      const int s = O + item / 27, n27 = item % 27;
-      const int bx = S.rbX[s] + n27 % 3 - 1, by = S.rbY[s] + (n27 / 3) % 3 - 1, bz = S.rbZ[s] + n27 / 9 - 1;
-      if (bx < 0 || by < 0 || bz < 0 || bx >= a.nbx || by >= a.nby || bz >= a.nbz) continue;
-      const int slot = hash_find(S, (bz * a.nby + by) * a.nbx + bx);
-      if (slot >= 0 && slot < O) atomicOr(&S.rbOwnMask[s], 1u << n27);
+    const int R = sOverflow ? 0 : nRegion;
+    // halo bricks: which of the bricks around them this CTA owns; owned
+    // bricks: which are foreign; and every brick's six face neighbours
+    for (int item = tid; item < R * 27; item += T) {
+      const int s = item / 27, n27 = item - s * 27, ox = n27 % 3 - 1, oy = (n27 / 3) % 3 - 1, oz = n27 / 9 - 1;
+      const int slot = slot_at(a, S, S2, s, ox, oy, oz);
+      if (slot >= 0 && (slot < O) != (s < O)) atomicOr(&S.dirs[s], 1u << n27);
+      const int dir = n27 == 12 ? 0 : n27 == 14 ? 1 : n27 == 10 ? 2 : n27 == 16 ? 3 : n27 == 4 ? 4 : n27 == 22 ? 5 : -1;
+      if (dir >= 0) S2.rbNb[dir][s] = slot >= 0 ? (unsigned short)slot : kNone;
     }
     __syncthreads();
-    // dense q of the region and the cell states: 0..4 the distance d of an
-    // interior fluid cell (5: farther), 254 constant (no interior fluid:
-    // never updated). One thread per 4-cell brick row (float4 loads when rows
-    // are 16-byte aligned), four rows in flight per thread.
-    // Update entries are counted per bucket (colour, d <= 3) here, two
-    // 8-bit counters per byte lane of two words per thread (at most 16 cells
-    // per bucket and pass, since R * 16 rows <= 4 T), so the bucketing below
-    // needs a single pass.
-    {
-      const bool vec = (d.nx & 3) == 0;
-      const int nRows = R * 16;
-      unsigned cnt0 = 0u, cnt1 = 0u;         // buckets 0-3 and 4-7, one byte each
-      for (int r0 = 0; r0 < nRows; r0 += 4 * T) {
-        float qv[4][4], pv[4][4];
-        int rowOk[4];
+    // class masks: a halo brick's cells at each d; an owned brick's cells
+    // that some halo stores with H = 2 and 4 (colour 0 to d = H - 1, 1 to H)
+    if (tid < R) {
+      const int s = tid;
+      u64 le[kHMax] = { 0, 0, 0, 0 };
+      for (unsigned m = S.dirs[s]; m; m &= m - 1) {
+        const int n27 = __ffs(m) - 1;
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int row = r0 + u * T + tid;
-          rowOk[u] = 0;
-#pragma unroll
-          for (int c = 0; c < 4; c++) { qv[u][c] = 0.f; pv[u][c] = -1.f; }
-          if (row >= nRows) continue;
-          const int sl = row >> 4, rr = row & 15;
-          const int j = S.rbY[sl] * 4 + (rr & 3), k = S.rbZ[sl] * 4 + (rr >> 2), i0 = S.rbX[sl] * 4;
-          if (j >= d.ny || k >= d.nz) continue;
-          rowOk[u] = 1;
-          const long long g0 = ((long long)k * d.ny + j) * d.nx + i0;
-          if (vec) {
-            const float4 q4 = __ldcg(reinterpret_cast<const float4*>(a.q + g0));
-            const float4 p4 = __ldcg(reinterpret_cast<const float4*>(a.pw + g0));
-            qv[u][0] = q4.x; qv[u][1] = q4.y; qv[u][2] = q4.z; qv[u][3] = q4.w;
-            pv[u][0] = p4.x; pv[u][1] = p4.y; pv[u][2] = p4.z; pv[u][3] = p4.w;
-          } else {
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-              if (i0 + c < d.nx) { qv[u][c] = __ldcg(a.q + g0 + c); pv[u][c] = __ldcg(a.pw + g0 + c); }
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int row = r0 + u * T + tid;
-          if (row >= nRows) continue;
-          const int sl = row >> 4, rr = row & 15, cy = rr & 3, cz = rr >> 2;
-          const unsigned mask = sl < O ? 0u : S.rbOwnMask[sl];
-#pragma unroll
-          for (int c = 0; c < 4; c++) {
-            const int x = row * 4 + c;
-            const int i = S.rbX[sl] * 4 + c, j = S.rbY[sl] * 4 + cy, k = S.rbZ[sl] * 4 + cz;
-            uint8_t st = 254;
-            if (rowOk[u] && i < d.nx && pv[u][c] >= 0.f && interior(d, i, j, k)) {
-              if (sl < O) st = 0;
-              else {
-                // L1 distance to the nearest owned brick box among the 26 around this one
-                int best = 5;
-                for (unsigned m = mask; m; m &= m - 1) {
-                  const int n27 = __ffs(m) - 1, ox = n27 % 3 - 1, oy = (n27 / 3) % 3 - 1, oz = n27 / 9 - 1;
-                  const int dd = (ox < 0 ? c + 1 : ox > 0 ? 4 - c : 0) + (oy < 0 ? cy + 1 : oy > 0 ? 4 - cy : 0) +
-                                 (oz < 0 ? cz + 1 : oz > 0 ? 4 - cz : 0);
-                  best = dd < best ? dd : best;
-                }
-                st = (uint8_t)best;
-              }
-              if (st <= 3) {
-                const unsigned inc = 1u << (8 * st);
-                if ((i + j + k) & 1) cnt1 += inc; else cnt0 += inc;
-              }
-            }
-            S.q[x] = rowOk[u] && i < d.nx ? qv[u][c] : 0.f;
-            S.dist[x] = st;
-          }
-        }
+        for (int q = 0; q < kHMax; q++) le[q] |= kNear.m[n27][q];
       }
+      const u64 f = S.mask[s];
+      // colour of a brick's cell: 4 divides the brick's origin, so it is the parity of x + y + z inside
+      if (s < O) {
+        S.cm[0][s] = f & ((le[0] & ~kOdd) | (le[1] & kOdd)); S.cm[1][s] = f & ((le[2] & ~kOdd) | (le[3] & kOdd));
+        S.cm[2][s] = f & le[0];
+      } else {
 #pragma unroll
-      for (int b = 0; b < 8; b++) {
-        const int v = warp_sum((int)(((b < 4 ? cnt0 : cnt1) >> (8 * (b & 3))) & 0xffu));
-        if (lane == 0 && v) atomicAdd(&bucket[b], v);
+        for (int q = 0; q < kHMax; q++) S.cm[q][s] = f & le[q] & ~(q ? le[q > 0 ? q - 1 : 0] : 0ull);
       }
     }
-    if (tid == 0) S.q[kZero] = 0.f;
+    __syncthreads();
+    // the cells a halo brick contributes to the fetch list: all it stores
+    auto fetched = [&](int s, bool h4) -> u64 {
+      const u64 d1 = S.cm[0][s], d2 = d1 | S.cm[1][s];
+      if (!h4) return (d1 & ~kOdd) | (d2 & kOdd);
+      const u64 d3 = d2 | S.cm[2][s];
+      return (d3 & ~kOdd) | ((d3 | S.cm[3][s]) & kOdd);
+    };
+    // bases: one warp per list scans the bricks' counts
+    if (warp < 15) {
+      const bool owned = warp < 5;                 // rows 0 .. 4 of the owned bricks, 0 .. 9 of the halo bricks
+      const int row = owned ? warp : warp - 5;
+      const int lo = owned ? 0 : O, hi = owned ? std::min(O, R) : R;   // none when the region overflowed
+      int run = 0;
+      for (int s0 = lo; s0 < hi; s0 += 32) {
+        const int s = s0 + lane;
+        u64 m = 0;
+        if (s < hi) {
+          if (owned) m = row == 0 ? S.mask[s] & ~S.cm[2][s] & ~kOdd : row == 1 ? S.mask[s] & kOdd
+                       : row == 4 ? S.cm[2][s] & ~kOdd : S.cm[row - 2][s];
+          else m = row < 8 ? S.cm[row >> 1][s] & (row & 1 ? kOdd : ~kOdd) : fetched(s, row == 9);
+        }
+        const int v = __popcll(m);
+        int x = v;
+        for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
+        if (s < hi) S.base[row][s] = (unsigned short)(run + x - v);
+        run += __shfl_sync(0xffffffffu, x, 31);
+      }
+      if (lane == 0) sCnt[warp] = run;
+    }
     __syncthreads();
     if (tid == 0) {
-      int acc = 0;
-      for (int b = 0; b < 8; b++) { bstart[b] = acc; bcur[b] = acc; acc += bucket[b]; }
-      if (acc > kEMax || bucket[0] + bucket[4] > kOMax) sOverflow = 1;
+      sL.nA = sCnt[0];
+      sL.n[0][0] = sCnt[0] + sCnt[4]; sL.n[1][0] = sCnt[1];
+      for (int q = 0; q < kHMax; q++) { sL.n[0][q + 1] = sCnt[5 + 2 * q]; sL.n[1][q + 1] = sCnt[6 + 2 * q]; }
+      const bool no = sOverflow || a.st->oddFluid != 0;
+      if (no || !make_layout(sL, 2, sCnt[2], sCnt[13])) atomicOr(&a.ctl->over2, 1);
+      if (no || !make_layout(sL, 4, sCnt[3], sCnt[14])) atomicOr(&a.ctl->over4, 1);
+    }
+    // where the other CTAs find this one's cells, for both epoch lengths
+    for (int x = tid; x < std::min(O, R) * 64; x += T) {
+      const int s = x >> 6, c = x & 63;
+#pragma unroll
+      for (int w = 0; w < 2; w++) {
+        const u64 m = S.cm[w][s];
+        if ((m >> c) & 1ull)
+          __stcg(a.xmap + (size_t)w * (size_t)d.nCells + cell_global(a, S2, s, c),
+                 (unsigned)p * (2u * kPubMax) + (unsigned)(S.base[2 + w][s] + bits_below(m, c)));
+      }
+    }
+    if (!tb_grid_barrier(a.ctl, ++nBar, a.err, &sAbort)) goto done;
+    if (tid == 0) {
+      const bool over4 = ld_acquire(reinterpret_cast<const unsigned*>(&a.ctl->over4)) != 0;
+      const bool over2 = ld_acquire(reinterpret_cast<const unsigned*>(&a.ctl->over2)) != 0;
+      sOverflow = over4 && over2;
+      if (!sOverflow) make_layout(sL, over4 ? 2 : 4, sCnt[over4 ? 2 : 3], sCnt[over4 ? 13 : 14]);
     }
     __syncthreads();
-    // update entries: cells with d <= 3, bucketed by (colour, d), and the
-    // halo cells reloaded after every epoch (1 <= d <= 4)
-    {
-      for (int x0 = 0; x0 < R * 64; x0 += T) {
-        const int x = x0 + tid;
-        int b = -1;
-        bool rl = false;
-        unsigned g = 0; int i = 0, j = 0, k = 0;
-        if (x < R * 64 && S.dist[x] <= 4) {
-          dense_global(a, S, x, g, i, j, k);
-          if (S.dist[x] <= 3) b = ((i + j + k) & 1) * 4 + S.dist[x];
-          rl = S.dist[x] >= 1;
-        }
-        const unsigned grp = __match_any_sync(0xffffffffu, b);
-        const int leader = __ffs(grp) - 1;
-        {
-          int base = 0;
-          if (b >= 0 && lane == leader) base = atomicAdd(&bcur[b], __popc(grp));
-          base = __shfl_sync(0xffffffffu, base, leader);
-          if (b >= 0) {
-            const int pos = base + __popc(grp & ((1u << lane) - 1u));
-            if (pos < kEMax) {
-              int nb[6];
-#pragma unroll
-              for (int dir = 0; dir < 6; dir++) nb[dir] = dense_nb(S, x, dir);
-              S.eSelf[pos] = (unsigned short)x;
-              S.eNb[pos][0] = (unsigned)nb[0] | ((unsigned)nb[1] << 16);
-              S.eNb[pos][1] = (unsigned)nb[2] | ((unsigned)nb[3] << 16);
-              S.eNb[pos][2] = (unsigned)nb[4] | ((unsigned)nb[5] << 16);
-              if (b == 0 || b == 4) {
-                const int o = b == 0 ? pos - bstart[0] : bucket[0] + pos - bstart[4];
-                if (o < kOMax) S.oGlob[o] = g;
-              }
+
+    if (sOverflow == 0) {
+      const TbLayout& L = sL;
+      const int which = L.H == 2 ? 0 : 1;
+      uint4* rec = reinterpret_cast<uint4*>(tb_smem_raw + record_at(L.NQ));
+      unsigned char* room = reinterpret_cast<unsigned char*>(&S2) - (size_t)R * 128;
+      const bool clear = room >= tb_smem_raw + sizeof(TbPlan) && room >= reinterpret_cast<unsigned char*>(rec + L.NE);
+      unsigned short* dense = clear ? reinterpret_cast<unsigned short*>(room) : a.dense + (size_t)p * 64 * kRbMax;
+      unsigned* gl = a.glist + (size_t)p * kQMax;
+      unsigned short* pl = a.plist + (size_t)p * kPubMax;
+      uint2* fl = a.flist + (size_t)p * kFetchMax;
+      // the stored index of every region cell (NQ, the zero cell, for the
+      // others), its global cell, and the lists of published and fetched cells
+      for (int x = tid; x < R * 64; x += T) {
+        const int s = x >> 6, c = x & 63, col = (int)((kOdd >> c) & 1ull);
+        const u64 cmask = col ? kOdd : ~kOdd, f = S.mask[s];
+        int e = L.NQ;
+        if ((f >> c) & 1ull) {
+          if (s < O) {
+            const u64 b = S.cm[2][s];
+            if (col) e = L.off[1][0] + S.base[1][s] + bits_below(f & kOdd, c);
+            else if ((b >> c) & 1ull) e = L.nA + S.base[4][s] + bits_below(b & ~kOdd, c);
+            else e = S.base[0][s] + bits_below(f & ~b & ~kOdd, c);
+          } else {
+            for (int q = 0; q < L.H + col - 1; q++) {
+              const u64 m = S.cm[q][s];
+              if ((m >> c) & 1ull) e = L.off[col][q + 1] + S.base[2 * q + col][s] + bits_below(m & cmask, c);
             }
           }
-          const unsigned m = __ballot_sync(0xffffffffu, rl);
-          int rbase = 0;
-          if (lane == 0 && m) rbase = atomicAdd(&nReload, __popc(m));
-          rbase = __shfl_sync(0xffffffffu, rbase, 0);
-          if (rl) {
-            const int rpos = rbase + __popc(m & ((1u << lane) - 1u));
-            if (rpos < kLMax) { S.lDense[rpos] = (unsigned short)x; S.lGlob[rpos] = g; }
-          }
+        }
+        dense[x] = (unsigned short)e;
+        if (e == L.NQ) continue;
+        const unsigned g = cell_global(a, S2, s, c);
+        if (s < O) {
+          gl[e] = g;
+          const u64 m = S.cm[which][s];
+          if ((m >> c) & 1ull) pl[S.base[2 + which][s] + bits_below(m, c)] = (unsigned short)e;
+        } else {
+          fl[S.base[8 + which][s] + bits_below(fetched(s, which != 0), c)] =
+              make_uint2(__ldcg(a.xmap + (size_t)which * (size_t)d.nCells + g), (unsigned)e);
         }
       }
       __syncthreads();
-    }
-    // right-hand side and relaxation weight of every entry, gathered after
-    // the bucketing (whose loop carries shuffles and shared atomics) with
-    // four loads in flight per thread
-    if (!sOverflow) {
-      const int nE = bstart[7] + bucket[7];
-      for (int e0 = tid; e0 < nE; e0 += 4 * T) {
-        float r[4], w[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int e = e0 + u * T;
-          r[u] = 0.f; w[u] = 0.f;
-          unsigned g; int i, j, k;
-          if (e < nE && dense_global(a, S, S.eSelf[e], g, i, j, k)) { r[u] = __ldcg(a.rhs + g); w[u] = __ldcg(a.pw + g); }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int e = e0 + u * T;
-          if (e < nE) { S.eRhs[e] = r[u]; S.ePw[e] = w[u]; }
-        }
-      }
-    }
-    if (tid == 0 && nReload > kLMax) sOverflow = 1;
-    __syncthreads();
-    if (tid == 0 && sOverflow) atomicOr(&a.ctl->overflow, 1);
-    // the owned cells' exchange words start with tag 0 (epochs count from 1)
-    if (!sOverflow) {
-      const int nOwn = bucket[0] + bucket[4];
-      for (int e = tid; e < nOwn; e += T) {
-        st_relaxed_u64(a.xq + S.oGlob[e], 0ull);
-        st_relaxed_u64(a.xq + (size_t)d.nCells + S.oGlob[e], 0ull);
+      // the values and every entry's record, over the first tables
+      float* sq = reinterpret_cast<float*>(tb_smem_raw);
+      if (tid == 0) sq[L.NQ] = 0.f;
+#pragma unroll 2
+      for (int x = tid; x < R * 64; x += T) {
+        const int e = dense[x], s = x >> 6, c = x & 63, cx = c & 3, cy = (c >> 2) & 3, cz = c >> 4;
+        if (e >= L.NQ) continue;
+        const unsigned g = cell_global(a, S2, s, c);
+        sq[e] = __ldcg(a.q + g);
+        if (e >= L.NE) continue;
+        const float rhs = __ldcg(a.rhs + g);
+        const unsigned k = __ldcg(a.diag8 + g);
+        auto nbr = [&](int dir, bool in, int step, int wrap) -> unsigned {
+          if (in) return (unsigned)dense[x + step] << 2;
+          const unsigned t = S2.rbNb[dir][s];
+          return (t == kNone ? (unsigned)L.NQ : (unsigned)dense[(int)t * 64 + c + wrap]) << 2;
+        };
+        const unsigned w0 = nbr(0, cx > 0, -1, 3) | (nbr(1, cx < 3, 1, -3) << 16);
+        const unsigned w1 = nbr(2, cy > 0, -4, 12) | (nbr(3, cy < 3, 4, -12) << 16);
+        const unsigned w2 = nbr(4, cz > 0, -16, 48) | (nbr(5, cz < 3, 16, -48) << 16);
+        rec[e] = make_uint4(w0 | (k & 3u), w1 | (k >> 2), w2, __float_as_uint(rhs));
       }
     }
   }
-  if (!tb_grid_barrier(a.ctl, a.err, &sAbort)) goto done;
-  if (tid == 0) sOverflow = (int)ld_acquire(reinterpret_cast<const unsigned*>(&a.ctl->overflow));
   __syncthreads();
 
   if (sOverflow == 0) {
-    // ---- phase 3: temporal-blocked iterations
-    int cum[2][4];
+    // ---- phase 3: iterations
+    const int H = sL.H, NQ = sL.NQ, c1s = sL.c1, nA = sL.nA, n00 = sL.n[0][0], n10 = sL.n[1][0];
+    const int nPub = sL.pub, nFetch = sL.fetch;
+    float* sq = reinterpret_cast<float*>(tb_smem_raw);
+    const uint4* rec = reinterpret_cast<const uint4*>(tb_smem_raw + record_at(NQ));
+    const unsigned* gl = a.glist + (size_t)p * kQMax;
+    const unsigned short* pl = a.plist + (size_t)p * kPubMax;
+    const uint2* fl = a.flist + (size_t)p * kFetchMax;
+    // a thread keeps its first four cells to fetch and to publish
+    unsigned fg[4];
+    unsigned short fe[4], pe[4];
 #pragma unroll
-    for (int c = 0; c < 2; c++) {
-      int acc = 0;
-#pragma unroll
-      for (int dd = 0; dd < 4; dd++) { acc += bucket[c * 4 + dd]; cum[c][dd] = acc; }
+    for (int u = 0; u < 4; u++) {
+      const int l = tid + u * T;
+      const uint2 v = l < nFetch ? fl[l] : make_uint2(0u, 0u);
+      fg[u] = v.x; fe[u] = (unsigned short)v.y;
+      pe[u] = l < nPub ? pl[l] : (unsigned short)0;
     }
-    const int st0 = bstart[0], st1 = bstart[4];
-    const int nOwn0 = bucket[0], nOwn1 = bucket[4];
+    __syncthreads();
     const double om1 = a.om1;
-    unsigned epoch = 0;
     int nChecks = 0;
     bool fresh = true, checked = false;
-    // the halo values of epoch `target`: four loads in flight per thread,
-    // then each word polled again (bounded) until its tag reads target
-    auto wait_and_reload = [&](unsigned target) -> bool {
-      const unsigned long long* src = a.xq + (size_t)(target & 1u) * (size_t)d.nCells;
-      for (int l0 = tid; l0 < nReload; l0 += 4 * T) {
-        unsigned long long v[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) { const int l = l0 + u * T; v[u] = l < nReload ? ld_relaxed_u64(src + S.lGlob[l]) : 0ull; }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int l = l0 + u * T;
-          if (l >= nReload) continue;
-          long long n = 0;
-          while ((unsigned)(v[u] >> 32) != target) {
-            if (++n > kTbSpinLimit || *(volatile int*)&sAbort) {
-              if (n > kTbSpinLimit) atomicOr(a.err, WS_DERR_TIMEOUT);
-              sAbort = 1;
-              break;
-            }
-            v[u] = ld_relaxed_u64(src + S.lGlob[l]);
+    // the halo values of epoch `ep`: four loads in flight per thread, then
+    // each word polled again (bounded) until its tag is the epoch's
+    auto wait_and_reload = [&](unsigned ep) -> bool {
+      const u64* src = a.xq + (ep & 1u) * (size_t)kPubMax;
+      const unsigned target = tag0 + ep;
+      u64 v[4];
+      auto settle = [&](int e, const u64* w, u64 val) {
+        long long n = 0;
+        while ((unsigned)(val >> 32) != target) {
+          if (++n > kTbSpinLimit || *(volatile int*)&sAbort) {
+            if (n > kTbSpinLimit) atomicOr(a.err, WS_DERR_TIMEOUT);
+            sAbort = 1;
+            break;
           }
-          S.q[S.lDense[l]] = __uint_as_float((unsigned)v[u]);
+          val = ld_relaxed_u64(w);
         }
+        sq[e] = __uint_as_float((unsigned)val);
+      };
+#pragma unroll
+      for (int u = 0; u < 4; u++) v[u] = tid + u * T < nFetch ? ld_relaxed_u64(src + fg[u]) : 0ull;
+#pragma unroll
+      for (int u = 0; u < 4; u++) if (tid + u * T < nFetch) settle(fe[u], src + fg[u], v[u]);
+      for (int l = tid + 4 * T; l < nFetch; l += T) {
+        const uint2 f = fl[l];
+        settle((int)f.y, src + f.x, ld_relaxed_u64(src + f.x));
       }
       __syncthreads();
       return *(volatile int*)&sAbort == 0;
     };
-    // the owned cells of epoch `ep` into exchange buffer ep & 1
-    auto publish_owned = [&](unsigned ep) {
-      unsigned long long* dst = a.xq + (size_t)(ep & 1u) * (size_t)d.nCells;
-      const unsigned long long tag = (unsigned long long)ep << 32;
-      for (int e = tid; e < nOwn0 + nOwn1; e += T)
-        st_relaxed_u64(dst + S.oGlob[e], tag | __float_as_uint(S.q[S.eSelf[e < nOwn0 ? st0 + e : st1 + (e - nOwn0)]]));
+    auto publish = [&](unsigned ep) {
+      u64* dst = a.xq + ((size_t)p * 2 + (ep & 1u)) * (size_t)kPubMax;
+      const u64 tag = (u64)(tag0 + ep) << 32;
+#pragma unroll
+      for (int u = 0; u < 4; u++) if (tid + u * T < nPub) st_relaxed_u64(dst + tid + u * T, tag | __float_as_uint(sq[pe[u]]));
+      for (int l = tid + 4 * T; l < nPub; l += T) st_relaxed_u64(dst + l, tag | __float_as_uint(sq[pl[l]]));
     };
-    auto write_owned = [&](float* dst) {
-      for (int e = tid; e < nOwn0 + nOwn1; e += T)
-        __stcg(dst + S.oGlob[e], S.q[S.eSelf[e < nOwn0 ? st0 + e : st1 + (e - nOwn0)]]);
+    // the six neighbour values of a record, and its stencil count
+    auto at = [&](unsigned off) -> float { return *reinterpret_cast<const float*>(tb_smem_raw + off); };
+    auto gather = [&](const uint4& r, float (&v)[6]) {
+      v[0] = at(r.x & 0xfffcu); v[1] = at(r.x >> 16); v[2] = at(r.y & 0xfffcu);
+      v[3] = at(r.y >> 16); v[4] = at(r.z & 0xfffcu); v[5] = at(r.z >> 16);
     };
+    auto count_of = [](const uint4& r) -> unsigned { return (r.x & 3u) | ((r.y & 3u) << 2); };
+    // entries [lo, hi): two updates per thread in flight where a thread has
+    // two entries (e and e + T are of one colour, so neither reads what the
+    // other writes); a thread with one entry reads nothing extra
+    auto sweep = [&](int lo, int hi) {
+      for (int e1 = lo + tid; e1 < hi; e1 += 2 * T) {
+        const uint4 r1 = rec[e1];
+        float v[6];
+        gather(r1, v);
+        const float p1 = sPw[count_of(r1)];
+        const int e2 = e1 + T;
+        if (e2 < hi) {
+          const uint4 r2 = rec[e2];
+          float u[6];
+          gather(r2, u);
+          const float p2 = sPw[count_of(r2)];
+          const float q1 = relax(sq[e1], p1, __uint_as_float(r1.w), v, om1);
+          const float q2 = relax(sq[e2], p2, __uint_as_float(r2.w), u, om1);
+          sq[e1] = q1;
+          sq[e2] = q2;
+        } else {
+          sq[e1] = relax(sq[e1], p1, __uint_as_float(r1.w), v, om1);
+        }
+      }
+    };
+    // residual of the owned cells of the state in sq (halo values fresh)
     auto check_residual = [&]() -> bool {
-      const double2 part = owned_residual(a, S, O, sRed);
+      double rr = 0, bb = 0;
+      for (int x = tid; x < n00 + n10; x += T) {
+        const int e = x < n00 ? x : c1s + (x - n00);
+        const uint4 rc = rec[e];
+        float v[6];
+        gather(rc, v);
+        double sum = (double)v[0];
+        sum += (double)v[1]; sum += (double)v[2]; sum += (double)v[3]; sum += (double)v[4]; sum += (double)v[5];
+        const double b = __uint_as_float(rc.w);
+        const double r = b + sum - (double)count_of(rc) * (double)sq[e];
+        rr += r * r; bb += b * b;
+      }
+      rr = warp_sum(rr); bb = warp_sum(bb);
+      if (lane == 0) sRed[warp] = make_double2(rr, bb);
+      __syncthreads();
+      double2 part = make_double2(0, 0);
+      if (warp == 0) {
+        const double2 v = sRed[lane];
+        part = make_double2(warp_sum(v.x), warp_sum(v.y));
+      }
+      __syncthreads();
       if (!global_residual(a, part, nChecks++, &sRel, &sAbort)) return false;
       rel = sRel;
       return true;
     };
     while (it < a.iters) {
-      int m = std::min(2, a.iters - it);
+      int m = std::min(H >> 1, a.iters - it);
       if (a.check > 0) m = std::min(m, a.check - it % a.check);
-      if (!fresh && !wait_and_reload(epoch)) goto done;
       const int s = 2 * m;
-      for (int t = 1; t <= s; t++) {
-        const int col = (t - 1) & 1, dmax = s - t;
-        const int n = cum[col][dmax], base = col ? st1 : st0;
-        // two updates per thread in flight where a thread has two entries
-        // (e and e + T are of one colour, so neither reads what the other
-        // writes); a thread with one entry reads nothing extra
-        for (int e = tid; e < n; e += 2 * T) {
-          const int i1 = base + e, e2 = e + T;
-          const unsigned a0 = S.eNb[i1][0], a1 = S.eNb[i1][1], a2 = S.eNb[i1][2];
-          float v[6];
-          v[0] = S.q[a0 & 0xffffu]; v[1] = S.q[a0 >> 16]; v[2] = S.q[a1 & 0xffffu];
-          v[3] = S.q[a1 >> 16]; v[4] = S.q[a2 & 0xffffu]; v[5] = S.q[a2 >> 16];
-          const int x1 = S.eSelf[i1];
-          if (e2 < n) {
-            const int i2 = base + e2;
-            const unsigned b0 = S.eNb[i2][0], b1 = S.eNb[i2][1], b2 = S.eNb[i2][2];
-            float u[6];
-            u[0] = S.q[b0 & 0xffffu]; u[1] = S.q[b0 >> 16]; u[2] = S.q[b1 & 0xffffu];
-            u[3] = S.q[b1 >> 16]; u[4] = S.q[b2 & 0xffffu]; u[5] = S.q[b2 >> 16];
-            const int x2 = S.eSelf[i2];
-            const float q1 = relax(S.q[x1], S.ePw[i1], S.eRhs[i1], v, om1);
-            const float q2 = relax(S.q[x2], S.ePw[i2], S.eRhs[i2], u, om1);
-            S.q[x1] = q1;
-            S.q[x2] = q2;
-          } else {
-            S.q[x1] = relax(S.q[x1], S.ePw[i1], S.eRhs[i1], v, om1);
-          }
-        }
+      if (fresh) {
+        sweep(0, sL.cum[0][s - 1]);
+      } else {
+        // the cells that read no halo first. With H = 4 some of them are
+        // published (colour 0 to d = 3): the barrier keeps their new values
+        // behind every thread's publication of the old ones
+        if (H != 2) __syncthreads();
+        sweep(0, nA);
+        if (!wait_and_reload(epoch)) goto done;
+        sweep(nA, sL.cum[0][s - 1]);
+      }
+      __syncthreads();
+      for (int t = 2; t <= s; t++) {
+        const int base = t & 1 ? 0 : c1s;
+        sweep(base, base + sL.cum[t & 1 ? 0 : 1][s - t]);
         __syncthreads();
       }
       it += m;
       epoch++;
-      // no barrier before the reload that follows: it writes halo cells
-      // (d >= 1) of S.q, this reads owned cells (d = 0)
-      publish_owned(epoch);
+      publish(epoch);
       fresh = false;
       checked = false;
       const bool doCheck = a.check > 0 && it % a.check == 0;
@@ -799,13 +828,18 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
     }
     if (!checked && !check_residual()) goto done;           // no iteration ran: residual of the start
     // the result lands in the solve's own q buffer
-    write_owned(a.q);
-  } else {
+    for (int x = tid; x < n00 + n10; x += T) {
+      const int e = x < n00 ? x : c1s + (x - n00);
+      __stcg(a.q + gl[e], sq[e]);
+    }
+    solved = true;
+  } else if (!a.listFallback) {
+    solved = true;
     // ---- fallback: red-black sweeps over the owned bricks in global memory,
     // a grid barrier per half-sweep
     path = 4;
     const int t0 = sT0;
-    O = sT1 - sT0;
+    const int O = sT1 - sT0;
     const double om1 = a.om1;
     const long long nxl = d.nx, nxy = (long long)d.nx * d.ny;
     int nChecks = 0;
@@ -838,7 +872,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
       __syncthreads();
       double2 part = make_double2(0, 0);
       if (tid < 32) {
-        const double2 v = tid < (T >> 5) ? sRed[tid] : make_double2(0, 0);
+        const double2 v = sRed[tid];
         part = make_double2(warp_sum(v.x), warp_sum(v.y));
       }
       __syncthreads();
@@ -858,7 +892,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
           v[3] = __ldcg(qc + nxl); v[4] = __ldcg(qc - nxy); v[5] = __ldcg(qc + nxy);
           __stcg(qc, relax(__ldcg(qc), a.pw[g], a.rhs[g], v, om1));
         }
-        if (!tb_grid_barrier(a.ctl, a.err, &sAbort)) goto done;
+        if (!tb_grid_barrier(a.ctl, ++nBar, a.err, &sAbort)) goto done;
       }
       it++;
       checked = false;
@@ -872,83 +906,101 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
     if (!checked && !residual()) goto done;
   }
 done:
-  if (p == 0 && tid == 0) { *a.outIters = it; *a.outRel = rel; *a.outPath = path; }
+  if (p == 0 && tid == 0) {
+    // every CTA read the tag base before its first barrier, which this CTA has passed
+    *(volatile unsigned*)&a.ctl->tagBase = tag0 + epoch + 1u;
+    if (solved || sAbort) a.ctl->solved = 1;         // after a timed-out wait nothing else runs either
+    if (solved || sAbort) { *a.outIters = it; *a.outRel = rel; *a.outPath = path; }
+  }
 }
 
 // ---------------------------------------------------------------- host side
 struct TbState {
+  void* slab = nullptr;
   TbCtl* ctl = nullptr;
-  unsigned long long* xq = nullptr;
-  int* brickW = nullptr;
+  u64* xq = nullptr;
   int2* cntPart = nullptr;
-  int *actLin = nullptr, *actWPre = nullptr, *brickOrd = nullptr, *chunkStart = nullptr;
+  int *actLin = nullptr, *wPre = nullptr, *chunkStart = nullptr;
+  unsigned *xmap = nullptr, *glist = nullptr;
+  unsigned short *plist = nullptr, *dense = nullptr;
+  uint2* flist = nullptr;
   double2* resPart = nullptr;
   int P = 0, nbx = 0, nby = 0, nbz = 0, mbits = 0;
 };
 
-size_t sor_tb_smem_bytes() { return sizeof(TbSmem); }
-
-// 0 when the temporal-blocked solve cannot run on this device (too little
-// shared memory or co-residency); the state is then left unallocated.
+// null when the solve cannot run on this device (too little shared memory or
+// co-residency) or grid (a brick coordinate beyond 8 bits); the state is
+// then left unallocated.
 cudaError_t sor_tb_init(void** statePtr, const Dims& d, int device) {
   *statePtr = nullptr;
   int smCount = 0, optin = 0;
   cudaDeviceGetAttribute(&smCount, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-  if (smCount < 1 || smCount > kMaxCtas || optin < (int)sizeof(TbSmem)) return cudaSuccess;
-  if (cudaFuncSetAttribute(k_sor_tb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TbSmem)) != cudaSuccess) {
+  if (smCount < 1 || smCount > kMaxCtas || optin < kTbSmem) return cudaSuccess;
+  if (std::max(d.nx, std::max(d.ny, d.nz)) > 1020) return cudaSuccess;
+  if (cudaFuncSetAttribute(k_sor_tb, cudaFuncAttributeMaxDynamicSharedMemorySize, kTbSmem) != cudaSuccess) {
     cudaGetLastError();
     return cudaSuccess;
   }
   int perSM = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_sor_tb, kTbThreads, sizeof(TbSmem)) != cudaSuccess ||
-      perSM < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_sor_tb, kTbThreads, kTbSmem) != cudaSuccess || perSM < 1) {
     cudaGetLastError();
     return cudaSuccess;
   }
   TbState* S = new TbState();
+  *statePtr = S;
   S->P = smCount;
   S->nbx = (d.nx + 3) / 4; S->nby = (d.ny + 3) / 4; S->nbz = (d.nz + 3) / 4;
   int mb = 0;
   while ((1 << mb) < std::max(S->nbx, std::max(S->nby, S->nbz))) mb++;
   S->mbits = mb;
-  const long long nB = (long long)S->nbx * S->nby * S->nbz, MC = 1LL << (3 * mb);
+  const long long nB = (long long)S->nbx * S->nby * S->nbz;
+  // every buffer from one allocation (exchange words zeroed: tags start at 1)
+  const size_t P = (size_t)smCount, words = 2 * kPubMax * P;
+  size_t at = 0;
+  auto place = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~(size_t)255; return o; };
+  const size_t oCtl = place(sizeof(TbCtl)), oXq = place(sizeof(u64) * words), oCnt = place(sizeof(int2) * P);
+  const size_t zeroed = at;
+  const size_t oAct = place(sizeof(int) * (size_t)nB), oPre = place(sizeof(int) * (size_t)nB);
+  const size_t oChunk = place(sizeof(int) * (P + 1)), oMap = place(sizeof(unsigned) * 2 * (size_t)d.nCells);
+  const size_t oG = place(sizeof(unsigned) * kQMax * P), oP = place(sizeof(unsigned short) * kPubMax * P);
+  const size_t oD = place(sizeof(unsigned short) * 64 * kRbMax * P), oF = place(sizeof(uint2) * kFetchMax * P);
+  const size_t oRes = place(sizeof(double2) * 2 * P);
   cudaError_t e;
-  if ((e = cudaMalloc(&S->ctl, sizeof(TbCtl))) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&S->xq, sizeof(unsigned long long) * 2 * d.nCells)) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&S->brickW, sizeof(int) * MC)) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&S->cntPart, sizeof(int2) * smCount)) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&S->actLin, sizeof(int) * nB)) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&S->actWPre, sizeof(int) * nB)) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&S->brickOrd, sizeof(int) * nB)) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&S->chunkStart, sizeof(int) * (smCount + 1))) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&S->resPart, sizeof(double2) * 2 * smCount)) != cudaSuccess) return e;
-  *statePtr = S;
+  if ((e = cudaMalloc(&S->slab, at)) != cudaSuccess) return e;
+  if ((e = cudaMemset(S->slab, 0, zeroed)) != cudaSuccess) return e;
+  unsigned char* base = (unsigned char*)S->slab;
+  S->ctl = (TbCtl*)(base + oCtl); S->xq = (u64*)(base + oXq); S->cntPart = (int2*)(base + oCnt);
+  S->actLin = (int*)(base + oAct); S->wPre = (int*)(base + oPre); S->chunkStart = (int*)(base + oChunk);
+  S->xmap = (unsigned*)(base + oMap); S->glist = (unsigned*)(base + oG); S->plist = (unsigned short*)(base + oP);
+  S->dense = (unsigned short*)(base + oD); S->flist = (uint2*)(base + oF); S->resPart = (double2*)(base + oRes);
   return cudaSuccess;
 }
 
 void sor_tb_free(void* statePtr) {
   TbState* S = (TbState*)statePtr;
   if (!S) return;
-  cudaFree(S->ctl); cudaFree(S->xq); cudaFree(S->brickW); cudaFree(S->cntPart); cudaFree(S->actLin);
-  cudaFree(S->actWPre); cudaFree(S->brickOrd); cudaFree(S->chunkStart); cudaFree(S->resPart);
+  cudaFree(S->slab);
   delete S;
 }
+const int* sor_tb_solved(void* statePtr) { return &((TbState*)statePtr)->ctl->solved; }
 
-// the control block reset and the solve (two stream operations, one kernel)
+// the control block reset and the solve (two stream operations, one kernel).
+// listFallback: leave a system that does not fit to the list kernels
 cudaError_t launch_sor_tb(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                          int iters, int check, double tol, int* err, int* outIters, double* outRel, int* outPath,
-                          cudaStream_t s) {
+                          int iters, int check, double tol, DevStatus* st, bool listFallback, int* outIters,
+                          double* outRel, int* outPath, cudaStream_t s) {
   TbState* S = (TbState*)statePtr;
-  cudaError_t e = cudaMemsetAsync(S->ctl, 0, sizeof(TbCtl), s);
+  cudaError_t e = cudaMemsetAsync(S->ctl, 0, offsetof(TbCtl, tagBase), s);
   if (e != cudaSuccess) return e;
   TbArgs a;
-  a.d = d; a.q = g.q; a.xq = S->xq; a.rhs = g.rhs; a.pw = g.pw; a.diag8 = diag8;
+  a.d = d; a.q = g.q; a.xq = S->xq; a.rhs = g.rhs; a.pw = g.pw; a.diag8 = diag8; a.fmask = g.fmask; a.st = st;
   a.nbx = S->nbx; a.nby = S->nby; a.nbz = S->nbz; a.mbits = S->mbits;
-  a.brickW = S->brickW; a.cntPart = S->cntPart; a.actLin = S->actLin; a.actWPre = S->actWPre;
-  a.brickOrd = S->brickOrd; a.chunkStart = S->chunkStart; a.resPart = S->resPart; a.ctl = S->ctl;
-  a.om1 = 1 - omega; a.iters = iters; a.check = check; a.tol = tol; a.err = err;
+  a.cntPart = S->cntPart; a.actLin = S->actLin; a.wPre = S->wPre; a.chunkStart = S->chunkStart;
+  a.xmap = S->xmap; a.glist = S->glist; a.plist = S->plist; a.dense = S->dense; a.flist = S->flist; a.resPart = S->resPart; a.ctl = S->ctl;
+  a.om1 = 1 - omega; a.iters = iters; a.check = check; a.tol = tol; a.err = &st->err;
+  a.listFallback = listFallback ? 1 : 0;
   a.outIters = outIters; a.outRel = outRel; a.outPath = outPath;
   void* args[] = { &a };
-  return cudaLaunchCooperativeKernel((void*)k_sor_tb, dim3(S->P), dim3(kTbThreads), args, sizeof(TbSmem), s);
+  return cudaLaunchCooperativeKernel((void*)k_sor_tb, dim3(S->P), dim3(kTbThreads), args, kTbSmem, s);
 }

@@ -55,6 +55,36 @@ def test_region_solve_bitwise(n, R, depth, particles, iters, paths):
     fs.close()
 
 
+@pytest.mark.parametrize("n,share,iters", [(64, 0.02, 60), (64, 0.2, 25), (96, 0.008, 80), (168, 0.01, 40)])
+def test_scattered_fluid_bitwise(n, share, iters):
+    """Scattered fluid cells: many bricks hold one or two, so a CTA often holds
+    a neighbour's cell in its halo while its own lie beyond that neighbour's
+    (each must still wait for the other before it overwrites an exchange
+    buffer). 168^3 takes the large-grid route."""
+    fs = FluidSolver(nx=n, ny=n, nz=n, dx=1.0, coreR=1.0, targetParticles=1000.0, capacity=1000)
+    r = np.random.default_rng(n)
+    ct = np.where(r.random((n, n, n)) < share, 1, 0).astype(np.uint8)
+    for a in range(3):
+        np.moveaxis(ct, a, 0)[[0, -1]] = 2
+    fs.set_params(sorTol=0.0, pressureIters=iters, omega=1.7)
+    fs.upload("cellType", ct.ravel())
+    for k in ("u", "v", "w"):
+        fs.upload(k, r.normal(size=fs.field_size(k)).astype(np.float32))
+    q0 = np.where(ct.ravel() == 1, r.normal(size=n ** 3), 0).astype(np.float32)
+    fs.upload("q", q0)
+    for _ in range(3):                       # tags count on from solve to solve
+        fs.upload("q", q0)
+        fs.stage("PRESSURE")
+    s = fs.scalars
+    assert s.sorIters == iters
+    q = fs.q.copy()
+    assert np.all(np.isfinite(q)) and np.any(q != q0)
+    fs.upload("q", q0)
+    fs.time_kernel(0, iters)
+    assert np.array_equal(q.view(np.uint32), fs.q.view(np.uint32))
+    fs.close()
+
+
 @pytest.mark.parametrize("check", [1, 3, 4, 10])
 def test_check_cadence_stops_where_fixed_iterations_do(check):
     """Tolerance mode stops at a multiple of the cadence with the iterates of

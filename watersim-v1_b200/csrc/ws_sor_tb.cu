@@ -44,8 +44,12 @@
 // scattered over a grid-sized array took half of the solve in L2 traffic and
 // polls. Double buffering makes the write of epoch e + 2 safe against
 // neighbours still reading epoch e: a CTA computes epoch e + 2 only after
-// reading its neighbours' epoch e + 1 values, which each neighbour wrote
-// after it had read this CTA's epoch e values (halo adjacency is symmetric).
+// reading its neighbours' epoch e + 1 words, which each neighbour wrote after
+// it had read this CTA's epoch e words. That needs every reader of a CTA to be
+// read by it, and cells alone do not give it (a CTA may hold a cell near a
+// foreign brick whose own fluid lies beyond the halo). So a list begins with
+// one word that stands for the CTA, and a CTA fetches that word of every owner
+// of an active brick around its own; brick adjacency is symmetric.
 // Tags count on from solve to solve (tagBase), so a word left by an earlier
 // solve never matches and nothing has to be cleared.
 //
@@ -161,6 +165,7 @@ struct TbPlan2 {
   unsigned short rbNb[6][kRbMax];         // face neighbours' slots (kNone: not in the region)
 };
 constexpr unsigned short kNone = 0xffffu;
+static_assert(kMaxCtas <= kTbThreads, "one thread per CTA builds the list of neighbours");
 static_assert(sizeof(TbPlan) + sizeof(TbPlan2) <= (size_t)kTbSmem, "plan tables");
 
 // bits of the cells with x + y + z odd
@@ -351,10 +356,10 @@ struct TbLayout {
   int n[2][kHMax + 1];           // its cells
   int nA;                        // colour 0, d = 0: cells without a foreign face neighbour (stored first)
   int cum[2][kHMax];             // cells of a colour with d <= index
-  int pub, fetch;                // published and fetched cells
+  int pub, fetch;                // words published and fetched: the cells and the CTAs' own words
 };
-// bytes of the solve's values and records: the cells and the zero cell, then the entries
-__device__ __forceinline__ int record_at(int NQ) { return (4 * (NQ + 1) + 15) & ~15; }
+// bytes of the solve's values and records: the cells, the zero cell and one that takes the CTAs' own words, then the entries
+__device__ __forceinline__ int record_at(int NQ) { return (4 * (NQ + 2) + 15) & ~15; }
 // whether the solve's values and records fit with epochs of H half-sweeps
 __device__ __forceinline__ bool make_layout(TbLayout& L, int H, int pub, int fetch) {
   L.H = H; L.pub = pub; L.fetch = fetch;
@@ -394,6 +399,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
   __shared__ int sAbort, sOverflow, nRegion, sT0, sT1, sA;
   __shared__ TbLayout sL;
   __shared__ int sCnt[16];
+  __shared__ unsigned sOwn[kMaxCtas / 32];             // the CTAs that own active bricks around this one's
   __shared__ float sPw[8];
   __shared__ int2 sScan[33];
   __shared__ double2 sRed[32];
@@ -493,6 +499,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
       if (nRegion > kRbMax) sOverflow = 1;
     }
     for (int h = tid; h < kHashSlots; h += T) S.hkey[h] = -1;
+    if (tid < kMaxCtas / 32) sOwn[tid] = 0u;
     __syncthreads();
     const int t0 = sT0, O = sT1 - sT0;
     if (!sOverflow) {
@@ -510,7 +517,9 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
         const int lin2 = (z * a.nby + y) * a.nbx + x;
         const u64 m = __ldcg(a.fmask + lin2);
         const int wp = __ldcg(&a.wPre[lin2]);
-        if (m && owner_of(wp, P, NF) != p) hash_insert(S, S2, lin2, m, &nRegion, &sOverflow, -1, a.nbx, a.nby);
+        const int ow = m ? owner_of(wp, P, NF) : p;
+        if (ow == p) continue;
+        if (hash_insert(S, S2, lin2, m, &nRegion, &sOverflow, -1, a.nbx, a.nby)) atomicOr(&sOwn[ow >> 5], 1u << (ow & 31));
       }
       __syncthreads();
     }
@@ -579,6 +588,9 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
     }
     __syncthreads();
     if (tid == 0) {
+      int nb = 0;                                  // one word per CTA around this one, and this one's own
+      for (int w = 0; w < kMaxCtas / 32; w++) nb += __popc(sOwn[w]);
+      sCnt[2]++; sCnt[3]++; sCnt[13] += nb; sCnt[14] += nb;
       sL.nA = sCnt[0];
       sL.n[0][0] = sCnt[0] + sCnt[4]; sL.n[1][0] = sCnt[1];
       for (int q = 0; q < kHMax; q++) { sL.n[0][q + 1] = sCnt[5 + 2 * q]; sL.n[1][q + 1] = sCnt[6 + 2 * q]; }
@@ -594,7 +606,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
         const u64 m = S.cm[w][s];
         if ((m >> c) & 1ull)
           __stcg(a.xmap + (size_t)w * (size_t)d.nCells + cell_global(a, S2, s, c),
-                 (unsigned)p * (2u * kPubMax) + (unsigned)(S.base[2 + w][s] + bits_below(m, c)));
+                 (unsigned)p * (2u * kPubMax) + 1u + (unsigned)(S.base[2 + w][s] + bits_below(m, c)));
       }
     }
     if (!tb_grid_barrier(a.ctl, ++nBar, a.err, &sAbort)) goto done;
@@ -616,6 +628,13 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
       unsigned* gl = a.glist + (size_t)p * kQMax;
       unsigned short* pl = a.plist + (size_t)p * kPubMax;
       uint2* fl = a.flist + (size_t)p * kFetchMax;
+      if (tid == 0) pl[0] = (unsigned short)L.NQ;
+      if (tid < P && ((sOwn[tid >> 5] >> (tid & 31)) & 1u)) {
+        int at = L.fetch - 1;                      // the list's end: the CTAs' own words
+        for (int w = kMaxCtas / 32 - 1; w > (tid >> 5); w--) at -= __popc(sOwn[w]);
+        at -= __popc(sOwn[tid >> 5] & ~((2u << (tid & 31)) - 1u));
+        fl[at] = make_uint2((unsigned)tid * (2u * kPubMax), (unsigned)L.NQ + 1u);
+      }
       // the stored index of every region cell (NQ, the zero cell, for the
       // others), its global cell, and the lists of published and fetched cells
       for (int x = tid; x < R * 64; x += T) {
@@ -641,7 +660,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
         if (s < O) {
           gl[e] = g;
           const u64 m = S.cm[which][s];
-          if ((m >> c) & 1ull) pl[S.base[2 + which][s] + bits_below(m, c)] = (unsigned short)e;
+          if ((m >> c) & 1ull) pl[1 + S.base[2 + which][s] + bits_below(m, c)] = (unsigned short)e;
         } else {
           fl[S.base[8 + which][s] + bits_below(fetched(s, which != 0), c)] =
               make_uint2(__ldcg(a.xmap + (size_t)which * (size_t)d.nCells + g), (unsigned)e);

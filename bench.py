@@ -433,8 +433,8 @@ def roofline(fs, ms_step, iters):
     us_pr = fs.time_kernel(10, 5)
     us_ex = fs.time_kernel(11, 5)
     Fa = 192.0 * active_bricks(fs)
-    # P2G as the substep runs it by default: particle index order, runs of up
-    # to four consecutive particles per atomic (id 1); the cell-ordered variant (id 12: counting
+    # P2G in particle index order, runs of two or
+    # four consecutive particles per thread (id 1; in a substep the marking rides along); the cell-ordered variant (id 12: counting
     # sort, prefix sum, scatter of particle ids, shared-memory sums per brick,
     # every brick visited) beside it
     us_p2g = fs.time_kernel(1, 5)

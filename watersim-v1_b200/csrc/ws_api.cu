@@ -819,18 +819,19 @@ static ws_status stage_clear_raster(ws_handle* h, bool bricks = false) {
   if (bricks) launch_clear_acc_bricks(h->d, grid_of(h), h->bricks, h->stream);
   return check_launch(h, bricks ? 2 : 1);
 }
+// the active-brick list from this substep's seeds
+static ws_status brick_activity(ws_handle* h) {
+  cudaError_t e = launch_brick_activity(h->bricks, h->stream);
+  if (e != cudaSuccess) return fail_cuda(h, e, "active bricks");
+  return check_launch(h, 1);
+}
 // bricks: the substep's own pipeline, where (with p2gCellOrder) the mark
 // pass also counts the particles per cell for the cell-ordered P2G
 static ws_status stage_mark(ws_handle* h, bool bricks = false) {
   launch_mark_fluid(h->d, grid_of(h), parts_of(h), h->terr, h->S.oceanR, h->S.coreR,
                     bricks && h->P.p2gCellOrder ? &h->csort : nullptr, h->st, h->stream);
   ws_status s = check_launch(h, 1); if (s) return s;
-  if (bricks) {
-    cudaError_t e = launch_brick_activity(h->bricks, h->stream);
-    if (e != cudaSuccess) return fail_cuda(h, e, "active bricks");
-    s = check_launch(h, 1); if (s) return s;
-  }
-  return WS_OK;
+  return bricks ? brick_activity(h) : WS_OK;
 }
 // P2G in particle index order, or (p2gCellOrder) in cell order: with bricks
 // the mark pass counted and the brick list is current; the stage-wise call
@@ -847,6 +848,24 @@ static ws_status stage_p2g(ws_handle* h, bool bricks = false) {
   if (bricks) launch_faces_normalize_bc_bricks(h->d, grid_of(h), h->bricks, h->stream);
   else launch_faces_normalize_bc(h->d, grid_of(h), h->stream);
   return check_launch(h, n + 1);
+}
+// the substep's marking and P2G: one pass in index order without balls (the
+// balls push particles between the two, and the cell sort bins them first)
+static ws_status stage_mark_p2g(ws_handle* h) {
+  ws_status s;
+  if (h->nBalls || h->P.p2gCellOrder) {
+    if ((s = stage_mark(h, true))) return s;
+    if (h->nBalls) {
+      launch_ball_push(parts_of(h), h->balls, h->nBalls, h->stream);
+      if ((s = check_launch(h, h->S.nP ? 1 : 0))) return s;
+    }
+    return stage_p2g(h, true);
+  }
+  launch_mark_p2g(h->d, grid_of(h), parts_of(h), h->terr, h->S.oceanR, h->S.coreR, h->st, h->stream);
+  if ((s = check_launch(h, 1))) return s;
+  if ((s = brick_activity(h))) return s;
+  launch_faces_normalize_bc_bricks(h->d, grid_of(h), h->bricks, h->stream);
+  return check_launch(h, 1);
 }
 // planet gravity ramp, js/solver.js:2656-2662: the applied scale of this
 // substep (0 = no gravity), advancing the ramp timer
@@ -950,12 +969,7 @@ static ws_status enqueue_substep(ws_handle* h, double dt, double gsA) {
     launch_ball_raster(h->d, h->type, h->sv, true, h->balls, h->nBalls, grid_of(h), h->stream);
     if ((s = check_launch(h, h->nBalls ? 1 : 0))) return s;
   }
-  if ((s = stage_mark(h, true))) return s;
-  if (h->nBalls) {
-    launch_ball_push(parts_of(h), h->balls, h->nBalls, h->stream);
-    if ((s = check_launch(h, h->S.nP ? 1 : 0))) return s;
-  }
-  if ((s = stage_p2g(h, true))) return s;
+  if ((s = stage_mark_p2g(h))) return s;
   if ((s = stage_forces(h, dt, gsA, true))) return s;
   if ((s = stage_pressure(h, true))) return s;
   bool vort = h->P.vorticity > 0;

@@ -114,25 +114,43 @@ void launch_clear_raster(const Dims& d, const GridDev& g, DevStatus* st, bool cl
 
 // ------------------------------------------------------------ 2. mark fluid
 // _markFluidCells, js/solver.js:945-1000 (sphere). Bytes: 13P + N.
-// the cell a grid-coupled particle marks, or -1 (not coupled, or it turns airborne: pflag 1)
-__device__ __forceinline__ long long mark_cell(const Dims& d, const GridDev& g, PartsDev& P, const TerrainDev& t,
-                                               double oceanR, double coreR, int p, int fl, double X, double Y,
-                                               double Z) {
-  if (fl != 0) return -1;
+// The range and NaN latch of the marking on the stored float position: a
+// float exceeds the double bound exactly when it exceeds the largest float
+// not above it.
+__device__ __forceinline__ bool mark_sound_f(const Dims& d, float x, float y, float z, int* err) {
+  if (!(isfinite(x) && isfinite(y) && isfinite(z))) { atomicOr(err, WS_DERR_NAN); return false; }
+  if (x < 0.f || y < 0.f || z < 0.f || x > __double2float_rd(d.W) || y > __double2float_rd(d.H) ||
+      z > __double2float_rd(d.D)) atomicOr(err, WS_DERR_RANGE);
+  return true;
+}
+// whether a float position may pass the sky test's radius or row condition:
+// the float radius is within 1e-6 of the double one, so below the bound less
+// 1e-5 of it the double test cannot pass
+__device__ __forceinline__ bool mark_high_f(const Dims& d, double oceanR, float x, float y, float z, int j) {
+  const float rx = x - (float)d.cx, ry = y - (float)d.cy, rz = z - (float)d.cz;
+  const float bound = (float)((oceanR + 0.3) * (oceanR + 0.3) * (1 - 1e-5));
+  return !(rx * rx + ry * ry + rz * rz < bound) || j >= d.ny - 2;
+}
+// whether a grid-coupled particle in grid row j turns airborne
+__device__ __forceinline__ bool mark_airborne(const Dims& d, const GridDev& g, const TerrainDev& t, double oceanR,
+                                              double coreR, int j, double X, double Y, double Z) {
   double rx = X - d.cx, ry = Y - d.cy, rz = Z - d.cz;
   double radius2 = rx * rx + ry * ry + rz * rz;
   double skyAlt = 2 * d.dx > 0.3 ? 2 * d.dx : 0.3;
   if (radius2 > (oceanR + 0.3) * (oceanR + 0.3) &&
       sqrt(radius2) - terrain_radius_at(t, coreR, X, Y, Z) > skyAlt &&
-      !(t.has && rock_cell_at(d, g.staticTypes, X, Y, Z))) {
-    P.pflag[p] = 1; return -1;
-  }
+      !(t.has && rock_cell_at(d, g.staticTypes, X, Y, Z))) return true;
+  return j >= d.ny - 2 && sqrt(radius2) - terrain_radius_at(t, coreR, X, Y, Z) > 0.3;
+}
+// the cell a grid-coupled particle marks, or -1 (not coupled, or it turns airborne: pflag 1)
+__device__ __forceinline__ long long mark_cell(const Dims& d, const GridDev& g, PartsDev& P, const TerrainDev& t,
+                                               double oceanR, double coreR, int p, int fl, double X, double Y,
+                                               double Z) {
+  if (fl != 0) return -1;
   int i = jfloor_clamp(over_dx(d, X), 0, d.nx - 1);
   int j = jfloor_clamp(over_dx(d, Y), 0, d.ny - 1);
   int k = jfloor_clamp(over_dx(d, Z), 0, d.nz - 1);
-  if (j >= d.ny - 2) {
-    if (sqrt(radius2) - terrain_radius_at(t, coreR, X, Y, Z) > 0.3) { P.pflag[p] = 1; return -1; }
-  }
+  if (mark_airborne(d, g, t, oceanR, coreR, j, X, Y, Z)) { P.pflag[p] = 1; return -1; }
   return ((long long)k * d.ny + j) * d.nx + i;
 }
 // Warp-aggregated increment of count[key] for every lane with key >= 0: the
@@ -259,94 +277,174 @@ void launch_mark_fluid(const Dims& d, const GridDev& g, const PartsDev& P, const
 // face indices and fractions are exact (face_coords_f), the weights and
 // terms carry FP32 rounding (a few 1e-8 relative against the double sums).
 //
-// Runs of consecutive particles: each thread scatters four consecutive
-// particles (the fill's lattice runs along x about a third of a cell apart,
-// so three or four neighbours in index order usually share a stencil). Per
-// component, the particles' (momentum, weight) terms are summed in registers
-// while their stencils start at the same face, and each run sends one set of
-// eight float2 atomics.
-template <int COMP>
-__device__ __forceinline__ void p2g_run_comp(const Dims& d, float2* __restrict__ acc, const float (&x)[4],
-                                             const float (&y)[4], const float (&z)[4], const float (&v)[4],
+// Runs of consecutive particles: each thread scatters R (2 or 4) consecutive
+// particles (the fill's lattice runs along x about a third of a cell apart).
+// Per component it holds the eight (momentum, weight) sums of one stencil in
+// registers. A particle whose stencil starts at the same face adds to them;
+// one whose stencil starts one face further along x sends the four faces of
+// the column left behind and keeps the other four as its own first column;
+// any other sends all eight.
+//
+// In a whole substep without balls the fluid marking (section 2) rides along:
+// it needs the same positions, its arithmetic runs while the load/store units
+// are full of reductions, and P2G reads nothing that it writes.
+//
+// What bounds it: the reductions (lanes sent to L2). Before, with four
+// particles a thread, all eight faces sent at each new stencil, and the
+// marking as its own kernel: 106.6 + 22.3 us for 1.86M particles at 128^3,
+// 789 + 152 us for 15.3M at 256^3, 43.1 + 12.5 us for 0.7M at 97^3; now 90,
+// 612 and 34.5 us. Eight particles a thread hold too many registers (103, 660
+// and 47 us).
+template <int COMP, int R>
+__device__ __forceinline__ void p2g_run_comp(const Dims& d, float2* __restrict__ acc, const float (&x)[R],
+                                             const float (&y)[R], const float (&z)[R], const float (&v)[R],
                                              unsigned okMask) {
   unsigned sj, sk;
   face_strides32(d, COMP, sj, sk);
   const unsigned nx = (unsigned)d.nx, ny = (unsigned)d.ny, uN = (unsigned)d.uN, vN = (unsigned)d.vN;
-  float m8[8], w8[8];
+  float m8[8], w8[8];                                 // corner q: x + 2 y + 4 z
   unsigned cur = 0xffffffffu;
-#define WS_P2G_FLUSH                                                                         \
-  if (cur != 0xffffffffu) {                                                                  \
-    float2* p = acc + cur;                                                                   \
-    atomicAdd(p, make_float2(m8[0], w8[0]));                                                 \
-    atomicAdd(p + 1, make_float2(m8[1], w8[1]));                                             \
-    atomicAdd(p + sj, make_float2(m8[2], w8[2]));                                            \
-    atomicAdd(p + sj + 1, make_float2(m8[3], w8[3]));                                        \
-    atomicAdd(p + sk, make_float2(m8[4], w8[4]));                                            \
-    atomicAdd(p + sk + 1, make_float2(m8[5], w8[5]));                                        \
-    atomicAdd(p + sk + sj, make_float2(m8[6], w8[6]));                                       \
-    atomicAdd(p + sk + sj + 1, make_float2(m8[7], w8[7]));                                   \
-  }
+  auto send = [&](int col) {                          // the four faces of column col (0: lower x)
+    float2* p = acc + cur + col;
+    atomicAdd(p, make_float2(m8[col], w8[col]));
+    atomicAdd(p + sj, make_float2(m8[2 + col], w8[2 + col]));
+    atomicAdd(p + sk, make_float2(m8[4 + col], w8[4 + col]));
+    atomicAdd(p + sk + sj, make_float2(m8[6 + col], w8[6 + col]));
+  };
 #pragma unroll
-  for (int r = 0; r < 4; r++) {
+  for (int r = 0; r < R; r++) {
     if (!((okMask >> r) & 1u)) continue;
     int i0, j0, k0; float tx, ty, tz;
     face_coords_f(d, COMP, x[r], y[r], z[r], i0, j0, k0, tx, ty, tz);
     const unsigned idx = COMP == 0 ? ((unsigned)k0 * ny + (unsigned)j0) * (nx + 1) + (unsigned)i0
                        : COMP == 1 ? uN + ((unsigned)k0 * (ny + 1) + (unsigned)j0) * nx + (unsigned)i0
                                    : uN + vN + ((unsigned)k0 * ny + (unsigned)j0) * nx + (unsigned)i0;
+    if (idx != cur) {
+      const bool next = idx == cur + 1u && cur != 0xffffffffu;
+      if (cur != 0xffffffffu) {
+        send(0);
+        if (!next) send(1);
+      }
+#pragma unroll
+      for (int q = 0; q < 8; q += 2) {                // column 1 becomes column 0, or both start anew
+        m8[q] = next ? m8[q + 1] : 0.f; w8[q] = next ? w8[q + 1] : 0.f;
+        m8[q + 1] = 0.f; w8[q + 1] = 0.f;
+      }
+      cur = idx;
+    }
     const float s0 = 1.f - tx, s1 = tx, t0 = 1.f - ty, t1 = ty, r0 = 1.f - tz, r1 = tz;
     const float wA = s0 * t0, wB = s1 * t0, wC = s0 * t1, wD = s1 * t1;
     const float w[8] = { wA * r0, wB * r0, wC * r0, wD * r0, wA * r1, wB * r1, wC * r1, wD * r1 };
-    if (idx != cur) {
-      WS_P2G_FLUSH
-      cur = idx;
 #pragma unroll
-      for (int q = 0; q < 8; q++) { m8[q] = w[q] * v[r]; w8[q] = w[q]; }
+    for (int q = 0; q < 8; q++) { m8[q] = fmaf(w[q], v[r], m8[q]); w8[q] += w[q]; }
+  }
+  if (cur != 0xffffffffu) { send(0); send(1); }
+}
+// R consecutive values of a 16-byte aligned array (p0 a multiple of R), 0 past the end
+template <int R>
+__device__ __forceinline__ void load_run(const float* __restrict__ a, int p0, int n, float (&v)[R]) {
+  if (p0 + R <= n) {
+    if constexpr (R == 2) {
+      const float2 l = *reinterpret_cast<const float2*>(a + p0);
+      v[0] = l.x; v[1] = l.y;
     } else {
 #pragma unroll
-      for (int q = 0; q < 8; q++) { m8[q] = fmaf(w[q], v[r], m8[q]); w8[q] += w[q]; }
+      for (int q = 0; q < R; q += 4) {
+        const float4 l = *reinterpret_cast<const float4*>(a + p0 + q);
+        v[q] = l.x; v[q + 1] = l.y; v[q + 2] = l.z; v[q + 3] = l.w;
+      }
     }
-  }
-  WS_P2G_FLUSH
-#undef WS_P2G_FLUSH
-}
-__global__ void __launch_bounds__(256, 4) k_p2g_runs(Dims d, GridDev g, PartsDev P, int* err) {
-  const int p0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-  if (p0 >= P.nP) return;
-  float x[4], y[4], z[4], u[4], v[4], w[4];
-  int fl[4];
-  if (p0 + 3 < P.nP) {                                // the arrays are 16-byte aligned and p0 % 4 == 0
-    const float4 X = *reinterpret_cast<const float4*>(P.px + p0), Y = *reinterpret_cast<const float4*>(P.py + p0);
-    const float4 Z = *reinterpret_cast<const float4*>(P.pz + p0), U = *reinterpret_cast<const float4*>(P.pvx + p0);
-    const float4 V = *reinterpret_cast<const float4*>(P.pvy + p0), W = *reinterpret_cast<const float4*>(P.pvz + p0);
-    const uchar4 F = *reinterpret_cast<const uchar4*>(P.pflag + p0);
-    x[0] = X.x; x[1] = X.y; x[2] = X.z; x[3] = X.w; y[0] = Y.x; y[1] = Y.y; y[2] = Y.z; y[3] = Y.w;
-    z[0] = Z.x; z[1] = Z.y; z[2] = Z.z; z[3] = Z.w; u[0] = U.x; u[1] = U.y; u[2] = U.z; u[3] = U.w;
-    v[0] = V.x; v[1] = V.y; v[2] = V.z; v[3] = V.w; w[0] = W.x; w[1] = W.y; w[2] = W.z; w[3] = W.w;
-    fl[0] = F.x; fl[1] = F.y; fl[2] = F.z; fl[3] = F.w;
   } else {
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const int p = p0 + r;
-      const bool has = p < P.nP;
-      x[r] = has ? P.px[p] : 0.f; y[r] = has ? P.py[p] : 0.f; z[r] = has ? P.pz[p] : 0.f;
-      u[r] = has ? P.pvx[p] : 0.f; v[r] = has ? P.pvy[p] : 0.f; w[r] = has ? P.pvz[p] : 0.f;
-      fl[r] = has ? P.pflag[p] : 1;
-    }
+    for (int r = 0; r < R; r++) v[r] = p0 + r < n ? a[p0 + r] : 0.f;
   }
+}
+// The marking of one thread's R particles (as k_mark_fluid): range and
+// NaN latch, seed bricks, the sky test, fluid cells. The cell types of this
+// substep are the static ones and what this pass marks (no balls), so a cell
+// is marked when its static type is air. Particles that turn airborne leave
+// fl. The cell of a float position: with a power-of-two cell size the scaled
+// position and its floor are exact in float (face_coords_f).
+template <int R>
+__device__ __forceinline__ void mark_run(const Dims& d, const GridDev& g, const PartsDev& P, const TerrainDev& t, double oceanR,
+                                      double coreR, int p0, const float (&x)[R], const float (&y)[R],
+                                      const float (&z)[R], int (&fl)[R], int* err) {
+  const float rd = (float)d.rdx;
+  int lastBrick = -1;
+  long long lastCell = -1;
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    if (p0 + r >= P.nP) continue;
+    mark_sound_f(d, x[r], y[r], z[r], err);
+    int i, j, k;
+    if (d.dxPow2) {
+      i = min(max((int)floorf(x[r] * rd), 0), d.nx - 1); j = min(max((int)floorf(y[r] * rd), 0), d.ny - 1);
+      k = min(max((int)floorf(z[r] * rd), 0), d.nz - 1);
+    } else {
+      i = jfloor_clamp((double)x[r] / d.dx, 0, d.nx - 1); j = jfloor_clamp((double)y[r] / d.dx, 0, d.ny - 1);
+      k = jfloor_clamp((double)z[r] / d.dx, 0, d.nz - 1);
+    }
+    const int sb = ((k >> 2) * g.nby + (j >> 2)) * g.nbx + (i >> 2);
+    if (sb != lastBrick) { g.seed[sb] = 1; lastBrick = sb; }
+    if (fl[r] != 0) continue;
+    if (mark_high_f(d, oceanR, x[r], y[r], z[r], j) &&
+        mark_airborne(d, g, t, oceanR, coreR, j, x[r], y[r], z[r])) { P.pflag[p0 + r] = 1; fl[r] = 1; continue; }
+    const long long c = ((long long)k * d.ny + j) * d.nx + i;
+    if (c != lastCell) { lastCell = c; if (g.staticTypes[c] == WS_AIR) g.type[c] = WS_FLUID; }
+  }
+}
+template <bool MARK, int R>
+__global__ void __launch_bounds__(128, 8) k_p2g_runs(Dims d, GridDev g, PartsDev P, TerrainDev t, double oceanR,
+                                                     double coreR, int* err) {
+  const int p0 = R * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (p0 >= P.nP) return;
+  float x[R], y[R], z[R], v[R];
+  int fl[R];
+  load_run<R>(P.px, p0, P.nP, x); load_run<R>(P.py, p0, P.nP, y); load_run<R>(P.pz, p0, P.nP, z);
+  if (R == 4 && p0 + R <= P.nP) {
+    const unsigned F = *reinterpret_cast<const unsigned*>(P.pflag + p0);
+#pragma unroll
+    for (int r = 0; r < R; r++) fl[r] = (int)((F >> (8 * r)) & 0xffu);
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; r++) fl[r] = p0 + r < P.nP ? P.pflag[p0 + r] : 1;
+  }
+  if (MARK) mark_run<R>(d, g, P, t, oceanR, coreR, p0, x, y, z, fl, err);
   // a fluid particle with a non-finite state is left out of the grid and latched
   unsigned ok = 0;
 #pragma unroll
-  for (int r = 0; r < 4; r++)
-    if (fl[r] == 0 && particle_sound_f(x[r], y[r], z[r], u[r], v[r], w[r], err)) ok |= 1u << r;
+  for (int r = 0; r < R; r++)
+    if (fl[r] == 0) ok |= 1u << r;
   if (!ok) return;
-  p2g_run_comp<0>(d, g.acc, x, y, z, u, ok);
-  p2g_run_comp<1>(d, g.acc, x, y, z, v, ok);
-  p2g_run_comp<2>(d, g.acc, x, y, z, w, ok);
+  {
+    float vy[R], vz[R];
+    load_run<R>(P.pvx, p0, P.nP, v); load_run<R>(P.pvy, p0, P.nP, vy); load_run<R>(P.pvz, p0, P.nP, vz);
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      if (((ok >> r) & 1u) && !particle_sound_f(x[r], y[r], z[r], v[r], vy[r], vz[r], err)) ok &= ~(1u << r);
+  }
+  p2g_run_comp<0, R>(d, g.acc, x, y, z, v, ok);
+  load_run<R>(P.pvy, p0, P.nP, v);                          // from L1: fewer registers than keeping all three
+  p2g_run_comp<1, R>(d, g.acc, x, y, z, v, ok);
+  load_run<R>(P.pvz, p0, P.nP, v);
+  p2g_run_comp<2, R>(d, g.acc, x, y, z, v, ok);
+}
+template <bool MARK>
+static void launch_p2g_runs(const Dims& d, const GridDev& g, const PartsDev& P, const TerrainDev& t, double oceanR,
+                            double coreR, int* err, cudaStream_t s) {
+  if (P.nP <= 0) return;
+  // four particles a thread send fewer reductions, two leave more threads and
+  // shorter chains (R = 4 against 2 in us: 10k particles 11.6/6.1, 0.7M
+  // 37.5/34.5, 1.86M 90.1/90.4, 15.3M 612/647)
+  if (P.nP < (3 << 19)) k_p2g_runs<MARK, 2><<<grid_for((P.nP + 1LL) / 2, 128), 128, 0, s>>>(d, g, P, t, oceanR, coreR, err);
+  else k_p2g_runs<MARK, 4><<<grid_for((P.nP + 3LL) / 4, 128), 128, 0, s>>>(d, g, P, t, oceanR, coreR, err);
 }
 void launch_p2g(const Dims& d, const GridDev& g, const PartsDev& P, DevStatus* st, cudaStream_t s) {
-  if (P.nP <= 0) return;
-  k_p2g_runs<<<grid_for((P.nP + 3) / 4, 256), 256, 0, s>>>(d, g, P, &st->err);
+  launch_p2g_runs<false>(d, g, P, TerrainDev{}, 0, 0, &st->err, s);
+}
+void launch_mark_p2g(const Dims& d, const GridDev& g, const PartsDev& P, const TerrainDev& t, double oceanR, double coreR,
+                     DevStatus* st, cudaStream_t s) {
+  launch_p2g_runs<true>(d, g, P, t, oceanR, coreR, &st->err, s);
 }
 
 // ------------------------------------------------------------ 3b. P2G in cell order

@@ -38,6 +38,9 @@ void launch_extrapolate_bricks(const Dims& d, const GridDev& g, const BrickSet& 
 void launch_mark_fluid(const Dims& d, const GridDev& g, const PartsDev& P, const TerrainDev& t,
                        double oceanR, double coreR, const CellSort* cs, DevStatus* st, cudaStream_t s);
 void launch_p2g(const Dims& d, const GridDev& g, const PartsDev& P, DevStatus* st, cudaStream_t s);
+// the fluid marking and P2G in index order in one pass (a substep without balls)
+void launch_mark_p2g(const Dims& d, const GridDev& g, const PartsDev& P, const TerrainDev& t, double oceanR, double coreR,
+                     DevStatus* st, cudaStream_t s);
 size_t cell_sort_scratch_bytes(long long nKeys);
 int launch_p2g_sorted(const Dims& d, const GridDev& g, const PartsDev& P, const CellSort& cs, const BrickSet& B,
                       bool binned, void* scratch, size_t scratchBytes, DevStatus* st, cudaStream_t s);

@@ -214,7 +214,7 @@ static void free_all(ws_handle* h) {
   if (h->mtScratch) cudaFree(h->mtScratch);
   if (h->queryBuf) cudaFree(h->queryBuf);
   {
-    void* bb[] = { h->bricks.seed, h->bricks.act, h->bricks.proc, h->bricks.list, h->bricks.count, h->bricks.forceAll, h->bricks.fmask,
+    void* bb[] = { h->bricks.seed, h->bricks.act, h->bricks.list, h->bricks.count, h->bricks.forceAll, h->bricks.fmask,
                    h->csort.count, h->csort.start, h->csort.pcell, h->csort.pslot,
                    h->csort.perm, h->csortCub };
     for (void* b : bb) if (b) cudaFree(b);
@@ -309,16 +309,16 @@ extern "C" ws_status ws_create(const ws_config* cfg, ws_handle** out) {
     B.nbx = (d.nx + 3) / 4; B.nby = (d.ny + 3) / 4; B.nbz = (d.nz + 3) / 4;
     B.dnbx = fastdiv_make((unsigned)B.nbx); B.dnby = fastdiv_make((unsigned)B.nby);
     const long long nB = (long long)B.nbx * B.nby * B.nbz;
-    AL(B.seed, nB) AL(B.act, nB) AL(B.proc, nB) AL(B.list, nB) AL(B.count, 1) AL(B.forceAll, 1) AL(B.fmask, nB)
+    AL(B.seed, nB) AL(B.act, nB) AL(B.list, nB) AL(B.count, 2) AL(B.forceAll, 2) AL(B.fmask, nB)
     CellSort& cs = h->csort;
     AL(cs.count, 64 * nB + 1) AL(cs.start, 64 * nB + 1) AL(cs.pcell, P) AL(cs.pslot, P) AL(cs.perm, P)
     cs.cap = (int)P;
     h->csortCubBytes = cell_sort_scratch_bytes(64 * nB);
     if ((e = cudaMalloc(&h->csortCub, h->csortCubBytes)) != cudaSuccess) { ws_status r = fail_cuda(h, e, "cudaMalloc"); free_all(h); delete h; return r; }
-    const int one = 1;
+    const int one[2] = { 1, 0 };
     if ((e = cudaMemset(B.seed, 0, (size_t)nB)) != cudaSuccess || (e = cudaMemset(B.act, 0, (size_t)nB)) != cudaSuccess ||
-        (e = cudaMemset(B.count, 0, sizeof(int))) != cudaSuccess ||
-        (e = cudaMemcpy(B.forceAll, &one, sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess) {
+        (e = cudaMemset(B.count, 0, 2 * sizeof(int))) != cudaSuccess ||
+        (e = cudaMemcpy(B.forceAll, one, sizeof(one), cudaMemcpyHostToDevice)) != cudaSuccess) {
       ws_status r = fail_cuda(h, e, "brick state"); free_all(h); delete h; return r;
     }
   }
@@ -501,7 +501,9 @@ extern "C" ws_status ws_upload_field(ws_handle* h, ws_field f, const void* host,
   if (count < 0 || count > r.count) return fail(h, WS_ERR_RANGE, "count exceeds the field size");
   if (r.kind != 0) return fail(h, WS_ERR_INVALID, "derived field is read-only");
   WS_TRY(cudaMemcpyAsync(r.ptr, host, (size_t)count * r.elem, cudaMemcpyHostToDevice, h->stream));
-  if (f >= WS_F_CELLTYPE) force_full_pass(h);          // a grid field: rewrite every brick next substep
+  // a grid field: rewrite every brick next substep (of q, the pressure setup alone)
+  if (f == WS_F_Q) WS_TRY(cudaMemsetAsync(h->bricks.forceAll + 1, 1, sizeof(int), h->stream));
+  else if (f >= WS_F_CELLTYPE) force_full_pass(h);
   WS_TRY(cudaStreamSynchronize(h->stream));
   if (f == WS_F_PFLAG && !h->vaporPossible && any_vapor_flag((const uint8_t*)host, count))
     h->vaporPossible = true;
@@ -815,14 +817,12 @@ static AdvectParams advect_params(ws_handle* h, double dt) {
 // over the active-brick list; a stage called on its own runs over the whole
 // grid and forces the next substep to process every brick.
 static ws_status stage_clear_raster(ws_handle* h, bool bricks = false) {
-  launch_clear_raster(h->d, grid_of(h), h->st, !bricks, h->stream);
-  if (bricks) launch_clear_acc_bricks(h->d, grid_of(h), h->bricks, h->stream);
-  return check_launch(h, bricks ? 2 : 1);
+  launch_clear_raster(h->d, grid_of(h), h->st, h->bricks, bricks, h->stream);
+  return check_launch(h, 1);
 }
 // the active-brick list from this substep's seeds
 static ws_status brick_activity(ws_handle* h) {
-  cudaError_t e = launch_brick_activity(h->bricks, h->stream);
-  if (e != cudaSuccess) return fail_cuda(h, e, "active bricks");
+  launch_brick_activity(h->bricks, h->stream);
   return check_launch(h, 1);
 }
 // bricks: the substep's own pipeline, where (with p2gCellOrder) the mark
@@ -845,8 +845,7 @@ static ws_status stage_p2g(ws_handle* h, bool bricks = false) {
   } else {
     launch_p2g(h->d, grid_of(h), parts_of(h), h->st, h->stream);
   }
-  if (bricks) launch_faces_normalize_bc_bricks(h->d, grid_of(h), h->bricks, h->stream);
-  else launch_faces_normalize_bc(h->d, grid_of(h), h->stream);
+  launch_faces_normalize_bc(h->d, grid_of(h), h->bricks, !bricks, h->stream);
   return check_launch(h, n + 1);
 }
 // the substep's marking and P2G: one pass in index order without balls (the
@@ -864,7 +863,7 @@ static ws_status stage_mark_p2g(ws_handle* h) {
   launch_mark_p2g(h->d, grid_of(h), parts_of(h), h->terr, h->S.oceanR, h->S.coreR, h->st, h->stream);
   if ((s = check_launch(h, 1))) return s;
   if ((s = brick_activity(h))) return s;
-  launch_faces_normalize_bc_bricks(h->d, grid_of(h), h->bricks, h->stream);
+  launch_faces_normalize_bc(h->d, grid_of(h), h->bricks, false, h->stream);
   return check_launch(h, 1);
 }
 // planet gravity ramp, js/solver.js:2656-2662: the applied scale of this
@@ -878,8 +877,7 @@ static ws_status stage_forces(ws_handle* h, double dt, double gsA, bool bricks =
   double nu = h->P.viscosity;
   double coef = std::min(nu * dt / (h->d.dx * h->d.dx), 0.24);
   int viscOn = nu > 1e-6;
-  if (bricks) launch_faces_forces_bricks(h->d, grid_of(h), h->bricks, coef, viscOn, dt, gsA, h->stream);
-  else launch_faces_forces(h->d, grid_of(h), coef, viscOn, dt, gsA, h->stream);
+  launch_faces_forces(h->d, grid_of(h), h->bricks, !bricks, coef, viscOn, dt, gsA, h->stream);
   return check_launch(h, 1);
 }
 // _pressureSolve: setup (diag, rhs, q = 0 off the fluid) then the whole SOR
@@ -892,7 +890,6 @@ static ws_status stage_pressure(ws_handle* h, bool bricks = false) {
   bool tolMode = h->P.sorTol > 0;
   int iters = tolMode ? h->P.sorMaxIters : h->P.pressureIters;
   int check = tolMode ? (h->P.sorCheckEvery > 0 ? h->P.sorCheckEvery : 1) : 0;
-  int* dIters = nullptr; double* dRel = nullptr; int* dPath = nullptr;
   cudaError_t e;
   if (h->net && h->unetCollect) {
     if ((e = h->net->collect_pre(h->q, h->rhs, h->diag8, h->type, h->stream)) != cudaSuccess)
@@ -903,13 +900,9 @@ static ws_status stage_pressure(ws_handle* h, bool bricks = false) {
       return fail_cuda(h, e, "learned warm start");
     h->launches += 23;
   }
-  e = launch_sor_solve(h->sor, h->d, g, h->diag8, h->P.omega, iters, check, h->P.sorTol, h->st, &dIters, &dRel, &dPath,
-                       h->stream);
+  e = launch_sor_solve(h->sor, h->d, g, h->diag8, h->P.omega, iters, check, h->P.sorTol, h->st, true, h->stream);
   if (e != cudaSuccess) return fail_cuda(h, e, "SOR solve launch");
   s = check_launch(h, sor_solve_launches(h->sor)); if (s) return s;
-  WS_TRY(cudaMemcpyAsync(&h->st->sorIters, dIters, sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
-  WS_TRY(cudaMemcpyAsync(&h->st->relres, dRel, sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-  WS_TRY(cudaMemcpyAsync(&h->st->pad2, dPath, sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
   if (h->net && h->unetCollect) {
     if ((e = h->net->collect_post(h->q, h->stream)) != cudaSuccess) return fail_cuda(h, e, "warm-start pair (after the solve)");
   }
@@ -929,8 +922,7 @@ static void pull_substep(ws_handle* h) {
   h->S.airborneCount = h->stHost->airborne;
 }
 static ws_status stage_project(ws_handle* h, bool clampToo, bool bricks = false) {
-  if (bricks) launch_project_bricks(h->d, grid_of(h), h->bricks, clampToo ? 1 : 0, h->P.maxSpeed, h->st, h->stream);
-  else launch_project(h->d, grid_of(h), clampToo ? 1 : 0, h->P.maxSpeed, h->st, h->stream);
+  launch_project(h->d, grid_of(h), h->bricks, !bricks, clampToo ? 1 : 0, h->P.maxSpeed, h->st, h->stream);
   return check_launch(h, 1);
 }
 static ws_status stage_vorticity(ws_handle* h, double dt) {
@@ -943,8 +935,7 @@ static ws_status stage_clamp(ws_handle* h) {
   return check_launch(h, 1);
 }
 static ws_status stage_extrapolate(ws_handle* h, bool bricks = false) {
-  if (bricks) launch_extrapolate_bricks(h->d, grid_of(h), h->bricks, h->stream);
-  else launch_extrapolate(h->d, grid_of(h), h->stream);
+  launch_extrapolate(h->d, grid_of(h), h->bricks, !bricks, h->stream);
   return check_launch(h, 1);
 }
 static ws_status stage_g2p_advect(ws_handle* h, double dt) {
@@ -1549,25 +1540,23 @@ extern "C" ws_status ws_time_kernel(ws_handle* h, int32_t kernel, int32_t reps, 
       case 1: launch_p2g(h->d, g, parts_of(h), h->st, h->stream); break;
       case 2: { AdvectParams ap = advect_params(h, h->S.dtLast > 0 ? h->S.dtLast : 0.01);
                 launch_g2p_advect(h->d, g, parts_of(h), h->terr, ap, h->st, h->stream); } break;
-      case 3: launch_faces_normalize_bc(h->d, g, h->stream); break;
-      case 4: launch_faces_forces(h->d, g, 5e-6, 1, 0.01, 9.81, h->stream); break;
-      case 5: launch_project(h->d, g, 1, h->P.maxSpeed, h->st, h->stream); break;
-      case 6: { int* di; double* dr; int* dp;
-                cudaError_t e6 = launch_sor_solve(h->sor, h->d, g, h->diag8, h->P.omega, h->P.pressureIters, 0, 0,
-                                                  h->st, &di, &dr, &dp, h->stream);
+      case 3: launch_faces_normalize_bc(h->d, g, h->bricks, true, h->stream); break;
+      case 4: launch_faces_forces(h->d, g, h->bricks, true, 5e-6, 1, 0.01, 9.81, h->stream); break;
+      case 5: launch_project(h->d, g, h->bricks, true, 1, h->P.maxSpeed, h->st, h->stream); break;
+      case 6: { cudaError_t e6 = launch_sor_solve(h->sor, h->d, g, h->diag8, h->P.omega, h->P.pressureIters, 0, 0,
+                                                  h->st, false, h->stream);
                 if (e6 != cudaSuccess) { cudaEventDestroy(e0); cudaEventDestroy(e1); return fail_cuda(h, e6, "SOR solve"); }
                 h->launches += sor_solve_launches(h->sor) - 1; } break;   // list build; timed per whole solve
-      case 8: launch_faces_normalize_bc_bricks(h->d, g, h->bricks, h->stream); break;
-      case 9: launch_faces_forces_bricks(h->d, g, h->bricks, 5e-6, 1, 0.01, 9.81, h->stream); break;
-      case 10: launch_project_bricks(h->d, g, h->bricks, 1, h->P.maxSpeed, h->st, h->stream); break;
-      case 11: launch_extrapolate_bricks(h->d, g, h->bricks, h->stream); break;
+      case 8: launch_faces_normalize_bc(h->d, g, h->bricks, false, h->stream); break;
+      case 9: launch_faces_forces(h->d, g, h->bricks, false, 5e-6, 1, 0.01, 9.81, h->stream); break;
+      case 10: launch_project(h->d, g, h->bricks, false, 1, h->P.maxSpeed, h->st, h->stream); break;
+      case 11: launch_extrapolate(h->d, g, h->bricks, false, h->stream); break;
       case 12: { const int n12 = launch_p2g_sorted(h->d, g, parts_of(h), h->csort, h->bricks, false, h->csortCub,
                                                    h->csortCubBytes, h->st, h->stream);
                  if (n12 < 0) { cudaEventDestroy(e0); cudaEventDestroy(e1); return fail_cuda(h, cudaGetLastError(), "cell sort"); }
                  h->launches += n12 - 1; } break;
-      case 7: { int* di; double* dr; int* dp;
-                cudaError_t e7 = launch_sor_solve_lists(h->sor, h->d, g, h->diag8, h->P.omega, h->P.pressureIters, 0, 0,
-                                                        h->st, &di, &dr, &dp, h->stream);
+      case 7: { cudaError_t e7 = launch_sor_solve_lists(h->sor, h->d, g, h->diag8, h->P.omega, h->P.pressureIters, 0, 0,
+                                                        h->st, false, h->stream);
                 if (e7 != cudaSuccess) { cudaEventDestroy(e0); cudaEventDestroy(e1); return fail_cuda(h, e7, "SOR solve"); }
                 h->launches += sor_list_solve_launches(h->sor) - 1; } break;
       default: cudaEventDestroy(e0); cudaEventDestroy(e1); return fail(h, WS_ERR_INVALID, "unknown kernel id");
@@ -1580,6 +1569,7 @@ extern "C" ws_status ws_time_kernel(ws_handle* h, int32_t kernel, int32_t reps, 
   cudaEventElapsedTime(&ms, e0, e1);
   cudaEventDestroy(e0); cudaEventDestroy(e1);
   *us = 1000.0 * ms / (reps * perRep);
+  force_full_pass(h);                            // the timed passes reset the flags
   return sync_status(h);
 }
 

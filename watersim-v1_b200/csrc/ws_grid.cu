@@ -95,21 +95,60 @@ void launch_gravity_geometry(const Dims& d, double oceanR, float* g, cudaStream_
 // u..wW.fill(0) (js/solver.js:2569-2570) and cellType <- static types
 // (:865-871). Bytes: 8F (acc) + 2N.
 // 16-byte stores: two faces of the accumulator, sixteen cell types per
-// thread (both buffers are separate allocations, 256-byte aligned).
-__global__ void k_clear_raster(Dims d, GridDev g, DevStatus* st, int clearAcc) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long F2 = d.F >> 1, n16 = d.nCells >> 4;
-  if (clearAcc) {
-    if (t < F2) reinterpret_cast<float4*>(g.acc)[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-    else if (t == F2 && (d.F & 1)) g.acc[d.F - 1] = make_float2(0.f, 0.f);
-  }
-  if (t < n16) reinterpret_cast<uint4*>(g.type)[t] = reinterpret_cast<const uint4*>(g.staticTypes)[t];
-  else if (t < n16 + (d.nCells & 15)) { const long long c = (n16 << 4) + (t - n16); g.type[c] = g.staticTypes[c]; }
-  if (t == 0) { st->umaxBits = 0u; st->airborne = 0; st->nFluid = 0; st->oddFluid = 0; }
+// thread (both buffers are separate allocations, 256-byte aligned). In a
+// substep (bricks) only the accumulator of the last substep's work list is
+// cleared, unless a forced full pass follows; the list's counter starts anew.
+__device__ __forceinline__ unsigned cell_faces(const Dims& d, int i, int j, int k, unsigned (&f)[3]) {
+  const unsigned nx = (unsigned)d.nx, ny = (unsigned)d.ny, row = (unsigned)k * ny + (unsigned)j;
+  const unsigned c = row * nx + (unsigned)i;
+  f[0] = c + row;                                       // u: rows of nx + 1
+  f[1] = (unsigned)d.uN + c + (unsigned)k * nx;         // v: planes of ny + 1 rows
+  f[2] = (unsigned)(d.uN + d.vN) + c;
+  return c;
 }
-void launch_clear_raster(const Dims& d, const GridDev& g, DevStatus* st, bool clearAcc, cudaStream_t s) {
-  const long long a = clearAcc ? (d.F >> 1) + 1 : 0, b = (d.nCells >> 4) + 16;
-  k_clear_raster<<<grid_for(a > b ? a : b, 256), 256, 0, s>>>(d, g, st, clearAcc ? 1 : 0);
+// A block of 256 threads on four bricks of the work list: the list holds
+// x-neighbours side by side, so a warp takes two y rows of all four (32 cells
+// along x by 2 lie in 2 to 4 lines) rather than half of one brick (8 rows of
+// 16 bytes). The brick's number among the four, and the cell in the brick.
+__device__ __forceinline__ void quad_cell(int& q, int& li, int& lj, int& lk) {
+  const int t = threadIdx.x;
+  li = t & 3; q = (t >> 2) & 3; lj = ((t >> 4) & 1) | ((t >> 4) & 2); lk = t >> 6;
+}
+__global__ void __launch_bounds__(256) k_clear_raster(Dims d, GridDev g, DevStatus* st, BrickSet B, int bricks) {
+  const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  const long long F2 = d.F >> 1, n16 = d.nCells >> 4;
+  for (long long t = t0; t < n16; t += step)
+    reinterpret_cast<uint4*>(g.type)[t] = reinterpret_cast<const uint4*>(g.staticTypes)[t];
+  if (t0 < (d.nCells & 15)) { const long long c = (n16 << 4) + t0; g.type[c] = g.staticTypes[c]; }
+  if (t0 == 0) {
+    st->umaxBits = 0u; st->airborne = 0; st->nFluid = 0; st->oddFluid = 0;
+    if (bricks) B.count[0] = 0;
+  }
+  if (!bricks || *B.forceAll) {
+    for (long long t = t0; t < F2; t += step) reinterpret_cast<float4*>(g.acc)[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t0 == 0 && (d.F & 1)) g.acc[d.F - 1] = make_float2(0.f, 0.f);
+    return;
+  }
+  const int n = B.count[1];                             // the last substep's list
+  int q, li, lj, lk;
+  quad_cell(q, li, lj, lk);
+  for (int it = blockIdx.x * 4 + q; it < n; it += gridDim.x * 4) {
+    int bx, by, bz;
+    brick_coords(B, B.list[it], bx, by, bz);
+    const int i = bx * 4 + li, j = by * 4 + lj, k = bz * 4 + lk;
+    if (i >= d.nx || j >= d.ny || k >= d.nz) continue;
+    unsigned f[3];
+    cell_faces(d, i, j, k, f);
+#pragma unroll
+    for (int a = 0; a < 3; a++) g.acc[f[a]] = make_float2(0.f, 0.f);
+    if (i == d.nx - 1) g.acc[f[0] + 1] = make_float2(0.f, 0.f);
+    if (j == d.ny - 1) g.acc[f[1] + d.nx] = make_float2(0.f, 0.f);
+    if (k == d.nz - 1) g.acc[f[2] + d.nx * d.ny] = make_float2(0.f, 0.f);
+  }
+}
+void launch_clear_raster(const Dims& d, const GridDev& g, DevStatus* st, const BrickSet& B, bool bricks, cudaStream_t s) {
+  const unsigned need = grid_for(bricks ? (d.nCells >> 4) + 16 : (d.F >> 1) + 16, 256);
+  k_clear_raster<<<std::min(std::max(need, 148u * 2u), 148u * 8u), 256, 0, s>>>(d, g, st, B, bricks ? 1 : 0);
 }
 
 // ------------------------------------------------------------ 2. mark fluid
@@ -601,83 +640,6 @@ int launch_p2g_sorted(const Dims& d, const GridDev& g, const PartsDev& P, const 
   return launches + 2;
 }
 
-// Solid-adjacent interior face: the velocity of the solid cell beside it,
-// the left one first (_applyBCSlice, js/solver.js:1153-1170): 0 for rock and
-// the domain shell, the ball's velocity for a ball cell.
-__device__ __forceinline__ float solid_face_velocity(const Dims& d, const GridDev& g, int comp, long long cL, long long cR) {
-  if (!g.sv) return 0.f;
-  const long long c = g.type[cL] == WS_SOLID ? cL : cR;
-  return g.sv[comp * d.nCells + c];
-}
-
-// ------------------------------------------------------------ 4. faces pass 1
-// _p2gNormalizeFace (:1109-1120) + _applyBC (:1130-1171)
-// + FLIP snapshot (:2579) + the extrapolation valid mark (:1578-1611).
-// Bytes: 8F read + 4F vel + 4F velO + 1F valid + 2 type reads per face.
-__device__ __forceinline__ void face_normalize_bc(const Dims& d, const GridDev& g, long long f, const FaceIJK& F) {
-  float2 a = g.acc[f];
-  float u = a.x;
-  if ((double)a.y > 1e-8) u = (float)((double)a.x / (double)a.y);
-  long long cL = 0, cR = 0;
-  bool solidAdj = face_cells(d, F, cL, cR);
-  if (solidAdj) u = 0.f;                                   // domain boundary plane
-  else if (g.type[cL] == WS_SOLID || g.type[cR] == WS_SOLID) { solidAdj = true; u = solid_face_velocity(d, g, F.comp, cL, cR); }
-  g.vel[f] = u;
-  g.velO[f] = u;
-  g.valid[f] = ((double)a.y > 1e-8 || solidAdj) ? 1 : 0;
-}
-__global__ void k_faces_normalize_bc(Dims d, GridDev g) {
-  long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (f >= d.F) return;
-  face_normalize_bc(d, g, f, decode_face(d, f));
-}
-void launch_faces_normalize_bc(const Dims& d, const GridDev& g, cudaStream_t s) {
-  k_faces_normalize_bc<<<grid_for(d.F, 256), 256, 0, s>>>(d, g);
-}
-
-// ------------------------------------------------------------ 5. forces
-// _viscosity (:1259-1304, Jacobi: neighbours from the snapshot, which equals
-// the post-BC field on entry), planet gravity (:1229-1256 with the ramp of
-// :2656-2662 applied by the caller in gs) and the BC again (:2598).
-__device__ __forceinline__ void face_forces(const Dims& d, const GridDev& g, long long f, const FaceIJK& F, double coef,
-                                            int viscOn, double dt, double gs) {
-  long long cL = 0, cR = 0;
-  if (face_cells(d, F, cL, cR)) { g.vel[f] = 0.f; return; }
-  int tL = g.type[cL], tR = g.type[cR];
-  if (tL == WS_SOLID || tR == WS_SOLID) { g.vel[f] = solid_face_velocity(d, g, F.comp, cL, cR); return; }
-  const float* __restrict__ o = g.velO;
-  float u = o[f];
-  if (viscOn && tL == WS_FLUID && tR == WS_FLUID) {
-    int nx = d.nx, ny = d.ny, nz = d.nz;
-    long long sI = 1, sJ, sK; int iLo, iHi, jLo, jHi, kLo, kHi;
-    if (F.comp == 0) { sJ = nx + 1; sK = (long long)ny * (nx + 1);
-      iLo = F.i - 1 >= 0; iHi = F.i + 1 <= nx; jLo = F.j - 1 >= 0; jHi = F.j + 1 < ny; kLo = F.k - 1 >= 0; kHi = F.k + 1 < nz; }
-    else if (F.comp == 1) { sJ = nx; sK = (long long)(ny + 1) * nx;
-      iLo = F.i - 1 >= 0; iHi = F.i + 1 < nx; jLo = F.j - 1 >= 0; jHi = F.j + 1 <= ny; kLo = F.k - 1 >= 0; kHi = F.k + 1 < nz; }
-    else { sJ = nx; sK = (long long)ny * nx;
-      iLo = F.i - 1 >= 0; iHi = F.i + 1 < nx; jLo = F.j - 1 >= 0; jHi = F.j + 1 < ny; kLo = F.k - 1 >= 0; kHi = F.k + 1 <= nz; }
-    double c0 = o[f];
-    double val = c0 * 6;
-    val -= iLo ? (double)o[f - sI] : c0;
-    val -= iHi ? (double)o[f + sI] : c0;
-    val -= jLo ? (double)o[f - sJ] : c0;
-    val -= jHi ? (double)o[f + sJ] : c0;
-    val -= kLo ? (double)o[f - sK] : c0;
-    val -= kHi ? (double)o[f + sK] : c0;
-    u = (float)(c0 + coef * val);
-  }
-  if (gs > 0 && (tL == WS_FLUID || tR == WS_FLUID)) u = (float)((double)u + (double)g.gvel[f] * dt * gs);
-  g.vel[f] = u;
-}
-__global__ void k_faces_forces(Dims d, GridDev g, double coef, int viscOn, double dt, double gs) {
-  long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (f >= d.F) return;
-  face_forces(d, g, f, decode_face(d, f), coef, viscOn, dt, gs);
-}
-void launch_faces_forces(const Dims& d, const GridDev& g, double coef, int viscOn, double dt, double gs, cudaStream_t s) {
-  k_faces_forces<<<grid_for(d.F, 256), 256, 0, s>>>(d, g, coef, viscOn, dt, gs);
-}
-
 // ------------------------------------------------------------ 6. pressure setup
 // _pressureSolve passes 1-2, js/solver.js:1321-1366: q = 0 off the fluid,
 // diag = Nf + Na, rhs = -dx^2 div, relaxation weight pw = omega/diag
@@ -686,25 +648,31 @@ void launch_faces_forces(const Dims& d, const GridDev& g, double coef, int viscO
 // of interior fluid cells, from which the solve builds its plan.
 // one cell of the setup: returns whether it is fluid and its SOR colour (-1 off the lists)
 __device__ __forceinline__ bool cell_pressure_setup(const Dims& d, const GridDev& g, uint8_t* __restrict__ diag8,
-                                                    double omega, long long c, int i, int j, int k, int& col) {
+                                                    double omega, unsigned c, int i, int j, int k, int& col) {
   col = -1;
-  const uint8_t* type = g.type;
-  if (type[c] != WS_FLUID) { g.q[c] = 0.f; g.pw[c] = -1.f; diag8[c] = 0; return false; }
-  int nx = d.nx, ny = d.ny, nz = d.nz; long long nxy = (long long)nx * ny;
-  long long nbr[6] = { i > 0 ? c - 1 : -1, i < nx - 1 ? c + 1 : -1, j > 0 ? c - nx : -1,
-                       j < ny - 1 ? c + nx : -1, k > 0 ? c - nxy : -1, k < nz - 1 ? c + nxy : -1 };
+  // every load in one round trip: most cells of a listed brick are not fluid,
+  // but their loads share lines with those that are
+  const unsigned nx = (unsigned)d.nx, nxy = nx * (unsigned)d.ny;
+  const bool in[6] = { i > 0, i < d.nx - 1, j > 0, j < d.ny - 1, k > 0, k < d.nz - 1 };
+  const unsigned o[6] = { c - 1u, c + 1u, c - nx, c + nx, c - nxy, c + nxy };
+  const int tc = g.type[c];
+  int tn[6];
+#pragma unroll
+  for (int q = 0; q < 6; q++) tn[q] = in[q] ? g.type[o[q]] : WS_SOLID;
+  unsigned f[3];
+  cell_faces(d, i, j, k, f);
+  const float u0 = g.vel[f[0]], u1 = g.vel[f[0] + 1u], v0 = g.vel[f[1]], v1 = g.vel[f[1] + nx];
+  const float w0 = g.vel[f[2]], w1 = g.vel[f[2] + nxy];
+  if (tc != WS_FLUID) { g.q[c] = 0.f; g.pw[c] = -1.f; diag8[c] = 0; return false; }
   int cnt = 0;
 #pragma unroll
-  for (int q = 0; q < 6; q++) if (nbr[q] >= 0 && type[nbr[q]] != WS_SOLID) cnt++;
-  const float* u = g.vel; const float* v = g.vel + d.uN; const float* w = g.vel + d.uN + d.vN;
-  double div = ((double)u[((long long)k * ny + j) * (nx + 1) + i + 1] - (double)u[((long long)k * ny + j) * (nx + 1) + i] +
-                (double)v[((long long)k * (ny + 1) + j + 1) * nx + i] - (double)v[((long long)k * (ny + 1) + j) * nx + i] +
-                (double)w[((long long)(k + 1) * ny + j) * nx + i] - (double)w[((long long)k * ny + j) * nx + i]) / d.dx;
+  for (int q = 0; q < 6; q++) cnt += tn[q] != WS_SOLID;
+  const double div = over_dx(d, (double)u1 - (double)u0 + (double)v1 - (double)v0 + (double)w1 - (double)w0);
   g.rhs[c] = (float)(-d.dx * d.dx * div);
   g.pw[c] = (float)(cnt > 0 ? omega / (double)cnt : 0.0);
   diag8[c] = (uint8_t)cnt;
   // membership of the SOR colour lists: interior fluid cells (sor_colour)
-  if (i >= 1 && j >= 1 && k >= 1 && i + 2 <= nx && j + 2 <= ny && k + 2 <= nz) col = (i + j + k) & 1;
+  if (in[0] && in[1] && in[2] && in[3] && in[4] && in[5]) col = (i + j + k) & 1;
   return true;
 }
 // ------------------------------------------------------------ 7. red-black SOR
@@ -800,10 +768,9 @@ void launch_residual(const Dims& d, const GridDev& g, const uint8_t* diag8, doub
   k_residual_final<<<1, 1024, 0, s>>>(partials, nb, st, hostMirror);
 }
 
-// ------------------------------------------------------------ 9. project (+clamp)
-// _projectSlice (:1417-1443) and, fused when vorticity is off,
+// ------------------------------------------------------------ 9. clamp and max |u|
 // _clampUmSlice (:2629-2653) with the max |u| reduction (exact: max of
-// non-negative float bit patterns).
+// non-negative float bit patterns); in the projection pass when vorticity is off.
 // block-level max, then one atomic per block (every thread of the block must call)
 __device__ __forceinline__ void umax_reduce(float a, DevStatus* st) {
   __shared__ unsigned sm[32];
@@ -817,30 +784,6 @@ __device__ __forceinline__ void umax_reduce(float a, DevStatus* st) {
     bits = warp_max_u(bits);
     if (lane == 0 && bits) atomicMax(&st->umaxBits, bits);
   }
-}
-__device__ __forceinline__ float face_project(const Dims& d, const GridDev& g, long long f, const FaceIJK& F, int doClamp,
-                                              float vcap) {
-  float u = g.vel[f];
-  long long cL = 0, cR = 0;
-  if (!face_cells(d, F, cL, cR)) {
-    int tL = g.type[cL], tR = g.type[cR];
-    if (tL != WS_SOLID && tR != WS_SOLID) {
-      double pL = tL == WS_FLUID ? (double)g.q[cL] : 0.0, pR = tR == WS_FLUID ? (double)g.q[cR] : 0.0;
-      u = (float)((double)u - (pR - pL) * (1.0 / d.dx));
-    }
-  }
-  if (doClamp) { if (u > vcap) u = vcap; else if (u < -vcap) u = -vcap; }
-  g.vel[f] = u;
-  return u;
-}
-__global__ void k_project(Dims d, GridDev g, int doClamp, float vcap, DevStatus* st) {
-  long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  float u = 0.f;
-  if (f < d.F) u = face_project(d, g, f, decode_face(d, f), doClamp, vcap);
-  if (doClamp) umax_reduce(u, st);
-}
-void launch_project(const Dims& d, const GridDev& g, int doClamp, double maxSpeed, DevStatus* st, cudaStream_t s) {
-  k_project<<<grid_for(d.F, 256), 256, 0, s>>>(d, g, doClamp, (float)(maxSpeed * 1.1), st);
 }
 __global__ void k_clamp_umax(Dims d, float* __restrict__ vel, float vcap, DevStatus* st) {
   long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -939,41 +882,6 @@ void launch_vorticity(const Dims& d, const GridDev& g, double eps, double dt, cu
   k_vort_splat<<<grid_for(d.F, 256), 256, 0, s>>>(d, g);
 }
 
-// ------------------------------------------------------------ 11. extrapolate
-// _extrapolate, js/solver.js:1562-1636 in Jacobi order: an invalid face takes
-// the mean of the neighbours (same component grid) that were valid before
-// the pass, summed in the reference's order -i, +i, -j, +j, -k, +k. Filled
-// faces are marked 2 so no thread reads a value written in this pass.
-__device__ __forceinline__ void face_extrapolate(const Dims& d, const GridDev& g, long long f, const FaceIJK& F) {
-  const uint8_t* valid = g.valid;
-  int d0, d1, d2;
-  if (F.comp == 0) { d0 = d.nx + 1; d1 = d.ny; d2 = d.nz; }
-  else if (F.comp == 1) { d0 = d.nx; d1 = d.ny + 1; d2 = d.nz; }
-  else { d0 = d.nx; d1 = d.ny; d2 = d.nz + 1; }
-  long long sK = (long long)d0 * d1;
-  const float* a = g.vel;
-  // every in-range neighbour's flag and velocity in one round trip, then the
-  // sum over the originally valid ones in the fixed order -x, +x, -y, +y, -z, +z
-  const long long o[6] = { f - 1, f + 1, f - d0, f + d0, f - sK, f + sK };
-  const bool in[6] = { F.i > 0, F.i < d0 - 1, F.j > 0, F.j < d1 - 1, F.k > 0, F.k < d2 - 1 };
-  uint8_t vv[6]; float av[6];
-#pragma unroll
-  for (int q = 0; q < 6; q++) { vv[q] = in[q] ? valid[o[q]] : (uint8_t)0; av[q] = in[q] ? a[o[q]] : 0.f; }
-  double sum = 0; int cnt = 0;
-#pragma unroll
-  for (int q = 0; q < 6; q++) if (vv[q] == 1) { sum += av[q]; cnt++; }
-  if (cnt > 0) { g.vel[f] = (float)(sum / cnt); g.valid[f] = 2; }
-}
-__global__ void k_extrapolate(Dims d, GridDev g) {
-  long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (f >= d.F) return;
-  if (g.valid[f] != 0) return;
-  face_extrapolate(d, g, f, decode_face(d, f));
-}
-void launch_extrapolate(const Dims& d, const GridDev& g, cudaStream_t s) {
-  k_extrapolate<<<grid_for(d.F, 256), 256, 0, s>>>(d, g);
-}
-
 // ------------------------------------------------------------ active bricks
 // Faces and cells far from every particle and moving solid hold fixed values
 // (zero velocity, the static valid flags, q = 0 and pw = -1 off the fluid), so
@@ -983,181 +891,293 @@ void launch_extrapolate(const Dims& d, const GridDev& g, cudaStream_t s) {
 // P2G's stencils, the extrapolation layer and G2P's midpoint sample is under
 // four cells), plus those active in the previous substep, so a brick that
 // empties is rewritten once to the fixed values. A forced full pass (after a
-// caller wrote grid fields) processes every brick.
-__global__ void k_brick_activity(int nbx, int nby, int nbz, const uint8_t* __restrict__ seed, uint8_t* __restrict__ act,
-                                 uint8_t* __restrict__ proc, const int* __restrict__ forceAll, int* __restrict__ list,
-                                 int* __restrict__ count) {
+// caller wrote grid fields) processes every brick; after a write of q alone,
+// which only the pressure setup turns back to the fixed value, that pass does.
+__global__ void __launch_bounds__(256) k_brick_activity(BrickSet B) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nB = nbx * nby * nbz;
+  const int nB = B.nbx * B.nby * B.nbz;
   int p = 0;
   if (b < nB) {
-    const int bx = b % nbx, t = b / nbx, by = t % nby, bz = t / nby;
+    int bx, by, bz;
+    brick_coords(B, b, bx, by, bz);
     int a = 0;
-    for (int dz = -1; dz <= 1 && !a; dz++) {
-      const int z = bz + dz;
-      if (z < 0 || z >= nbz) continue;
-      for (int dy = -1; dy <= 1 && !a; dy++) {
-        const int y = by + dy;
-        if (y < 0 || y >= nby) continue;
-        const uint8_t* row = seed + ((long long)z * nby + y) * nbx;
-        for (int dx = -1; dx <= 1; dx++) {
-          const int x = bx + dx;
-          if (x >= 0 && x < nbx && row[x]) { a = 1; break; }
-        }
+    // all 27 seeds in flight at once (a clamped neighbour only repeats a seed of the block)
+#pragma unroll
+    for (int dz = -1; dz <= 1; dz++) {
+      const int z = min(max(bz + dz, 0), B.nbz - 1);
+#pragma unroll
+      for (int dy = -1; dy <= 1; dy++) {
+        const uint8_t* row = B.seed + (z * B.nby + min(max(by + dy, 0), B.nby - 1)) * B.nbx;
+        a |= row[max(bx - 1, 0)] | row[bx] | row[min(bx + 1, B.nbx - 1)];
       }
     }
-    p = a | act[b] | (*forceAll != 0);
-    proc[b] = (uint8_t)p;
-    act[b] = (uint8_t)a;
+    p = a | B.act[b] | (*B.forceAll != 0);
+    B.act[b] = (uint8_t)a;
   }
   // the work list: one atomic per warp (the passes over it do not depend on its order)
   const unsigned m = __ballot_sync(0xffffffffu, p != 0);
   const int lane = threadIdx.x & 31;
   int base = 0;
-  if (lane == 0 && m) base = atomicAdd(count, __popc(m));
+  if (lane == 0 && m) base = atomicAdd(B.count, __popc(m));
   base = __shfl_sync(0xffffffffu, base, 0);
-  if (p) list[base + __popc(m & ((1u << lane) - 1u))] = b;
+  if (p) B.list[base + __popc(m & ((1u << lane) - 1u))] = b;
 }
-// the count reset, activity and work list, then the seeds and the
-// forced-pass flag cleared for the next substep
-cudaError_t launch_brick_activity(const BrickSet& B, cudaStream_t s) {
-  const int nB = B.nbx * B.nby * B.nbz;
-  cudaError_t e = cudaMemsetAsync(B.count, 0, sizeof(int), s);
-  if (e != cudaSuccess) return e;
-  k_brick_activity<<<grid_for(nB, 256), 256, 0, s>>>(B.nbx, B.nby, B.nbz, B.seed, B.act, B.proc, B.forceAll, B.list,
-                                                      B.count);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(B.seed, 0, (size_t)nB, s)) != cudaSuccess) return e;
-  return cudaMemsetAsync(B.forceAll, 0, sizeof(int), s);
+// activity and work list; the normalising pass that follows clears the seeds
+// and the projection the forced-pass flags for the next substep
+void launch_brick_activity(const BrickSet& B, cudaStream_t s) {
+  k_brick_activity<<<grid_for((long long)B.nbx * B.nby * B.nbz, 256), 256, 0, s>>>(B);
 }
 
-// The faces a brick owns: per component, the 64 faces whose lower cell lies
-// in the brick, and on the last brick along the component's axis the 16
-// faces of the domain's upper plane. Slot t in [0, 240): its component and
-// offsets in the brick are the same for every brick, so a thread decodes
-// them once (face_slot) and each brick adds only its coordinates.
-struct FaceSlot { int comp, la, lb, lc; bool upper; };
-__device__ __forceinline__ FaceSlot face_slot(int t) {
-  FaceSlot sl;
-  sl.comp = t >= 160 ? 2 : t >= 80 ? 1 : 0;
-  const int s = t - sl.comp * 80;
-  sl.upper = s >= 64;
-  if (!sl.upper) { sl.la = s & 3; sl.lb = (s >> 2) & 3; sl.lc = s >> 4; }
-  else { sl.la = 0; sl.lb = (s - 64) & 3; sl.lc = (s - 64) >> 2; }
-  return sl;
+// ------------------------------------------------------------ the face passes
+// 4. _p2gNormalizeFace (:1109-1120) + _applyBC (:1130-1171) + FLIP snapshot
+//    (:2579) + the extrapolation valid mark (:1578-1611)
+// 5. forces: _viscosity (:1259-1304, Jacobi: neighbours from the snapshot,
+//    which equals the post-BC field on entry), planet gravity (:1229-1256
+//    with the ramp of :2656-2662 applied by the caller in gs), BC again (:2598)
+// 9. _projectSlice (:1417-1443) and, fused when vorticity is off, the clamp
+//    and max |u| of _clampUmSlice (:2629-2653)
+// 11. _extrapolate (:1562-1636) in Jacobi order: an invalid face takes the
+//    mean of the neighbours (same component grid) that were valid before the
+//    pass, summed in the reference's order -i, +i, -j, +j, -k, +k. Filled
+//    faces are marked 2 so no thread reads a value written in this pass.
+//
+// One thread per cell of a 4^3 brick handles the cell's three lower faces
+// (and the domain's upper plane where the cell is the last along the axis):
+// its loads are issued together and its type is shared by the three faces.
+// Bytes per face: normalise 8 + 4 + 4 + 1, forces 4 + 4 + 4 (+ neighbours from
+// cache), project 4 + 4 + 4/3, extrapolate 1; types 4/3. FP64 where the
+// reference's doubles round differently from floats; a quotient of two floats
+// is the same either way (53 bits hold twice 24 + 2).
+enum FaceOp { kNormalize, kForces, kProject, kExtrapolate };
+struct FacePassArgs { double coef, dt, gs; int viscOn, doClamp; float vcap; int all; };
+// Solid-adjacent interior face: the velocity of the solid cell beside it,
+// the left one first (_applyBCSlice, js/solver.js:1153-1170): 0 for rock and
+// the domain shell, the ball's velocity for a ball cell.
+__device__ __forceinline__ float solid_face_velocity(const Dims& d, const GridDev& g, int comp, int tL, unsigned cL, unsigned cR) {
+  return g.sv ? g.sv[comp * d.nCells + (tL == WS_SOLID ? cL : cR)] : 0.f;
 }
-__device__ __forceinline__ bool brick_face(const Dims& d, const BrickSet& B, int bx, int by, int bz, const FaceSlot& sl,
-                                           long long& f, FaceIJK& F) {
-  const int comp = sl.comp, la = sl.la, lb = sl.lb, lc = sl.lc;
-  const bool upper = sl.upper;
-  const int nx = d.nx, ny = d.ny, nz = d.nz;
-  F.comp = comp;
-  if (comp == 0) {
-    if (upper && bx != B.nbx - 1) return false;
-    F.i = upper ? nx : bx * 4 + la; F.j = by * 4 + lb; F.k = bz * 4 + lc;
-    if ((!upper && F.i >= nx) || F.j >= ny || F.k >= nz) return false;
-    f = ((long long)F.k * ny + F.j) * (nx + 1) + F.i;
-  } else if (comp == 1) {
-    if (upper && by != B.nby - 1) return false;
-    F.j = upper ? ny : by * 4 + la; F.i = bx * 4 + lb; F.k = bz * 4 + lc;
-    if ((!upper && F.j >= ny) || F.i >= nx || F.k >= nz) return false;
-    f = d.uN + ((long long)F.k * (ny + 1) + F.j) * nx + F.i;
-  } else {
-    if (upper && bz != B.nbz - 1) return false;
-    F.k = upper ? nz : bz * 4 + la; F.i = bx * 4 + lb; F.j = by * 4 + lc;
-    if ((!upper && F.k >= nz) || F.i >= nx || F.j >= ny) return false;
-    f = d.uN + d.vN + ((long long)F.k * ny + F.j) * nx + F.i;
-  }
-  F.local = 0;
-  return true;
-}
-
-// one face pass over the brick list (persistent blocks, one brick per
-// iteration); op 0 normalise + BC, 1 forces, 2 project (+ clamp, umax),
-// 3 extrapolate, 4 clear the P2G accumulator
-struct FacePassArgs { double coef, dt, gs; int viscOn, doClamp; float vcap; };
 template <int OP>
-__global__ void __launch_bounds__(256) k_faces_bricks(Dims d, GridDev g, BrickSet B, FacePassArgs fa, DevStatus* st) {
-  if (OP == 4 && *B.forceAll) {                          // after a forced full pass: the whole accumulator
-    const long long F2 = d.F >> 1;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t <= F2; t += (long long)gridDim.x * blockDim.x) {
-      if (t < F2) reinterpret_cast<float4*>(g.acc)[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-      else if (d.F & 1) g.acc[d.F - 1] = make_float2(0.f, 0.f);
+__device__ __forceinline__ void upper_face(const GridDev& g, unsigned f, const FacePassArgs& fa, float& umax) {
+  if (OP == kNormalize) { g.vel[f] = 0.f; g.velO[f] = 0.f; g.valid[f] = 1; }
+  if (OP == kForces) g.vel[f] = 0.f;
+  if (OP == kProject && fa.doClamp) {
+    float u = g.vel[f];
+    if (u > fa.vcap) u = fa.vcap; else if (u < -fa.vcap) u = -fa.vcap;
+    g.vel[f] = u; umax = fmaxf(umax, fabsf(u));
+  }
+}
+template <int OP>
+__device__ __forceinline__ void cell_pass(const Dims& d, const GridDev& g, int i, int j, int k, const FacePassArgs& fa, float& umax) {
+  unsigned f[3];
+  const unsigned c = cell_faces(d, i, j, k, f), nx = (unsigned)d.nx, nxy = nx * (unsigned)d.ny;
+  const unsigned cl[3] = { c - 1u, c - nx, c - nxy };   // the cell below each face
+  const bool edge[3] = { i == 0, j == 0, k == 0 };      // a domain plane
+  const bool last[3] = { i == d.nx - 1, j == d.ny - 1, k == d.nz - 1 };
+  // strides of each component's face grid along y and z
+  const unsigned sJ[3] = { nx + 1u, nx, nx }, sK[3] = { nxy + (unsigned)d.ny, nxy + nx, nxy };
+  if (OP == kExtrapolate) {
+    uint8_t v[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) v[a] = g.valid[f[a]];
+    uint8_t vv[3][6];
+    float av[3][6];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      if (v[a]) continue;
+      const unsigned o[6] = { f[a] - 1u, f[a] + 1u, f[a] - sJ[a], f[a] + sJ[a], f[a] - sK[a], f[a] + sK[a] };
+      const bool in[6] = { !edge[0], a == 0 || !last[0], !edge[1], a == 1 || !last[1], !edge[2], a == 2 || !last[2] };
+#pragma unroll
+      for (int q = 0; q < 6; q++) { vv[a][q] = in[q] ? g.valid[o[q]] : (uint8_t)0; av[a][q] = in[q] ? g.vel[o[q]] : 0.f; }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      if (v[a]) continue;
+      double sum = 0; int cnt = 0;
+#pragma unroll
+      for (int q = 0; q < 6; q++) if (vv[a][q] == 1) { sum += av[a][q]; cnt++; }
+      if (cnt > 0) { g.vel[f[a]] = (float)(sum / cnt); g.valid[f[a]] = 2; }
+    }
+    // the domain's upper plane: always valid after the normalising pass, not after a caller's own fields
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      if (!last[a]) continue;
+      const unsigned fu = f[a] + (a == 0 ? 1u : a == 1 ? nx : nxy);
+      if (g.valid[fu]) continue;
+      const unsigned o[6] = { fu - 1u, fu + 1u, fu - sJ[a], fu + sJ[a], fu - sK[a], fu + sK[a] };
+      double sum = 0; int cnt = 0;
+#pragma unroll
+      for (int q = 0; q < 6; q++) {
+        const bool in = q >> 1 == a ? !(q & 1) : q & 1 ? !last[q >> 1] : !edge[q >> 1];
+        if (in && g.valid[o[q]] == 1) { sum += g.vel[o[q]]; cnt++; }
+      }
+      if (cnt > 0) { g.vel[fu] = (float)(sum / cnt); g.valid[fu] = 2; }
     }
     return;
   }
-  const int n = *B.count;
+  int t[3];
+  const int tc = g.type[c];
+#pragma unroll
+  for (int a = 0; a < 3; a++) t[a] = edge[a] ? WS_SOLID : g.type[cl[a]];
+  if (OP == kNormalize) {
+    float2 A[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) A[a] = g.acc[f[a]];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const bool some = (double)A[a].y > 1e-8, solid = t[a] == WS_SOLID || tc == WS_SOLID;
+      float u = some ? A[a].x / A[a].y : A[a].x;
+      if (edge[a]) u = 0.f;
+      else if (solid) u = solid_face_velocity(d, g, a, t[a], cl[a], c);
+      g.vel[f[a]] = u; g.velO[f[a]] = u; g.valid[f[a]] = some || solid ? 1 : 0;
+    }
+  }
+  if (OP == kForces) {
+    const float* __restrict__ o = g.velO;
+    float u[3], gv[3], nb[3][6];
+    bool visc[3], grav[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const bool open = t[a] != WS_SOLID && tc != WS_SOLID;
+      visc[a] = fa.viscOn && t[a] == WS_FLUID && tc == WS_FLUID;
+      grav[a] = fa.gs > 0 && open && (t[a] == WS_FLUID || tc == WS_FLUID);
+      u[a] = open ? o[f[a]] : 0.f;
+      gv[a] = grav[a] ? g.gvel[f[a]] : 0.f;
+      if (visc[a]) {
+        const unsigned p[6] = { f[a] - 1u, f[a] + 1u, f[a] - sJ[a], f[a] + sJ[a], f[a] - sK[a], f[a] + sK[a] };
+        const bool in[6] = { !edge[0], a == 0 || !last[0], !edge[1], a == 1 || !last[1], !edge[2], a == 2 || !last[2] };
+#pragma unroll
+        for (int q = 0; q < 6; q++) nb[a][q] = o[in[q] ? p[q] : f[a]];   // off the grid: the face's own value
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      float r = u[a];
+      if (visc[a]) {
+        const double c0 = u[a];
+        double val = c0 * 6;
+#pragma unroll
+        for (int q = 0; q < 6; q++) val -= (double)nb[a][q];
+        r = (float)(c0 + fa.coef * val);
+      }
+      if (grav[a]) r = (float)((double)r + (double)gv[a] * fa.dt * fa.gs);
+      if (!edge[a] && (t[a] == WS_SOLID || tc == WS_SOLID)) r = solid_face_velocity(d, g, a, t[a], cl[a], c);
+      g.vel[f[a]] = r;
+    }
+  }
+  if (OP == kProject) {
+    float u[3], ql[3];
+    const float qc = g.q[c];
+#pragma unroll
+    for (int a = 0; a < 3; a++) { u[a] = g.vel[f[a]]; ql[a] = edge[a] ? 0.f : g.q[cl[a]]; }
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const bool open = t[a] != WS_SOLID && tc != WS_SOLID;
+      if (open) {
+        const double pL = t[a] == WS_FLUID ? (double)ql[a] : 0.0, pR = tc == WS_FLUID ? (double)qc : 0.0;
+        u[a] = (float)((double)u[a] - (pR - pL) * d.rdx);
+      }
+      if (fa.doClamp) {
+        if (u[a] > fa.vcap) u[a] = fa.vcap; else if (u[a] < -fa.vcap) u[a] = -fa.vcap;
+        umax = fmaxf(umax, fabsf(u[a]));
+      }
+      g.vel[f[a]] = u[a];
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+    if (last[a]) upper_face<OP>(g, f[a] + (a == 0 ? 1u : a == 1 ? nx : nxy), fa, umax);
+}
+// One pass over the work list (all: over every brick), four bricks per block
+// and iteration. Bound by load latency (L1 and L2 at a third of their rates).
+// Normalise / forces / project / extrapolate, one thread per face of a brick
+// before: 24.4 / 29.7 / 22.2 / 28.6 us at 128^3, now 13.3 / 15.5 / 10.4 / 15.6;
+// 110 / 140 / 96 / 90 -> 87 / 73 / 50 / 64 at 256^3; with half a brick
+// per warp instead of two rows of four, normalise and project took 19.3 and
+// 14.0 us at 128^3, 129 and 61 at 256^3. Clearing in the raster pass instead of
+// its own 10.1 -> 3.9 us at 128^3.
+template <int OP>
+__global__ void __launch_bounds__(256) k_faces(Dims d, GridDev g, BrickSet B, FacePassArgs fa, DevStatus* st) {
+  const int nB = B.nbx * B.nby * B.nbz;
+  if (OP == kNormalize && !fa.all) {                    // the substep's seeds have been read
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int t = t0; t < nB >> 4; t += gridDim.x * blockDim.x) reinterpret_cast<uint4*>(B.seed)[t] = make_uint4(0, 0, 0, 0);
+    if (t0 < (nB & 15)) B.seed[(nB & ~15) + t0] = 0;
+    if (t0 == 0) B.count[1] = *B.count;
+  }
+  if (OP == kProject && !fa.all && blockIdx.x == 0 && threadIdx.x == 0) { B.forceAll[0] = 0; B.forceAll[1] = 0; }
+  const int n = fa.all ? nB : *B.count, step = gridDim.x * 4;
+  int q, li, lj, lk;
+  quad_cell(q, li, lj, lk);
   float umax = 0.f;
-  const FaceSlot sl = face_slot(threadIdx.x < 240 ? (int)threadIdx.x : 0);
-  int b = (int)blockIdx.x < n ? B.list[blockIdx.x] : 0;
-  for (int it = blockIdx.x; it < n; it += gridDim.x) {
-    // the next brick's id is loaded before this brick's faces are touched, so
-    // its round trip overlaps this brick's loads and stores
-    const int bNext = it + (int)gridDim.x < n ? B.list[it + gridDim.x] : 0;
-    long long f; FaceIJK F;
+  int it = blockIdx.x * 4 + q;
+  int b = fa.all ? it : it < n ? B.list[it] : 0;
+  for (; it < n; it += step) {
+    // the next brick's id is loaded before this brick's faces are touched
+    const int bNext = fa.all ? it + step : it + step < n ? B.list[it + step] : 0;
     int bx, by, bz;
     brick_coords(B, b, bx, by, bz);
-    if (threadIdx.x < 240 && brick_face(d, B, bx, by, bz, sl, f, F)) {
-      if (OP == 0) face_normalize_bc(d, g, f, F);
-      else if (OP == 1) face_forces(d, g, f, F, fa.coef, fa.viscOn, fa.dt, fa.gs);
-      else if (OP == 2) umax = fmaxf(umax, fabsf(face_project(d, g, f, F, fa.doClamp, fa.vcap)));
-      else if (OP == 3) { if (g.valid[f] == 0) face_extrapolate(d, g, f, F); }
-      else g.acc[f] = make_float2(0.f, 0.f);
-    }
+    const int i = bx * 4 + li, j = by * 4 + lj, k = bz * 4 + lk;
+    if (i < d.nx && j < d.ny && k < d.nz) cell_pass<OP>(d, g, i, j, k, fa, umax);
     b = bNext;
   }
-  if (OP == 2 && fa.doClamp) umax_reduce(umax, st);
+  if (OP == kProject && fa.doClamp) umax_reduce(umax, st);
 }
 static unsigned brick_grid(const BrickSet& B) {
   const int nB = B.nbx * B.nby * B.nbz;
-  return (unsigned)std::min(nB, 148 * 8);
+  return (unsigned)std::min((nB + 3) / 4, 148 * 8);
 }
-void launch_faces_normalize_bc_bricks(const Dims& d, const GridDev& g, const BrickSet& B, cudaStream_t s) {
-  k_faces_bricks<0><<<brick_grid(B), 256, 0, s>>>(d, g, B, FacePassArgs{}, nullptr);
+void launch_faces_normalize_bc(const Dims& d, const GridDev& g, const BrickSet& B, bool all, cudaStream_t s) {
+  FacePassArgs fa{}; fa.all = all;
+  k_faces<kNormalize><<<brick_grid(B), 256, 0, s>>>(d, g, B, fa, nullptr);
 }
-void launch_faces_forces_bricks(const Dims& d, const GridDev& g, const BrickSet& B, double coef, int viscOn, double dt,
-                                double gs, cudaStream_t s) {
-  FacePassArgs fa{}; fa.coef = coef; fa.viscOn = viscOn; fa.dt = dt; fa.gs = gs;
-  k_faces_bricks<1><<<brick_grid(B), 256, 0, s>>>(d, g, B, fa, nullptr);
+void launch_faces_forces(const Dims& d, const GridDev& g, const BrickSet& B, bool all, double coef, int viscOn, double dt,
+                         double gs, cudaStream_t s) {
+  FacePassArgs fa{}; fa.coef = coef; fa.viscOn = viscOn; fa.dt = dt; fa.gs = gs; fa.all = all;
+  k_faces<kForces><<<brick_grid(B), 256, 0, s>>>(d, g, B, fa, nullptr);
 }
-void launch_project_bricks(const Dims& d, const GridDev& g, const BrickSet& B, int doClamp, double maxSpeed,
-                           DevStatus* st, cudaStream_t s) {
-  FacePassArgs fa{}; fa.doClamp = doClamp; fa.vcap = (float)(maxSpeed * 1.1);
-  k_faces_bricks<2><<<brick_grid(B), 256, 0, s>>>(d, g, B, fa, st);
+void launch_project(const Dims& d, const GridDev& g, const BrickSet& B, bool all, int doClamp, double maxSpeed,
+                    DevStatus* st, cudaStream_t s) {
+  FacePassArgs fa{}; fa.doClamp = doClamp; fa.vcap = (float)(maxSpeed * 1.1); fa.all = all;
+  k_faces<kProject><<<brick_grid(B), 256, 0, s>>>(d, g, B, fa, st);
 }
-void launch_extrapolate_bricks(const Dims& d, const GridDev& g, const BrickSet& B, cudaStream_t s) {
-  k_faces_bricks<3><<<brick_grid(B), 256, 0, s>>>(d, g, B, FacePassArgs{}, nullptr);
+void launch_extrapolate(const Dims& d, const GridDev& g, const BrickSet& B, bool all, cudaStream_t s) {
+  FacePassArgs fa{}; fa.all = all;
+  k_faces<kExtrapolate><<<brick_grid(B), 256, 0, s>>>(d, g, B, fa, nullptr);
 }
-// the accumulator of the bricks in the list (those the previous substep's
-// P2G may have written), or all of it after a forced full pass
-void launch_clear_acc_bricks(const Dims& d, const GridDev& g, const BrickSet& B, cudaStream_t s) {
-  k_faces_bricks<4><<<brick_grid(B), 256, 0, s>>>(d, g, B, FacePassArgs{}, nullptr);
-}
-// the pressure setup over the brick list (or every brick): four bricks per
-// 256-thread block, a brick's two warps ballot its mask
+// the pressure setup over the brick list (or every brick), four bricks per block
 __global__ void __launch_bounds__(256) k_pressure_setup(Dims d, GridDev g, uint8_t* __restrict__ diag8, double omega,
                                                         DevStatus* st, BrickSet B, int allBricks) {
-  const int n = allBricks ? B.nbx * B.nby * B.nbz : *B.count;
-  unsigned* mask = reinterpret_cast<unsigned*>(g.fmask);
-  int fluid = 0, odd = 0;
+  const bool every = allBricks || B.forceAll[1];        // every brick after a caller wrote q (q = 0 off the fluid)
+  const int n = every ? B.nbx * B.nby * B.nbz : *B.count;
+  uint8_t* mask = reinterpret_cast<uint8_t*>(g.fmask);
+  int fluid = 0, odd = 0, q, li, lj, lk;
+  quad_cell(q, li, lj, lk);
   for (int it = blockIdx.x * 4; it < n; it += gridDim.x * 4) {
-    const int e = it + (threadIdx.x >> 6);
-    if (e >= n) continue;                              // uniform over the warp
-    const int b = allBricks ? e : B.list[e], c = threadIdx.x & 63;
-    int bx, by, bz;
-    brick_coords(B, b, bx, by, bz);
-    const int i = bx * 4 + (c & 3), j = by * 4 + ((c >> 2) & 3), k = bz * 4 + (c >> 4);
+    const int e = it + q, b = e >= n ? -1 : every ? e : B.list[e];
     int col = -1;
-    if (i < d.nx && j < d.ny && k < d.nz &&
-        cell_pressure_setup(d, g, diag8, omega, ((long long)k * d.ny + j) * d.nx + i, i, j, k, col)) {
-      fluid++;
-      odd |= col < 0;
+    if (b >= 0) {
+      int bx, by, bz;
+      brick_coords(B, b, bx, by, bz);
+      const int i = bx * 4 + li, j = by * 4 + lj, k = bz * 4 + lk;
+      if (i < d.nx && j < d.ny && k < d.nz &&
+          cell_pressure_setup(d, g, diag8, omega, ((unsigned)k * (unsigned)d.ny + (unsigned)j) * (unsigned)d.nx + (unsigned)i, i, j, k, col)) {
+        fluid++;
+        odd |= col < 0;
+      }
     }
-    const unsigned m = __ballot_sync(0xffffffffu, col >= 0);
-    if ((threadIdx.x & 31) == 0) mask[2 * b + (c >> 5)] = m;
+    // bit 16 z + 4 y + x: the warp's two rows of a brick are one byte of its mask
+    const unsigned m = __ballot_sync(0xffffffffu, col >= 0) >> (4 * q);
+    if ((threadIdx.x & 19) == 0 && b >= 0) mask[8 * b + (threadIdx.x >> 5)] = (uint8_t)((m & 15u) | (m >> 12 & 0xf0u));
   }
+  // one atomic per block: thousands of warps on one address take microseconds
   fluid = warp_sum(fluid);
-  if ((threadIdx.x & 31) == 0 && fluid) atomicAdd(&st->nFluid, fluid);
+  __shared__ int sFluid[8];
+  if ((threadIdx.x & 31) == 0) sFluid[threadIdx.x >> 5] = fluid;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) fluid += sFluid[w];
+    if (fluid) atomicAdd(&st->nFluid, fluid);
+  }
   if (odd) atomicOr(&st->oddFluid, 1);
   if (blockIdx.x == 0 && threadIdx.x == 0) st->sorOmega = omega;
 }

@@ -132,6 +132,15 @@ struct DevStatus {
   unsigned int evSEnd, evSStart;   // stream after the pass; start state of a restarted pass
   int oddFluid;            // the pressure setup met a fluid cell on the domain's outermost layer (zeroed by the raster)
   double sorOmega;         // omega of the last pressure setup (pw = omega / diag)
+  double timedRel;         // the outcome of a solve that a timing call runs, apart from the substep's
+  int timedIters, timedPath;
+};
+// where a solve leaves its iteration count, relative residual and path
+struct SorOut {
+  int* iters; double* rel; int* path;
+  SorOut(DevStatus* st, bool report)
+      : iters(report ? &st->sorIters : &st->timedIters), rel(report ? &st->relres : &st->timedRel),
+        path(report ? &st->pad2 : &st->timedPath) {}
 };
 
 struct GridDev {
@@ -155,10 +164,9 @@ struct BrickSet {
   int nbx, nby, nbz;
   uint8_t* seed;            // bricks holding a particle or moving solid this substep
   uint8_t* act;             // seeds dilated by one brick (kept for the next substep)
-  uint8_t* proc;            // this substep's work: act | last substep's act | forced
-  int* list;                // the bricks with proc set (in no particular order)
-  int* count;
-  int* forceAll;            // device flag: process every brick once
+  int* list;                // this substep's work, act | last substep's act | forced (in no particular order)
+  int* count;               // [0] entries of list, [1] the same kept until the next substep's clear
+  int* forceAll;            // device flags: [0] process every brick once, [1] in the pressure setup only
   FastDiv dnbx, dnby;       // division by nbx and nby (brick coordinates of a linear brick index)
   unsigned long long* fmask;   // per brick: its interior fluid cells as of the last pressure setup
 };

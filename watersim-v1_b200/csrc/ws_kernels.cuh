@@ -24,16 +24,16 @@ struct PhaseParams {
 // ---- ws_grid.cu
 void launch_static_types(const Dims& d, const TerrainDev& t, double coreR, uint8_t* st, cudaStream_t s);
 void launch_gravity_geometry(const Dims& d, double oceanR, float* g, cudaStream_t s);
-void launch_clear_raster(const Dims& d, const GridDev& g, DevStatus* st, bool clearAcc, cudaStream_t s);
-// the substep's face and cell passes over the active-brick list (ws_grid.cu)
-cudaError_t launch_brick_activity(const BrickSet& B, cudaStream_t s);
-void launch_clear_acc_bricks(const Dims& d, const GridDev& g, const BrickSet& B, cudaStream_t s);
-void launch_faces_normalize_bc_bricks(const Dims& d, const GridDev& g, const BrickSet& B, cudaStream_t s);
-void launch_faces_forces_bricks(const Dims& d, const GridDev& g, const BrickSet& B, double coef, int viscOn, double dt,
-                                double gs, cudaStream_t s);
-void launch_project_bricks(const Dims& d, const GridDev& g, const BrickSet& B, int doClamp, double maxSpeed,
-                           DevStatus* st, cudaStream_t s);
-void launch_extrapolate_bricks(const Dims& d, const GridDev& g, const BrickSet& B, cudaStream_t s);
+// bricks: clear the accumulator of the last substep's work list only
+void launch_clear_raster(const Dims& d, const GridDev& g, DevStatus* st, const BrickSet& B, bool bricks, cudaStream_t s);
+void launch_brick_activity(const BrickSet& B, cudaStream_t s);
+// the face passes over the active-brick list, or (all) over every brick of the grid
+void launch_faces_normalize_bc(const Dims& d, const GridDev& g, const BrickSet& B, bool all, cudaStream_t s);
+void launch_faces_forces(const Dims& d, const GridDev& g, const BrickSet& B, bool all, double coef, int viscOn, double dt,
+                         double gs, cudaStream_t s);
+void launch_project(const Dims& d, const GridDev& g, const BrickSet& B, bool all, int doClamp, double maxSpeed,
+                    DevStatus* st, cudaStream_t s);
+void launch_extrapolate(const Dims& d, const GridDev& g, const BrickSet& B, bool all, cudaStream_t s);
 // cs: count every particle P2G will scatter in its cell (null: mark only)
 void launch_mark_fluid(const Dims& d, const GridDev& g, const PartsDev& P, const TerrainDev& t,
                        double oceanR, double coreR, const CellSort* cs, DevStatus* st, cudaStream_t s);
@@ -44,8 +44,6 @@ void launch_mark_p2g(const Dims& d, const GridDev& g, const PartsDev& P, const T
 size_t cell_sort_scratch_bytes(long long nKeys);
 int launch_p2g_sorted(const Dims& d, const GridDev& g, const PartsDev& P, const CellSort& cs, const BrickSet& B,
                       bool binned, void* scratch, size_t scratchBytes, DevStatus* st, cudaStream_t s);
-void launch_faces_normalize_bc(const Dims& d, const GridDev& g, cudaStream_t s);
-void launch_faces_forces(const Dims& d, const GridDev& g, double coef, int viscOn, double dt, double gs, cudaStream_t s);
 // over the brick list, or every brick of the grid (allBricks)
 void launch_pressure_setup(const Dims& d, const GridDev& g, uint8_t* diag8, double omega, DevStatus* st,
                            const BrickSet& B, bool allBricks, cudaStream_t s);
@@ -53,10 +51,8 @@ void launch_sor_color(const Dims& d, const GridDev& g, int color, double om1, cu
 int residual_blocks(const Dims& d);
 void launch_residual(const Dims& d, const GridDev& g, const uint8_t* diag8, double2* partials,
                      DevStatus* st, double* hostMirror, cudaStream_t s);
-void launch_project(const Dims& d, const GridDev& g, int doClamp, double maxSpeed, DevStatus* st, cudaStream_t s);
 void launch_clamp_umax(const Dims& d, const GridDev& g, double maxSpeed, DevStatus* st, cudaStream_t s);
 void launch_vorticity(const Dims& d, const GridDev& g, double eps, double dt, cudaStream_t s);
-void launch_extrapolate(const Dims& d, const GridDev& g, cudaStream_t s);
 void launch_extract_weight(const Dims& d, const float2* acc, float* out, long long off, long long n, cudaStream_t s);
 
 // ---- ws_particles.cu
@@ -135,11 +131,9 @@ void sor_free(void* statePtr);
 // the whole solve of the last pressure setup's system; iterations, residual
 // and path land in device memory
 cudaError_t launch_sor_solve(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                             int iters, int check, double tol, DevStatus* st, int** outIters, double** outRel,
-                             int** outPath, cudaStream_t s);
+                             int iters, int check, double tol, DevStatus* st, bool report, cudaStream_t s);
 cudaError_t launch_sor_solve_lists(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                                   int iters, int check, double tol, DevStatus* st, int** outIters, double** outRel,
-                                   int** outPath, cudaStream_t s);
+                                   int iters, int check, double tol, DevStatus* st, bool report, cudaStream_t s);
 int sor_solve_launches(void* state);
 int sor_list_solve_launches(void* state);
 

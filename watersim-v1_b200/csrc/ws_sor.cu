@@ -614,9 +614,6 @@ struct SorState {
   int* blockOffs = nullptr;    // their exclusive scan: each block's first list slot per colour
   GridBar* bar = nullptr;
   double2* partials = nullptr;
-  int* outIters = nullptr;
-  double* outRel = nullptr;
-  int* outPath = nullptr;
   int grid = 0, block = 1024;
   long long cap = 0;
   int clusterSize = 0;       // 0: cluster path unavailable on this device
@@ -629,8 +626,8 @@ cudaError_t sor_tb_init(void** statePtr, const Dims& d, int device);
 void sor_tb_free(void* statePtr);
 const int* sor_tb_solved(void* statePtr);
 cudaError_t launch_sor_tb(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                          int iters, int check, double tol, DevStatus* st, bool listFallback, int* outIters,
-                          double* outRel, int* outPath, cudaStream_t s);
+                          int iters, int check, double tol, DevStatus* st, bool listFallback, bool report,
+                          cudaStream_t s);
 // grids up to this many cells sweep a system whose regions do not fit shared
 // memory from the region kernel itself; larger ones on the colour lists
 static const long long kTbMaxCells = 160LL * 160 * 160;
@@ -687,9 +684,6 @@ cudaError_t sor_init(void** statePtr, const Dims& d, int device) {
   if ((e = cudaMalloc(&S->bar, sizeof(GridBar))) != cudaSuccess) return e;
   if ((e = cudaMemset(S->bar, 0, sizeof(GridBar))) != cudaSuccess) return e;
   if ((e = cudaMalloc(&S->partials, sizeof(double2) * (S->grid + 1))) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&S->outIters, sizeof(int))) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&S->outRel, sizeof(double))) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&S->outPath, sizeof(int))) != cudaSuccess) return e;
   return cudaSuccess;
 }
 
@@ -709,7 +703,6 @@ void sor_free(void* statePtr) {
   for (int c = 0; c < 2; c++) { cudaFree(S->L.idx[c]); cudaFree(S->L.rhs[c]); cudaFree(S->L.pw[c]); cudaFree(S->L.dg[c]); cudaFree(S->L.code[c]); }
   cudaFree(S->L.pos);
   cudaFree(S->L.count); cudaFree(S->blockCounts); cudaFree(S->blockOffs); cudaFree(S->bar); cudaFree(S->partials);
-  cudaFree(S->outIters); cudaFree(S->outRel); cudaFree(S->outPath);
   delete S;
 }
 
@@ -731,12 +724,13 @@ static cudaError_t build_lists(SorState* S, const Dims& d, const GridDev& g, con
 // cluster, else the grid-wide persistent kernel (each returns at once when
 // the other path applies).
 static cudaError_t run_lists(SorState* S, const Dims& d, const GridDev& g, double omega, int iters, int check,
-                             double tol, int* err, bool cluster, const int* solved, cudaStream_t s) {
+                             double tol, DevStatus* st, bool report, bool cluster, const int* solved, cudaStream_t s) {
   const int C = cluster ? S->clusterSize : 0;
+  const SorOut out(st, report);
   if (C) {
     ClusterArgs ca;
     ca.d = d; ca.q = g.q; ca.L = S->L; ca.om1 = 1 - omega; ca.iters = iters; ca.check = check; ca.tol = tol;
-    ca.outIters = S->outIters; ca.outRel = S->outRel; ca.outPath = S->outPath;
+    ca.outIters = out.iters; ca.outRel = out.rel; ca.outPath = out.path;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -748,8 +742,8 @@ static cudaError_t run_lists(SorState* S, const Dims& d, const GridDev& g, doubl
   }
   SorArgs a;
   a.d = d; a.q = g.q; a.L = S->L; a.om1 = 1 - omega; a.iters = iters; a.check = check; a.tol = tol;
-  a.bar = S->bar; a.partials = S->partials; a.err = err; a.outIters = S->outIters; a.outRel = S->outRel;
-  a.outPath = S->outPath;
+  a.bar = S->bar; a.partials = S->partials; a.err = &st->err;
+  a.outIters = out.iters; a.outRel = out.rel; a.outPath = out.path;
   a.clusterCap = C ? C * kSmax : -1;
   a.offs = S->blockOffs; a.nChunks = (int)grid_for(d.nCells, 256);
   a.solved = solved;
@@ -761,26 +755,21 @@ static cudaError_t run_lists(SorState* S, const Dims& d, const GridDev& g, doubl
 // kernels follow and leave at once when the regions fitted: four launches of
 // about 1.5 us against a list solve of 15-20 us an iteration where they did not.
 cudaError_t launch_sor_solve(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                             int iters, int check, double tol, DevStatus* st, int** outIters, double** outRel,
-                             int** outPath, cudaStream_t s) {
+                             int iters, int check, double tol, DevStatus* st, bool report, cudaStream_t s) {
   SorState* S = (SorState*)statePtr;
-  if (!S->tb) return launch_sor_solve_lists(statePtr, d, g, diag8, omega, iters, check, tol, st, outIters, outRel, outPath, s);
-  *outPath = S->outPath; *outIters = S->outIters; *outRel = S->outRel;
-  cudaError_t e = launch_sor_tb(S->tb, d, g, diag8, omega, iters, check, tol, st, S->big, S->outIters, S->outRel,
-                                S->outPath, s);
+  if (!S->tb) return launch_sor_solve_lists(statePtr, d, g, diag8, omega, iters, check, tol, st, report, s);
+  cudaError_t e = launch_sor_tb(S->tb, d, g, diag8, omega, iters, check, tol, st, S->big, report, s);
   if (e != cudaSuccess || !S->big) return e;
   const int* solved = sor_tb_solved(S->tb);
   if ((e = build_lists(S, d, g, diag8, false, solved, s)) != cudaSuccess) return e;
-  return run_lists(S, d, g, omega, iters, check, tol, &st->err, false, solved, s);
+  return run_lists(S, d, g, omega, iters, check, tol, st, report, false, solved, s);
 }
 // the same solve on the colour lists (cluster-resident or grid-wide), whatever
 // the default path; for comparisons of the two paths
 cudaError_t launch_sor_solve_lists(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                                   int iters, int check, double tol, DevStatus* st, int** outIters, double** outRel,
-                                   int** outPath, cudaStream_t s) {
+                                   int iters, int check, double tol, DevStatus* st, bool report, cudaStream_t s) {
   SorState* S = (SorState*)statePtr;
-  *outPath = S->outPath; *outIters = S->outIters; *outRel = S->outRel;
   cudaError_t e = build_lists(S, d, g, diag8, S->clusterSize > 0, nullptr, s);
   if (e != cudaSuccess) return e;
-  return run_lists(S, d, g, omega, iters, check, tol, &st->err, true, nullptr, s);
+  return run_lists(S, d, g, omega, iters, check, tol, st, report, true, nullptr, s);
 }

@@ -1007,8 +1007,8 @@ const int* sor_tb_solved(void* statePtr) { return &((TbState*)statePtr)->ctl->so
 // the control block reset and the solve (two stream operations, one kernel).
 // listFallback: leave a system that does not fit to the list kernels
 cudaError_t launch_sor_tb(void* statePtr, const Dims& d, const GridDev& g, const uint8_t* diag8, double omega,
-                          int iters, int check, double tol, DevStatus* st, bool listFallback, int* outIters,
-                          double* outRel, int* outPath, cudaStream_t s) {
+                          int iters, int check, double tol, DevStatus* st, bool listFallback, bool report,
+                          cudaStream_t s) {
   TbState* S = (TbState*)statePtr;
   cudaError_t e = cudaMemsetAsync(S->ctl, 0, offsetof(TbCtl, tagBase), s);
   if (e != cudaSuccess) return e;
@@ -1019,7 +1019,8 @@ cudaError_t launch_sor_tb(void* statePtr, const Dims& d, const GridDev& g, const
   a.xmap = S->xmap; a.glist = S->glist; a.plist = S->plist; a.dense = S->dense; a.flist = S->flist; a.resPart = S->resPart; a.ctl = S->ctl;
   a.om1 = 1 - omega; a.iters = iters; a.check = check; a.tol = tol; a.err = &st->err;
   a.listFallback = listFallback ? 1 : 0;
-  a.outIters = outIters; a.outRel = outRel; a.outPath = outPath;
+  const SorOut out(st, report);
+  a.outIters = out.iters; a.outRel = out.rel; a.outPath = out.path;
   void* args[] = { &a };
   return cudaLaunchCooperativeKernel((void*)k_sor_tb, dim3(S->P), dim3(kTbThreads), args, kTbSmem, s);
 }

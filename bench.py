@@ -452,10 +452,10 @@ def roofline(fs, ms_step, iters):
     cand = {sor_name: (us_sor, 13.0 * nF * it),
             "k_p2g_runs": (us_p2g, 25.0 * nP + 8.0 * F),
             "k_g2p_advect": (us_g2p, 52.0 * nP + 8.0 * F),
-            "k_faces_bricks<normalize_bc>": (us_f1, 17.0 * Fa),
-            "k_faces_bricks<forces>": (us_f2, 12.0 * Fa),
-            "k_faces_bricks<project>": (us_pr, 8.0 * Fa),
-            "k_faces_bricks<extrapolate>": (us_ex, 5.0 * Fa)}
+            "k_faces<normalize_bc>": (us_f1, 17.0 * Fa),
+            "k_faces<forces>": (us_f2, 12.0 * Fa),
+            "k_faces<project>": (us_pr, 8.0 * Fa),
+            "k_faces<extrapolate>": (us_ex, 5.0 * Fa)}
     name = max(cand, key=lambda k: cand[k][0])
     us, nbytes = cand[name]
     achieved = nbytes / (us * 1e-6) / 1e9

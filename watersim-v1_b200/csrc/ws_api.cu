@@ -38,7 +38,7 @@ struct ws_handle {
   int capacity = 0;
   long long launches = 0;
   // grid
-  uint8_t *type = nullptr, *staticTypes = nullptr, *valid = nullptr, *diag8 = nullptr;
+  uint8_t *type = nullptr, *staticTypes = nullptr, *nearRock = nullptr, *valid = nullptr, *diag8 = nullptr;
   float *vel = nullptr, *velO = nullptr, *gvel = nullptr, *q = nullptr, *rhs = nullptr, *pw = nullptr;
   float *vort = nullptr, *dens = nullptr;
   float2* acc = nullptr;
@@ -140,7 +140,7 @@ static ws_status check_launch(ws_handle* h, int n) {
 
 static GridDev grid_of(ws_handle* h) {
   GridDev g;
-  g.type = h->type; g.staticTypes = h->staticTypes; g.vel = h->vel; g.velO = h->velO; g.acc = h->acc;
+  g.type = h->type; g.staticTypes = h->staticTypes; g.nearRock = h->nearRock; g.vel = h->vel; g.velO = h->velO; g.acc = h->acc;
   g.valid = h->valid; g.gvel = h->gvel; g.q = h->q; g.rhs = h->rhs; g.pw = h->pw;
   long long N = h->d.nCells;
   g.vfx = h->vort; g.vfy = h->vort + N; g.vfz = h->vort + 2 * N; g.omg = h->vort + 3 * N;
@@ -203,7 +203,7 @@ extern "C" ws_status ws_default_params(ws_params* p) {
 }
 
 static void free_all(ws_handle* h) {
-  void* bufs[] = { h->type, h->staticTypes, h->valid, h->diag8, h->vel, h->velO, h->gvel, h->q, h->rhs, h->pw,
+  void* bufs[] = { h->type, h->staticTypes, h->nearRock, h->valid, h->diag8, h->vel, h->velO, h->gvel, h->q, h->rhs, h->pw,
                    h->vort, h->dens, h->acc, h->tsolid, h->tR, h->st, h->partials, h->red, h->rng,
                    h->blockCounts, h->list, h->listCount, h->cand, h->cellCnt, h->cellSum, h->cellChange,
                    h->parts.px, h->parts.py, h->parts.pz, h->parts.pvx, h->parts.pvy, h->parts.pvz, h->parts.pT,
@@ -289,7 +289,7 @@ extern "C" ws_status ws_create(const ws_config* cfg, ws_handle** out) {
   long long N = d.nCells, F = d.F, P = cfg->capacity;
   long long ND = (long long)(d.nx + 1) * (d.ny + 1) * (d.nz + 1);
 #define AL(ptr, n) if ((e = dalloc(&(ptr), (size_t)(n))) != cudaSuccess) { ws_status r = fail_cuda(h, e, "cudaMalloc"); free_all(h); delete h; return r; }
-  AL(h->type, N) AL(h->staticTypes, N) AL(h->diag8, N) AL(h->valid, F)
+  AL(h->type, N) AL(h->staticTypes, N) AL(h->nearRock, N) AL(h->diag8, N) AL(h->valid, F)
   AL(h->vel, F) AL(h->velO, F) AL(h->gvel, F) AL(h->acc, F)
   AL(h->q, N) AL(h->rhs, N) AL(h->pw, N) AL(h->vort, 7 * N) AL(h->dens, ND)
   AL(h->st, 1) AL(h->red, 8) AL(h->rng, 4)
@@ -332,7 +332,7 @@ extern "C" ws_status ws_create(const ws_config* cfg, ws_handle** out) {
   cudaMemcpy(h->rng, rng0, sizeof(rng0), cudaMemcpyHostToDevice);
   // static types without terrain (the shell only) until a terrain arrives
   h->terr = TerrainDev{}; h->terr.has = 0;
-  launch_static_types(d, h->terr, S.coreR, h->staticTypes, h->stream);
+  launch_static_types(d, h->terr, S.coreR, h->staticTypes, h->nearRock, h->stream);
   e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) { ws_status r = fail_cuda(h, e, "init"); free_all(h); delete h; return r; }
   *out = h;
@@ -601,8 +601,8 @@ static ws_status terrain_to_device(ws_handle* h) {
   if (reuse && std::memcmp(&before, &t, sizeof(TerrainDev)) != 0) drop_graph(h);
   h->S.landFrac = T.landFrac;
   h->hasTerrain = true;
-  launch_static_types(h->d, t, h->S.coreR, h->staticTypes, h->stream);
-  ws_status s = check_launch(h, 1); if (s) return s;
+  launch_static_types(h->d, t, h->S.coreR, h->staticTypes, h->nearRock, h->stream);
+  ws_status s = check_launch(h, 2); if (s) return s;
   WS_TRY(cudaStreamSynchronize(h->stream));
   return WS_OK;
 }
@@ -810,6 +810,15 @@ static AdvectParams advect_params(ws_handle* h, double dt) {
     double L = std::sqrt(sx * sx + sy * sy + sz * sz); if (L == 0) L = 1;
     a.windS[0] = sx / L; a.windS[1] = sy / L; a.windS[2] = sz / L;
   }
+  const Dims& d = h->d;
+  a.picF = (float)a.pic; a.flipF = (float)(1 - a.pic); a.maxSpeedF = (float)a.maxSpeed; a.halfDt = (float)(0.5 * dt);
+  const double size[3] = { d.W, d.H, d.D };
+  for (int c = 0; c < 3; c++) { a.lo[c] = (float)(d.dx * 1.02); a.hi[c] = (float)(size[c] - d.dx * 1.02); }
+  const double domHi = d.domainR - d.dx * 0.02;
+  a.domIn2 = domHi > 0 ? (float)(domHi * domHi * (1 - 1e-5)) : 0.f;
+  a.damp = (float)std::min(dt, 0.5);
+  a.drag = (float)std::max(1 - 0.42 * dt, 0.0);
+  a.rockDrag = (float)std::max(1 - 0.6 * dt, 0.0);
   return a;
 }
 

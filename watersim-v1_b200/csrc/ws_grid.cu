@@ -70,8 +70,22 @@ __global__ void k_static_types(Dims d, TerrainDev t, double coreR, uint8_t* __re
   }
   st[c] = (shell || rock) ? WS_SOLID : WS_AIR;
 }
-void launch_static_types(const Dims& d, const TerrainDev& t, double coreR, uint8_t* st, cudaStream_t s) {
+// rock within one cell of each interior cell (the shell's own solid cells do
+// not count: rock_cell_at clamps to the interior)
+__global__ void k_near_rock(Dims d, const uint8_t* __restrict__ st, uint8_t* __restrict__ near) {
+  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (c >= d.nCells) return;
+  int i, j, k; decode_cell(d, c, i, j, k);
+  bool rock = false;
+  for (int z = max(k - 1, 1); z <= min(k + 1, d.nz - 2); z++)
+    for (int y = max(j - 1, 1); y <= min(j + 1, d.ny - 2); y++)
+      for (int x = max(i - 1, 1); x <= min(i + 1, d.nx - 2); x++)
+        rock |= st[((long long)z * d.ny + y) * d.nx + x] == WS_SOLID;
+  near[c] = rock ? WS_SOLID : WS_AIR;
+}
+void launch_static_types(const Dims& d, const TerrainDev& t, double coreR, uint8_t* st, uint8_t* nearRock, cudaStream_t s) {
   k_static_types<<<grid_for(d.nCells, 256), 256, 0, s>>>(d, t, coreR, st);
+  k_near_rock<<<grid_for(d.nCells, 256), 256, 0, s>>>(d, st, nearRock);
 }
 
 // _buildPlanetGravity, js/solver.js:1177-1210: unit-g radial geometry per face
@@ -402,13 +416,11 @@ __device__ __forceinline__ void load_run(const float* __restrict__ a, int p0, in
 // NaN latch, seed bricks, the sky test, fluid cells. The cell types of this
 // substep are the static ones and what this pass marks (no balls), so a cell
 // is marked when its static type is air. Particles that turn airborne leave
-// fl. The cell of a float position: with a power-of-two cell size the scaled
-// position and its floor are exact in float (face_coords_f).
+// fl.
 template <int R>
 __device__ __forceinline__ void mark_run(const Dims& d, const GridDev& g, const PartsDev& P, const TerrainDev& t, double oceanR,
                                       double coreR, int p0, const float (&x)[R], const float (&y)[R],
                                       const float (&z)[R], int (&fl)[R], int* err) {
-  const float rd = (float)d.rdx;
   int lastBrick = -1;
   long long lastCell = -1;
 #pragma unroll
@@ -416,13 +428,7 @@ __device__ __forceinline__ void mark_run(const Dims& d, const GridDev& g, const 
     if (p0 + r >= P.nP) continue;
     mark_sound_f(d, x[r], y[r], z[r], err);
     int i, j, k;
-    if (d.dxPow2) {
-      i = min(max((int)floorf(x[r] * rd), 0), d.nx - 1); j = min(max((int)floorf(y[r] * rd), 0), d.ny - 1);
-      k = min(max((int)floorf(z[r] * rd), 0), d.nz - 1);
-    } else {
-      i = jfloor_clamp((double)x[r] / d.dx, 0, d.nx - 1); j = jfloor_clamp((double)y[r] / d.dx, 0, d.ny - 1);
-      k = jfloor_clamp((double)z[r] / d.dx, 0, d.nz - 1);
-    }
+    cell_of_f(d, x[r], y[r], z[r], i, j, k);
     const int sb = ((k >> 2) * g.nby + (j >> 2)) * g.nbx + (i >> 2);
     if (sb != lastBrick) { g.seed[sb] = 1; lastBrick = sb; }
     if (fl[r] != 0) continue;

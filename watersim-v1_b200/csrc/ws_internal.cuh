@@ -59,6 +59,7 @@ struct Dims {
   long long nCells, uN, vN, wN, F;
   FastDiv dnx, dnx1, dny, dny1;   // nx, nx + 1, ny, ny + 1
   double rdx; int dxPow2;         // 1 / dx, and whether dx is a power of two
+  float rdxf, iHi, jHi, kHi;      // 1 / dx; nx - 1, ny - 2, nz - 2 (the last first face of a stencil), as floats
 };
 // A power-of-two divisor b = 2^k: a / b and a * 2^-k are both the correctly
 // rounded value of the same real number, so the product is bit-identical to
@@ -68,6 +69,7 @@ inline void dims_fastdiv(Dims& d) {
   d.dnx = fastdiv_make((unsigned)d.nx); d.dnx1 = fastdiv_make((unsigned)d.nx + 1);
   d.dny = fastdiv_make((unsigned)d.ny); d.dny1 = fastdiv_make((unsigned)d.ny + 1);
   d.dxPow2 = is_pow2(d.dx) ? 1 : 0; d.rdx = 1.0 / d.dx;
+  d.rdxf = (float)d.rdx; d.iHi = (float)(d.nx - 1); d.jHi = (float)(d.ny - 2); d.kHi = (float)(d.nz - 2);
 }
 // (i, j, k) of flat cell index c (c < 2^32) by the invariant-divisor multiply
 __device__ __forceinline__ void cell_ijk(const Dims& d, long long c64, int& i, int& j, int& k) {
@@ -146,6 +148,7 @@ struct SorOut {
 struct GridDev {
   uint8_t* type;
   const uint8_t* staticTypes;
+  const uint8_t* nearRock;  // per cell: WS_SOLID where one of the 27 cells around it is static rock (within the shell)
   float* vel;
   float* velO;
   float2* acc;
@@ -308,6 +311,16 @@ __device__ __forceinline__ bool rock_cell_at(const Dims& d, const uint8_t* __res
   return staticTypes[((long long)k * d.ny + j) * d.nx + i] == WS_SOLID;
 }
 
+// whether any of the 27 cells around (x, y, z), clamped as rock_cell_at, is rock
+// (1.5 2^52 + X rounded down holds floor(X) in its low word, without a conversion)
+__device__ __forceinline__ bool rock_near_at(const Dims& d, const uint8_t* __restrict__ nearRock, double x, double y, double z) {
+  const double magic = 6755399441055744.0;
+  const int i = min(max(__double2loint(__dadd_rd(over_dx(d, x), magic)), 1), d.nx - 2);
+  const int j = min(max(__double2loint(__dadd_rd(over_dx(d, y), magic)), 1), d.ny - 2);
+  const int k = min(max(__double2loint(__dadd_rd(over_dx(d, z), magic)), 1), d.nz - 2);
+  return nearRock[((unsigned)k * (unsigned)d.ny + (unsigned)j) * (unsigned)d.nx + (unsigned)i] == WS_SOLID;
+}
+
 // Face-grid coordinates of component comp, js/solver.js:737-748
 __device__ __forceinline__ void face_coords(const Dims& d, int comp, double x, double y, double z,
                                             int& i0, int& j0, int& k0, double& tx, double& ty, double& tz) {
@@ -347,6 +360,20 @@ __device__ __forceinline__ void sample_vel3(const Dims& d, const float* __restri
   face_coords(d, 2, x, y, z, i0, j0, k0, tx, ty, tz); face_strides(d, 2, i0, j0, k0, idx, sj, sk);
   oz = tri_sample(vel, idx, sj, sk, tx, ty, tz);
 }
+// The floor of a clamped to [0, hi] (hi < 2^22), and the fraction of a above
+// it in [0, 1]. 1.5 2^23 + a rounded down holds the floor in its low mantissa
+// bits: two additions and a mask, where floorf and a conversion take two slots
+// of the conversion unit (an eighth of the issue rate). A NaN takes index 0
+// and fraction 0; its particle is latched by the marking.
+__device__ __forceinline__ float floor_clamp(float a, float hi) {
+  return fminf(fmaxf(__fadd_rd(a, 12582912.f) - 12582912.f, 0.f), hi);
+}
+__device__ __forceinline__ int small_int(float f) { return __float_as_int(f + 12582912.f) & 0x3fffff; }   // whole f in [0, 2^22)
+__device__ __forceinline__ void axis_floor_frac(float a, float hi, int& i0, float& t) {
+  const float f = floor_clamp(a, hi);
+  i0 = small_int(f);
+  t = __saturatef(a - f);
+}
 
 // ---- FP32 sampling of the hot particle passes (P2G, G2P, advection)
 // Face-grid coordinates of component comp in FP32. With a power-of-two cell
@@ -363,13 +390,24 @@ __device__ __forceinline__ void face_coords_f(const Dims& d, int comp, float x, 
     tx = (float)a; ty = (float)b; tz = (float)c;
     return;
   }
-  const float r = (float)d.rdx;
+  const float r = d.rdxf;
   const float X = x * r, Y = y * r, Z = z * r;
-  const float a = comp == 0 ? X : X - 0.5f, b = comp == 1 ? Y : Y - 0.5f, c = comp == 2 ? Z : Z - 0.5f;
-  const float fi = floorf(a), fj = floorf(b), fk = floorf(c);
-  if (fi < 0.f) { i0 = 0; tx = 0.f; } else if (fi > (float)(d.nx - 1)) { i0 = d.nx - 1; tx = 1.f; } else { i0 = (int)fi; tx = a - fi; }
-  if (fj < 0.f) { j0 = 0; ty = 0.f; } else if (fj > (float)(d.ny - 2)) { j0 = d.ny - 2; ty = 1.f; } else { j0 = (int)fj; ty = b - fj; }
-  if (fk < 0.f) { k0 = 0; tz = 0.f; } else if (fk > (float)(d.nz - 2)) { k0 = d.nz - 2; tz = 1.f; } else { k0 = (int)fk; tz = c - fk; }
+  axis_floor_frac(comp == 0 ? X : X - 0.5f, d.iHi, i0, tx);
+  axis_floor_frac(comp == 1 ? Y : Y - 0.5f, d.jHi, j0, ty);
+  axis_floor_frac(comp == 2 ? Z : Z - 0.5f, d.kHi, k0, tz);
+}
+// the clamped cell of a float position (jfloor_clamp of each coordinate over
+// dx): with a power-of-two cell size the scaled position and its floor are
+// exact in float
+__device__ __forceinline__ void cell_of_f(const Dims& d, float x, float y, float z, int& i, int& j, int& k) {
+  if (d.dxPow2) {
+    const float r = d.rdxf;
+    i = small_int(floor_clamp(x * r, d.iHi)); j = small_int(floor_clamp(y * r, d.jHi + 1.f));
+    k = small_int(floor_clamp(z * r, d.kHi + 1.f));
+  } else {
+    i = jfloor_clamp((double)x / d.dx, 0, d.nx - 1); j = jfloor_clamp((double)y / d.dx, 0, d.ny - 1);
+    k = jfloor_clamp((double)z / d.dx, 0, d.nz - 1);
+  }
 }
 // trilinear blend of the eight faces around idx, FP32 with fused multiply-adds
 __device__ __forceinline__ float tri_sample_f(const float* __restrict__ a, long long idx, long long sj, long long sk,
@@ -392,10 +430,6 @@ struct Stencil3 {
   unsigned idx[3];              // first face of each component's 2x2x2 stencil
   float tx[3], ty[3], tz[3];
 };
-__device__ __forceinline__ void axis_floor_frac(float a, int hi, int& i0, float& t) {
-  const float f = floorf(a);
-  if (f < 0.f) { i0 = 0; t = 0.f; } else if (f > (float)hi) { i0 = hi; t = 1.f; } else { i0 = (int)f; t = a - f; }
-}
 // j and k strides of component comp, 32-bit
 __device__ __forceinline__ void face_strides32(const Dims& d, int comp, unsigned& sj, unsigned& sk) {
   const unsigned nx = (unsigned)d.nx, ny = (unsigned)d.ny;
@@ -416,13 +450,13 @@ __device__ __forceinline__ void face_stencil3_f(const Dims& d, float x, float y,
     }
     return;
   }
-  const float r = (float)d.rdx;
+  const float r = d.rdxf;
   const float X = x * r, Y = y * r, Z = z * r;
   int iF, iH, jF, jH, kF, kH;
   float txF, txH, tyF, tyH, tzF, tzH;
-  axis_floor_frac(X, d.nx - 1, iF, txF); axis_floor_frac(X - 0.5f, d.nx - 1, iH, txH);
-  axis_floor_frac(Y, d.ny - 2, jF, tyF); axis_floor_frac(Y - 0.5f, d.ny - 2, jH, tyH);
-  axis_floor_frac(Z, d.nz - 2, kF, tzF); axis_floor_frac(Z - 0.5f, d.nz - 2, kH, tzH);
+  axis_floor_frac(X, d.iHi, iF, txF); axis_floor_frac(X - 0.5f, d.iHi, iH, txH);
+  axis_floor_frac(Y, d.jHi, jF, tyF); axis_floor_frac(Y - 0.5f, d.jHi, jH, tyH);
+  axis_floor_frac(Z, d.kHi, kF, tzF); axis_floor_frac(Z - 0.5f, d.kHi, kH, tzH);
   S.idx[0] = ((unsigned)kH * ny + (unsigned)jH) * (nx + 1) + (unsigned)iF;
   S.tx[0] = txF; S.ty[0] = tyH; S.tz[0] = tzH;
   S.idx[1] = uN + ((unsigned)kH * (ny + 1) + (unsigned)jF) * nx + (unsigned)iH;

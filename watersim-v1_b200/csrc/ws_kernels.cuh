@@ -7,6 +7,8 @@ struct AdvectParams {
   double rainTe, rainLiftAge;
   double windS[3];
   int ceilReflect;
+  // what every particle's FP32 arithmetic uses of the above and the grid
+  float picF, flipF, maxSpeedF, halfDt, lo[3], hi[3], domIn2, damp, drag, rockDrag;
 };
 
 struct HeatParams {
@@ -22,7 +24,7 @@ struct PhaseParams {
 };
 
 // ---- ws_grid.cu
-void launch_static_types(const Dims& d, const TerrainDev& t, double coreR, uint8_t* st, cudaStream_t s);
+void launch_static_types(const Dims& d, const TerrainDev& t, double coreR, uint8_t* st, uint8_t* nearRock, cudaStream_t s);
 void launch_gravity_geometry(const Dims& d, double oceanR, float* g, cudaStream_t s);
 // bricks: clear the accumulator of the last substep's work list only
 void launch_clear_raster(const Dims& d, const GridDev& g, DevStatus* st, const BrickSet& B, bool bricks, cudaStream_t s);

@@ -13,12 +13,10 @@
 #include <atomic>
 #include <thread>
 
-// a marching-tets mesh in device memory: vertices (pos, nrm: 3 floats each),
-// the per-block emission offsets, both grown on demand
+// a marching-tets mesh in device memory: vertices (pos, nrm: 3 floats each), grown on demand
 struct MeshBuf {
   float *pos = nullptr, *nrm = nullptr;
-  long long* offs = nullptr;
-  long long cap = 0, offsCap = 0, verts = 0;
+  long long cap = 0, verts = 0;
 };
 
 struct ws_handle {
@@ -101,8 +99,7 @@ struct ws_handle {
   // metaball corner field: FP64 accumulator and its float copy, (m+1)^3 corners
   double* mbAcc = nullptr;
   float* mbField = nullptr;
-  double2* mbPartials = nullptr;
-  long long mbCorners = 0, mbCells = 0;
+  long long mbCorners = 0;
   int mbM = 0;
   // render-side particle prep: sorted draw list + scratch, sized for capacity
   RenderOut rdr{};
@@ -225,8 +222,8 @@ static void free_all(ws_handle* h) {
   if (h->curr.cfx) { cudaFree(h->curr.cfx); cudaFree(h->curr.cfy); cudaFree(h->curr.cfz); }
   if (h->currWaves) cudaFree(h->currWaves);
   for (MeshBuf* mb : { &h->surf, &h->mball })
-    for (void* b : { (void*)mb->pos, (void*)mb->nrm, (void*)mb->offs }) if (b) cudaFree(b);
-  for (void* b : { (void*)h->mbAcc, (void*)h->mbField, (void*)h->mbPartials }) if (b) cudaFree(b);
+    for (void* b : { (void*)mb->pos, (void*)mb->nrm }) if (b) cudaFree(b);
+  for (void* b : { (void*)h->mbAcc, (void*)h->mbField }) if (b) cudaFree(b);
   for (void* b : { (void*)h->balls, (void*)h->sv, (void*)h->ballHist, (void*)h->ballSurf }) if (b) cudaFree(b);
   for (float* b : { h->rdr.pos, h->rdr.col, h->rdr.alpha, h->rdr.size, h->rdr.sprite }) if (b) cudaFree(b);
   if (h->rdrScratch) cudaFree(h->rdrScratch);
@@ -716,11 +713,11 @@ static ws_status mt_scratch(ws_handle* h, long long nCells, void** out) {
   return WS_OK;
 }
 static ws_status mt_volume(ws_handle* h, double iso, double* vol, int64_t* cnt) {
-  if ((long long)grid_for(h->d.nCells, 128) > h->partialsCap) return fail(h, WS_ERR_RANGE, "partials too small");
   void* scr = nullptr;
   ws_status s = mt_scratch(h, h->d.nCells, &scr); if (s) return s;
-  launch_mt_volume(h->d, h->dens, iso, h->partials, h->red, scr, h->stream);
-  s = check_launch(h, 6); if (s) return s;
+  const int n = launch_mt_list(h->d, h->dens, iso, scr, h->stream) +
+                launch_mt_emit(h->d, h->dens, iso, 0, nullptr, nullptr, h->red, scr, h->stream);
+  s = check_launch(h, n); if (s) return s;
   WS_TRY(cudaMemcpyAsync(h->redHost, h->red, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream));
   WS_TRY(cudaStreamSynchronize(h->stream));
   if (vol) *vol = std::fabs(h->redHost[0]);
@@ -1961,27 +1958,21 @@ extern "C" ws_status ws_unet_load(ws_handle* h, const void* buf, int64_t size) {
 
 // ------------------------------------------------------------ surface mesh
 // MarchingTetrahedra.build (js/surface.js:66-177) of a corner field on the
-// lattice dd into mb, vertices in the reference's emission order. partials
-// holds grid_for(dd.nCells, 128) + 1 entries; the volume pass leaves the
-// per-block vertex counts there for the emission scan.
-static ws_status mt_build(ws_handle* h, const Dims& dd, const float* field, double iso, double2* partials, MeshBuf& mb,
-                          int64_t* vertices, double* volume) {
-  const long long nb = grid_for(dd.nCells, 128);
+// lattice dd into mb, vertices in the reference's emission order. The buffers'
+// present size is tried first; a larger mesh grows them and emits once more.
+static ws_status mt_build(ws_handle* h, const Dims& dd, const float* field, double iso, MeshBuf& mb, int64_t* vertices,
+                          double* volume) {
   void* scr = nullptr;
   ws_status s = mt_scratch(h, dd.nCells, &scr); if (s) return s;
-  launch_mt_volume(dd, field, iso, partials, h->red, scr, h->stream);
-  s = check_launch(h, 6); if (s) return s;
-  WS_TRY(cudaMemcpyAsync(h->redHost, h->red, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream));
-  WS_TRY(cudaStreamSynchronize(h->stream));
-  const double vol = std::fabs(h->redHost[0]);
-  const long long cnt = llround(h->redHost[1]);
-  if (nb + 1 > mb.offsCap) {
-    if (mb.offs) cudaFree(mb.offs);
-    mb.offs = nullptr; mb.offsCap = 0;
-    WS_TRY(cudaMalloc(&mb.offs, sizeof(long long) * (size_t)(nb + 1)));
-    mb.offsCap = nb + 1;
-  }
-  if (cnt > mb.cap) {
+  int n = launch_mt_list(dd, field, iso, scr, h->stream);
+  long long cnt = 0;
+  for (;;) {
+    n += launch_mt_emit(dd, field, iso, mb.cap, mb.pos, mb.nrm, h->red, scr, h->stream);
+    if ((s = check_launch(h, n))) return s;
+    WS_TRY(cudaMemcpyAsync(h->redHost, h->red, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream));
+    WS_TRY(cudaStreamSynchronize(h->stream));
+    cnt = llround(h->redHost[1]);
+    if (cnt <= mb.cap) break;
     long long cap = std::max<long long>(cnt + cnt / 4, 1 << 16);
     if (mb.pos) cudaFree(mb.pos);
     if (mb.nrm) cudaFree(mb.nrm);
@@ -1989,10 +1980,9 @@ static ws_status mt_build(ws_handle* h, const Dims& dd, const float* field, doub
     WS_TRY(cudaMalloc(&mb.pos, sizeof(float) * 3 * (size_t)cap));
     WS_TRY(cudaMalloc(&mb.nrm, sizeof(float) * 3 * (size_t)cap));
     mb.cap = cap;
+    n = 0;
   }
-  launch_mt_mesh(dd, field, iso, partials, mb.offs, mb.cap, mb.pos, mb.nrm, scr, h->stream);
-  if ((s = check_launch(h, 2))) return s;
-  WS_TRY(cudaStreamSynchronize(h->stream));
+  const double vol = std::fabs(h->redHost[0]);
   mb.verts = cnt;
   if (vertices) *vertices = cnt;
   if (volume) *volume = vol;
@@ -2012,8 +2002,7 @@ extern "C" ws_status ws_surface_mesh(ws_handle* h, double iso, int64_t* vertices
   if (!h) return WS_ERR_INVALID;
   cudaSetDevice(h->device);
   ws_status s = sync_status(h); if (s) return s;
-  if ((long long)grid_for(h->d.nCells, 128) + 1 > h->partialsCap) return fail(h, WS_ERR_RANGE, "partials too small");
-  return mt_build(h, h->d, h->dens, iso, h->partials, h->surf, vertices, volume);
+  return mt_build(h, h->d, h->dens, iso, h->surf, vertices, volume);
 }
 extern "C" ws_status ws_surface_download(ws_handle* h, float* pos, float* nrm, int64_t max_vertices) {
   if (h && h->asyncRunning.load(std::memory_order_acquire)) return WS_ERR_BUSY;
@@ -2058,19 +2047,13 @@ extern "C" ws_status ws_metaball_mesh(ws_handle* h, double tension, double detai
     WS_TRY(cudaMalloc(&h->mbField, sizeof(float) * (size_t)corners));
     h->mbCorners = corners;
   }
-  if (cells > h->mbCells) {
-    if (h->mbPartials) cudaFree(h->mbPartials);
-    h->mbPartials = nullptr; h->mbCells = 0;
-    WS_TRY(cudaMalloc(&h->mbPartials, sizeof(double2) * (size_t)(grid_for(cells, 128) + 1)));
-    h->mbCells = cells;
-  }
   h->mbM = m;
   launch_metaball_field(parts_of(h), m, mdx, R * R, rad, h->mbAcc, h->mbField, h->stream);
   if ((s = check_launch(h, h->S.nP ? 2 : 1))) return s;
   Dims dd = h->d;
   dd.nx = dd.ny = dd.nz = m; dd.dx = mdx; dd.nCells = cells;
   dims_fastdiv(dd);
-  return mt_build(h, dd, h->mbField, iso, h->mbPartials, h->mball, vertices, volume);
+  return mt_build(h, dd, h->mbField, iso, h->mball, vertices, volume);
 }
 extern "C" ws_status ws_metaball_download(ws_handle* h, float* pos, float* nrm, int64_t max_vertices) {
   if (h && h->asyncRunning.load(std::memory_order_acquire)) return WS_ERR_BUSY;

@@ -60,6 +60,9 @@ void launch_extract_weight(const Dims& d, const float2* acc, float* out, long lo
 // ---- ws_particles.cu
 void launch_g2p_advect(const Dims& d, const GridDev& g, const PartsDev& P, const TerrainDev& t,
                        const AdvectParams& ap, DevStatus* st, cudaStream_t s);
+// copies between device memory and mapped host memory, in one launch
+struct HostCopies { const void* from[16]; void* to[16]; unsigned bytes[16]; int n; };
+void launch_host_copies(const HostCopies& c, cudaStream_t s);
 void launch_compact(const uint8_t* fl, int nP, int mode, int* blockCounts, int* out, int* total, cudaStream_t s);
 void launch_vapor_advect(const Dims& d, const GridDev& g, const PartsDev& P, const TerrainDev& t, const AdvectParams& ap,
                          const int* vIdx, const int* nV, uint32_t* rng, DevStatus* st, cudaStream_t s);

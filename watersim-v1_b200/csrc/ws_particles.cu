@@ -2,6 +2,7 @@
 // (js/solver.js:1646-2292), the serial-order vapour pass, order-preserving
 // compaction, and the interaction impulses (:3852-3908).
 #include "ws_kernels.cuh"
+#include <algorithm>
 
 // ------------------------------------------------------------ fused G2P + advect
 // One thread per particle. The G2P part (_g2pChunk :1646-1756) leaves the
@@ -315,6 +316,24 @@ void launch_g2p_advect(const Dims& d, const GridDev& g, const PartsDev& P, const
   const G2pArgs A{ d, g, P, t, ap, st };
   if (P.nP <= 148 * 256) k_g2p_advect<false><<<grid_for(P.nP, 256), 256, 0, s>>>(A);
   else k_g2p_advect<true><<<grid_for(P.nP, 256), 256, 0, s>>>(A);
+}
+
+// ------------------------------------------------------------ small host transfers
+// One array per blockIdx.y, both ends 16-byte aligned. Uncached loads: the host may have rewritten the buffer since the
+// last launch. Bound by the link's latency and rate.
+__global__ void __launch_bounds__(256) k_host_copies(HostCopies c) {
+  const unsigned t = blockIdx.x * 256 + threadIdx.x, step = gridDim.x * 256, bytes = c.bytes[blockIdx.y];
+  const char* from = (const char*)c.from[blockIdx.y];
+  char* to = (char*)c.to[blockIdx.y];
+  const unsigned n16 = bytes >> 4;
+  for (unsigned i = t; i < n16; i += step) ((uint4*)to)[i] = __ldcv((const uint4*)from + i);
+  for (unsigned i = (n16 << 4) + t; i < bytes; i += step) to[i] = __ldcv(from + i);
+}
+void launch_host_copies(const HostCopies& c, cudaStream_t s) {
+  unsigned most = 0;
+  for (int i = 0; i < c.n; i++) most = std::max(most, c.bytes[i]);
+  const unsigned bx = std::min(std::max((most + 4095u) / 4096u, 1u), 148u);
+  k_host_copies<<<dim3(bx, (unsigned)c.n), 256, 0, s>>>(c);
 }
 
 // ------------------------------------------------------------ order-preserving compaction

@@ -55,7 +55,8 @@ struct ws_handle {
   double2* partials = nullptr;
   int partialsCap = 0;
   double* red = nullptr;                // device reduction outputs
-  double* redHost = nullptr;            // pinned
+  double* redHost = nullptr;            // pinned: reductions write their results here
+  unsigned* ticket = nullptr;           // of a reduction's last block (0 between launches)
   uint32_t* rng = nullptr;              // device: cfS, bfS, evS
   int *blockCounts = nullptr, *list = nullptr, *listCount = nullptr;
   uint8_t* cand = nullptr;
@@ -202,7 +203,7 @@ extern "C" ws_status ws_default_params(ws_params* p) {
 
 static void free_all(ws_handle* h) {
   void* bufs[] = { h->type, h->staticTypes, h->nearRock, h->valid, h->diag8, h->vel, h->velO, h->gvel, h->q, h->rhs, h->pw,
-                   h->vort, h->dens, h->acc, h->tsolid, h->tR, h->st, h->partials, h->red, h->rng,
+                   h->vort, h->dens, h->acc, h->tsolid, h->tR, h->st, h->partials, h->red, h->ticket, h->rng,
                    h->blockCounts, h->list, h->listCount, h->cand, h->cellCnt, h->cellSum, h->cellChange,
                    h->parts.px, h->parts.py, h->parts.pz, h->parts.pvx, h->parts.pvy, h->parts.pvz, h->parts.pT,
                    h->parts.pAir, h->parts.pLight, h->parts.pWx, h->parts.pWy, h->parts.pWz, h->parts.pPh,
@@ -290,7 +291,7 @@ extern "C" ws_status ws_create(const ws_config* cfg, ws_handle** out) {
   AL(h->type, N) AL(h->staticTypes, N) AL(h->nearRock, N) AL(h->diag8, N) AL(h->valid, F)
   AL(h->vel, F) AL(h->velO, F) AL(h->gvel, F) AL(h->acc, F)
   AL(h->q, N) AL(h->rhs, N) AL(h->pw, N) AL(h->vort, 7 * N) AL(h->dens, ND)
-  AL(h->st, 1) AL(h->red, 8) AL(h->rng, 4)
+  AL(h->st, 1) AL(h->red, 8) AL(h->ticket, 1) AL(h->rng, 4)
   AL(h->cellCnt, N) AL(h->cellSum, N) AL(h->cellChange, N)
   PartsDev& pp = h->parts;
   AL(pp.px, P) AL(pp.py, P) AL(pp.pz, P) AL(pp.pvx, P) AL(pp.pvy, P) AL(pp.pvz, P)
@@ -766,9 +767,8 @@ static ws_status mt_volume(ws_handle* h, double iso, double* vol, int64_t* cnt) 
   void* scr = nullptr;
   ws_status s = mt_scratch(h, h->d.nCells, &scr); if (s) return s;
   const int n = launch_mt_list(h->d, h->dens, iso, scr, h->stream) +
-                launch_mt_emit(h->d, h->dens, iso, 0, nullptr, nullptr, h->red, scr, h->stream);
+                launch_mt_emit(h->d, h->dens, iso, 0, nullptr, nullptr, h->redHost, scr, h->stream);
   s = check_launch(h, n); if (s) return s;
-  WS_TRY(cudaMemcpyAsync(h->redHost, h->red, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream));
   WS_TRY(cudaStreamSynchronize(h->stream));
   if (vol) *vol = std::fabs(h->redHost[0]);
   if (cnt) *cnt = (int64_t)llround(h->redHost[1]);
@@ -806,9 +806,8 @@ static ws_status splat_and_iso(ws_handle* h) {
   return WS_OK;
 }
 static ws_status particle_reduce(ws_handle* h, int mode, double mp, double out[3]) {
-  launch_particle_reduce(parts_of(h), mode, mp, (double*)h->partials, h->red, h->stream);
-  ws_status s = check_launch(h, 2); if (s) return s;
-  WS_TRY(cudaMemcpyAsync(h->redHost, h->red, sizeof(double) * 3, cudaMemcpyDeviceToHost, h->stream));
+  launch_particle_reduce(parts_of(h), mode, mp, (double*)h->partials, h->ticket, h->redHost, h->stream);
+  ws_status s = check_launch(h, 1); if (s) return s;
   WS_TRY(cudaStreamSynchronize(h->stream));
   out[0] = h->redHost[0]; out[1] = h->redHost[1]; out[2] = h->redHost[2];
   return WS_OK;
@@ -2017,10 +2016,9 @@ static ws_status mt_build(ws_handle* h, const Dims& dd, const float* field, doub
   int n = launch_mt_list(dd, field, iso, scr, h->stream);
   long long cnt = 0;
   for (;;) {
-    n += launch_mt_emit(dd, field, iso, mb.cap, mb.pos, mb.nrm, h->red, scr, h->stream);
+    n += launch_mt_emit(dd, field, iso, mb.cap, mb.pos, mb.nrm, h->redHost, scr, h->stream);
     if ((s = check_launch(h, n))) return s;
-    WS_TRY(cudaMemcpyAsync(h->redHost, h->red, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream));
-    WS_TRY(cudaStreamSynchronize(h->stream));
+    if ((s = sync_status(h))) return s;            // the one wait: results, and faults latched before
     cnt = llround(h->redHost[1]);
     if (cnt <= mb.cap) break;
     long long cap = std::max<long long>(cnt + cnt / 4, 1 << 16);
@@ -2051,7 +2049,6 @@ extern "C" ws_status ws_surface_mesh(ws_handle* h, double iso, int64_t* vertices
   join_copies(h);
   if (!h) return WS_ERR_INVALID;
   cudaSetDevice(h->device);
-  ws_status s = sync_status(h); if (s) return s;
   return mt_build(h, h->d, h->dens, iso, h->surf, vertices, volume);
 }
 extern "C" ws_status ws_surface_download(ws_handle* h, float* pos, float* nrm, int64_t max_vertices) {
@@ -2078,7 +2075,6 @@ extern "C" ws_status ws_metaball_mesh(ws_handle* h, double tension, double detai
   join_copies(h);
   if (!h) return WS_ERR_INVALID;
   cudaSetDevice(h->device);
-  ws_status s = sync_status(h); if (s) return s;
   double f = 1;
   if (std::isfinite(detail) && detail > 0) f = detail < 0.5 ? 0.5 : (detail > 1.6 ? 1.6 : detail);
   const int nx = h->d.nx;
@@ -2099,7 +2095,7 @@ extern "C" ws_status ws_metaball_mesh(ws_handle* h, double tension, double detai
   }
   h->mbM = m;
   launch_metaball_field(parts_of(h), m, mdx, R * R, rad, h->mbAcc, h->mbField, h->stream);
-  if ((s = check_launch(h, h->S.nP ? 2 : 1))) return s;
+  ws_status s = check_launch(h, h->S.nP ? 2 : 1); if (s) return s;
   Dims dd = h->d;
   dd.nx = dd.ny = dd.nz = m; dd.dx = mdx; dd.nCells = cells;
   dims_fastdiv(dd);

@@ -680,6 +680,22 @@ void launch_splat(const Dims& d, const GridDev& g, const PartsDev& P, double spa
   k_splat<<<grid_for(P.nP, 256), 256, 0, s>>>(d, g, P, spacing);
 }
 
+// whether this block is the last of `blocks` to come here, with the others'
+// global writes visible; the ticket is back at zero afterwards. Every thread
+// of those blocks calls.
+__device__ __forceinline__ bool last_block(unsigned* ticket, unsigned blocks) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(ticket, 1u) == blocks - 1;
+    if (last) *ticket = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
+}
+
 // ------------------------------------------------------------ marching tets (FP64)
 // MarchingTetrahedra.build (js/surface.js:66-177): six tets per cell, up to
 // two triangles each, vertices in the reference's order (cells in index
@@ -773,7 +789,7 @@ __global__ void __launch_bounds__(256) k_mt_count(Dims d, const float* __restric
     tot[blockIdx.x] = (unsigned long long)(mine >> 16) << 34 | (mine & 0xffffu);
   }
 }
-// exclusive scan in place; the total lands in tot[nb]
+// exclusive scan in place; the total lands in tot[nb], the emission's ticket (0) behind it
 __global__ void __launch_bounds__(1024) k_mt_scan(unsigned long long* __restrict__ tot, int nb) {
   __shared__ unsigned long long ws[32];
   unsigned long long carry = 0;
@@ -795,7 +811,7 @@ __global__ void __launch_bounds__(1024) k_mt_scan(unsigned long long* __restrict
     carry += ws[31];
     __syncthreads();                                     // ws is rewritten by the next round
   }
-  if (threadIdx.x == 0) tot[nb] = carry;
+  if (threadIdx.x == 0) { tot[nb] = carry; tot[nb + 1] = 0; }
 }
 // (cell, its first triangle) of every listed cell
 __global__ void __launch_bounds__(256) k_mt_list(const uint8_t* __restrict__ cfg, const unsigned long long* __restrict__ tot,
@@ -828,14 +844,15 @@ __global__ void __launch_bounds__(256) k_mt_list(const uint8_t* __restrict__ cfg
 // (FP64 division and square root, five per vertex) at the ten blocks an SM
 // whose vertices fit. A thread per cell that walked its triangles, once to
 // count and once to emit, took 53 + 95 us for 1.3M vertices at 128^3 (29 + 35
-// at 48^3, where its chain was the whole time); this: 54 and 14. Rounds of 32
+// at 48^3, where its chain was the whole time); this, with the sums of the last
+// block, which writes them to host memory: 57 and 18. Rounds of 32
 // cells and 128 threads: the same.
 // pos null, or a mesh beyond maxVerts: the volume only, of whole cells
 constexpr int kMtCells = 16, kMtThreads = 4 * kMtCells;
 __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __restrict__ dens, double iso, float isoF,
                                                  const uint2* __restrict__ list, const unsigned long long* __restrict__ total,
                                                  long long maxVerts, float* __restrict__ pos, float* __restrict__ nrm,
-                                                 double* __restrict__ partials) {
+                                                 double* __restrict__ partials, unsigned* ticket, double* __restrict__ out) {
   __shared__ float cv[kMtCells][9];
   __shared__ double gr[3][kMtCells * 8];
   __shared__ double P[3][kMtCells * kMtVerts], N[3][kMtCells * kMtVerts];
@@ -846,12 +863,14 @@ __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __r
   __shared__ uint8_t cfg[kMtCells], sFrom[kMtEdges], sTo[kMtEdges], sId[6][6], sTet[6][4], sCase[16][2][3], sNTri[16];
   __shared__ double sv[kMtThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31;
+  const unsigned n = (unsigned)(*total >> 34);
+  const unsigned blocks = min(gridDim.x, max((n + kMtCells - 1) / kMtCells, 1u));   // those with cells (one without any)
+  if (blockIdx.x >= blocks) return;
   for (int t = tid; t < 16 * 6; t += kMtThreads) ((uint8_t*)sCase)[t] = ((const uint8_t*)g_mt.cases)[t];
   if (tid < kMtEdges) { sFrom[tid] = g_mt.from[tid]; sTo[tid] = g_mt.to[tid]; }
   if (tid < 36) ((uint8_t*)sId)[tid] = ((const uint8_t*)g_mt.id)[tid];
   if (tid < 24) ((uint8_t*)sTet)[tid] = ((const uint8_t*)g_mt.tet)[tid];
   if (tid < 16) sNTri[tid] = g_mt.nTri[tid];
-  const unsigned n = (unsigned)(*total >> 34);
   const unsigned sj = (unsigned)d.nx + 1u, sk = ((unsigned)d.ny + 1u) * sj;
   const double dx = d.dx, r2dx = 0.5 * d.rdx;
   double vol = 0;
@@ -969,27 +988,24 @@ __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __r
     for (int w = 1; w < kMtThreads / 32; w++) vol += sv[w];
     partials[blockIdx.x] = vol;
   }
-}
-// fixed-order sum of the blocks' volumes, and the vertex count
-__global__ void k_mt_total(const double* __restrict__ partials, int n, const unsigned long long* __restrict__ total,
-                           double* __restrict__ out) {
-  __shared__ double sa[8];
-  double a = 0;
-  for (int i = threadIdx.x; i < n; i += 256) a += partials[i];
-  a = warp_sum(a);
-  if ((threadIdx.x & 31) == 0) sa[threadIdx.x >> 5] = a;
+  // the last block: the volumes in a fixed order, and the vertex count
+  if (!last_block(ticket, blocks)) return;
+  vol = 0;
+  for (unsigned i = tid; i < blocks; i += kMtThreads) vol += __ldcg(partials + i);
+  vol = warp_sum(vol);
+  if (lane == 0) sv[tid >> 5] = vol;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; w++) a += sa[w];
-    out[0] = a; out[1] = 3.0 * (double)(*total & ((1ull << 34) - 1));
+  if (tid == 0) {
+    for (int w = 1; w < kMtThreads / 32; w++) vol += sv[w];
+    out[0] = vol; out[1] = 3.0 * (double)(*total & ((1ull << 34) - 1));
   }
 }
-// scratch: list (8 bytes a cell), block totals, partial volumes, sign patterns
+// scratch: list (8 bytes a cell), block totals and ticket, partial volumes, sign patterns
 static int mt_blocks(long long nCells) { return (int)grid_for(nCells, kMtBlock); }
 constexpr int kMtGrid = 148 * 10;
 size_t mt_scratch_bytes(long long nCells) {
   const size_t nb = (size_t)mt_blocks(nCells);
-  return 8 * (size_t)nCells + 8 * (nb + 1) + 8 * kMtGrid + kMtBlock * nb;
+  return 8 * (size_t)nCells + 8 * (nb + 2) + 8 * kMtGrid + kMtBlock * nb;
 }
 struct MtScratch { uint2* list; unsigned long long* tot; double* partials; uint8_t* cfg; int nb; };
 static MtScratch mt_carve(void* scratch, long long nCells) {
@@ -997,7 +1013,7 @@ static MtScratch mt_carve(void* scratch, long long nCells) {
   char* q = (char*)scratch;
   m.nb = mt_blocks(nCells);
   m.list = (uint2*)q; q += 8 * (size_t)nCells;
-  m.tot = (unsigned long long*)q; q += 8 * (size_t)(m.nb + 1);
+  m.tot = (unsigned long long*)q; q += 8 * (size_t)(m.nb + 2);
   m.partials = (double*)q; q += 8 * kMtGrid;
   m.cfg = (uint8_t*)q;
   return m;
@@ -1019,24 +1035,27 @@ int launch_mt_emit(const Dims& d, const float* dens, double iso, long long maxVe
                    void* scratch, cudaStream_t s) {
   const MtScratch m = mt_carve(scratch, d.nCells);
   const int grid = (int)std::min<long long>(grid_for(d.nCells, kMtCells), kMtGrid);
-  k_mt_emit<<<grid, kMtThreads, 0, s>>>(d, dens, iso, iso_floor(iso), m.list, m.tot + m.nb, maxVerts, pos, nrm, m.partials);
-  k_mt_total<<<1, 256, 0, s>>>(m.partials, grid, m.tot + m.nb, out);
-  return 2;
+  k_mt_emit<<<grid, kMtThreads, 0, s>>>(d, dens, iso, iso_floor(iso), m.list, m.tot + m.nb, maxVerts, pos, nrm, m.partials,
+                                           (unsigned*)(m.tot + m.nb + 1), out);
+  return 1;
 }
 
 // ------------------------------------------------------------ particle reductions
 // mode 0: kinetic energy sum of 0.5 mp v^2 (FP64); mode 1: census counts
 // (liquid 0/1/4, ice 5, vapour 2/3) as exact FP64 integers. Both read their
-// input once (12 or 1 bytes per particle) and are bound by that read and two
-// launches: persistent blocks, four particles per thread and step (the
+// input once (12 or 1 bytes per particle) and are bound by that read and the
+// launch: persistent blocks, four particles per thread and step (the
 // arrays are separate allocations and p % 4 == 0, so the 16- and 4-byte
-// loads are aligned), one partial per block. The partials are then summed by
-// one warp per value, lanes striding the blocks and a fixed butterfly, so the
-// sums are the same on every call. A single thread adding one partial per 256
-// particles took 562 us of the 576 of a call at 1.86M particles (this: 13).
-constexpr int kReduceBlocks = 148 * 4;
-__global__ void __launch_bounds__(256) k_particle_reduce(PartsDev P, int mode, double mp, double* __restrict__ partials) {
-  __shared__ double s0[8], s1[8], s2[8];
+// loads are aligned), one partial per block. The last block sums the
+// partials, one warp per value, lanes striding the blocks and a fixed
+// butterfly, so the sums are the same on every call, and writes them where the
+// host reads them. A single thread adding one partial per 256 particles took
+// 562 us of the 576 of a call at 1.86M particles; a second kernel and a copy
+// back, 29 us a call; this, 18.
+constexpr int kReduceBlocks = 148 * 2, kReduceThreads = 512;
+__global__ void __launch_bounds__(kReduceThreads) k_particle_reduce(PartsDev P, int mode, double mp, double* __restrict__ partials,
+                                                         unsigned* ticket, double* __restrict__ out) {
+  __shared__ double s0[kReduceThreads / 32], s1[kReduceThreads / 32], s2[kReduceThreads / 32];
   double a = 0, b = 0, c = 0;
   auto energy = [&](float x, float y, float z) {
     const double vx = x, vy = y, vz = z;
@@ -1067,22 +1086,19 @@ __global__ void __launch_bounds__(256) k_particle_reduce(PartsDev P, int mode, d
   if (threadIdx.x < 3) {
     const double* w = threadIdx.x == 0 ? s0 : threadIdx.x == 1 ? s1 : s2;
     double t = 0;
-    for (int k = 0; k < 8; k++) t += w[k];
+    for (int k = 0; k < kReduceThreads / 32; k++) t += w[k];
     partials[3 * blockIdx.x + threadIdx.x] = t;
   }
+  if (!last_block(ticket, gridDim.x) || wid >= 3) return;
+  double v = 0;                                              // one warp per value
+  for (int i = lane; i < (int)gridDim.x; i += 32) v += __ldcg(partials + 3 * i + wid);
+  v = warp_sum(v);
+  if (lane == 0) out[wid] = v;
 }
-__global__ void __launch_bounds__(96) k_reduce_triples(const double* __restrict__ partials, int n, double* __restrict__ out) {
-  const int v = threadIdx.x >> 5, lane = threadIdx.x & 31;   // one warp per value
-  double a = 0;
-  for (int i = lane; i < n; i += 32) a += partials[3 * i + v];
-  a = warp_sum(a);
-  if (lane == 0) out[v] = a;
-}
-void launch_particle_reduce(const PartsDev& P, int mode, double mp, double* partials, double* out, cudaStream_t s) {
+void launch_particle_reduce(const PartsDev& P, int mode, double mp, double* partials, unsigned* ticket, double* out, cudaStream_t s) {
   // one partial per 256 particles at most: the caller's buffer holds three per 256 of capacity
-  const int nb = (int)std::min<long long>(grid_for(P.nP > 0 ? P.nP : 1, 256), kReduceBlocks);
-  k_particle_reduce<<<nb, 256, 0, s>>>(P, mode, mp, partials);
-  k_reduce_triples<<<1, 96, 0, s>>>(partials, nb, out);
+  const int nb = (int)std::min<long long>(grid_for(P.nP > 0 ? P.nP : 1, kReduceThreads), kReduceBlocks);
+  k_particle_reduce<<<nb, kReduceThreads, 0, s>>>(P, mode, mp, partials, ticket, out);
 }
 
 // ------------------------------------------------------------ subsurface currents

@@ -97,7 +97,7 @@ void launch_currents(const Dims& d, const PartsDev& P, const CurrField& F, doubl
                      double oceanR, double coreR, double dt, cudaStream_t s);
 // marching tets in scratch (mt_scratch_bytes(d.nCells) bytes): the cells that
 // straddle iso, then (at the same iso) the signed volume and the vertex count
-// into out[0..1] and, with pos, the vertices of the cells that fit in maxVerts.
+// into out[0..1] (device or mapped host memory) and, with pos, the vertices of the cells that fit in maxVerts.
 // Both return the kernels launched.
 size_t mt_scratch_bytes(long long nCells);
 int launch_mt_list(const Dims& d, const float* dens, double iso, void* scratch, cudaStream_t s);
@@ -118,7 +118,8 @@ void launch_metaball_field(const PartsDev& P, int m, double mdx, double R2, int 
                            cudaStream_t s);
 size_t render_scratch_bytes(long long capacity);
 void launch_render_particles(const RenderCfg& c, const PartsDev& P, void* scratch, RenderOut o, cudaStream_t s);
-void launch_particle_reduce(const PartsDev& P, int mode, double mp, double* partials, double* out, cudaStream_t s);
+// ticket: zero before the first call (and after each); out: three doubles, device or mapped host memory
+void launch_particle_reduce(const PartsDev& P, int mode, double mp, double* partials, unsigned* ticket, double* out, cudaStream_t s);
 
 // ---- ws_queries.cu
 void launch_wave_impulse(const Dims& d, const PartsDev& P, const double dir[3], uint32_t s0, double dvx, cudaStream_t s);

@@ -400,12 +400,15 @@ void launch_compact(const uint8_t* fl, int nP, int mode, int* blockCounts, int* 
 
 // ------------------------------------------------------------ vapour pass
 // Atmospheric branch of _advectChunk (js/solver.js:1978-2174) with the
-// reference's serial LCG draws reproduced exactly: one CTA walks the vapour
-// list in index order, 1024 parcels at a time. Which parcels draw from _cfS
-// (ceiling bounce) depends only on each parcel's own state, so a block scan
-// gives each drawing parcel its position k in the stream and lcg_jump gives
-// its value; the floor draws (_bfS) depend on the ceiling outcome and get a
-// second scan. RNG states live in device memory between calls.
+// reference's serial LCG draws reproduced exactly: one cluster of eight blocks
+// walks the vapour list in index order, 4096 parcels at a time. Which parcels
+// draw from _cfS (ceiling bounce) depends only on each parcel's own state, so
+// a scan over the cluster gives each drawing parcel its position k in the
+// stream and lcg_jump gives its value; the floor draws (_bfS) depend on the
+// ceiling outcome and get a second scan. RNG states live in device memory
+// between calls. Bound by the chain of a round (double-precision roots and
+// divisions): one block of 1024 threads took 40 us for 4000 parcels, four
+// rounds; this, 11.8.
 __device__ __forceinline__ int block_excl_scan(int v, int* warpTot, int& total) {
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   int x = v;
@@ -423,17 +426,38 @@ __device__ __forceinline__ int block_excl_scan(int v, int* warpTot, int& total) 
   __syncthreads();
   return excl;
 }
-__global__ void __launch_bounds__(1024) k_vapor_advect(Dims d, GridDev g, PartsDev P, TerrainDev t, AdvectParams ap,
+// exclusive scan over the cluster's blocks in rank order: each block's total is
+// written to every block's tot[]. Two scans alternate, so a slot is written
+// again only after a later cluster barrier than the one its readers passed.
+constexpr int kVapBlocks = 8, kVapThreads = 512;
+__device__ __forceinline__ int cluster_excl_scan(int v, int* warpTot, int* tot, int rank, int& total) {
+  int mine;
+  int excl = block_excl_scan(v, warpTot, mine);
+  if (threadIdx.x < kVapBlocks) {
+    const unsigned at = (unsigned)__cvta_generic_to_shared(tot + rank);
+    unsigned far;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(at), "r"(threadIdx.x));
+    asm volatile("st.shared::cluster.s32 [%0], %1;" :: "r"(far), "r"(mine) : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  total = 0;
+#pragma unroll
+  for (int q = 0; q < kVapBlocks; q++) { if (q < rank) excl += tot[q]; total += tot[q]; }
+  return excl;
+}
+__global__ void __cluster_dims__(kVapBlocks, 1, 1) __launch_bounds__(kVapThreads) k_vapor_advect(Dims d, GridDev g, PartsDev P, TerrainDev t, AdvectParams ap,
                                                        const int* __restrict__ vIdx, const int* __restrict__ nVp,
                                                        uint32_t* __restrict__ rng, DevStatus* st) {
-  __shared__ int warpTot[32];
-  const int nV = *nVp;
+  __shared__ int warpTot[32], clTot[2][kVapBlocks];
+  const int nV = *nVp, rank = (int)blockIdx.x;          // the grid is one cluster
   uint32_t cfS = rng[0], bfS = rng[1];
   const double dx = d.dx, dt = ap.dt, maxSpeed = ap.maxSpeed, oceanR = ap.oceanR;
   const double cx = d.cx, cy = d.cy, cz = d.cz, domHi = d.domainR - dx * 0.02;
   int drawsA = 0, drawsB = 0;
-  for (int base = 0; base < nV; base += blockDim.x) {
-    int idx = base + threadIdx.x;
+  // no block's shared memory is written before it runs, nor after it leaves
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  for (int base = 0; base < nV; base += kVapBlocks * kVapThreads) {
+    int idx = base + rank * kVapThreads + threadIdx.x;
     bool act = idx < nV;
     int p = act ? vIdx[idx] : 0;
     double x = 0, y = 0, z = 0, Tv = 0, vCx = 0, vCy = 0, vCz = 0, vCr = 1, vrC2 = 0, prf = 0;
@@ -487,7 +511,7 @@ __global__ void __launch_bounds__(1024) k_vapor_advect(Dims d, GridDev g, PartsD
       }
     }
     int totA;
-    int kA = block_excl_scan(wantA, warpTot, totA);
+    int kA = cluster_excl_scan(wantA, warpTot, clTot[0], rank, totA);
     int wantB = 0; double fCx = 0, fCy = 0, fCz = 0, fCr = 1, vrF = 0;
     if (act) {
       if (wantA) {
@@ -505,7 +529,7 @@ __global__ void __launch_bounds__(1024) k_vapor_advect(Dims d, GridDev g, PartsD
     }
     cfS = lcg_jump(cfS, (uint32_t)totA); drawsA += totA;
     int totB;
-    int kB = block_excl_scan(wantB, warpTot, totB);
+    int kB = cluster_excl_scan(wantB, warpTot, clTot[1], rank, totB);
     if (act) {
       if (wantB) {
         uint32_t sB = lcg_jump(bfS, (uint32_t)kB + 1u);
@@ -548,13 +572,14 @@ __global__ void __launch_bounds__(1024) k_vapor_advect(Dims d, GridDev g, PartsD
       P.pvx[p] = fvx; P.pvy[p] = fvy; P.pvz[p] = fvz; P.pAir[p] = fAir; P.pflag[p] = (uint8_t)fl;
     }
     bfS = lcg_jump(bfS, (uint32_t)totB); drawsB += totB;
-    __syncthreads();
   }
-  if (threadIdx.x == 0) { rng[0] = cfS; rng[1] = bfS; st->cfA = drawsA; st->bfB = drawsB; }
+  // every block has read its stream states; only the first writes them back
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  if (rank == 0 && threadIdx.x == 0) { rng[0] = cfS; rng[1] = bfS; st->cfA = drawsA; st->bfB = drawsB; }
 }
 void launch_vapor_advect(const Dims& d, const GridDev& g, const PartsDev& P, const TerrainDev& t, const AdvectParams& ap,
                          const int* vIdx, const int* nV, uint32_t* rng, DevStatus* st, cudaStream_t s) {
-  k_vapor_advect<<<1, 1024, 0, s>>>(d, g, P, t, ap, vIdx, nV, rng, st);
+  k_vapor_advect<<<kVapBlocks, kVapThreads, 0, s>>>(d, g, P, t, ap, vIdx, nV, rng, st);
 }
 
 // ------------------------------------------------------------ impulses

@@ -336,25 +336,30 @@ __global__ void __launch_bounds__(1024) k_evap_band(const double* __restrict__ w
   if (tid == 0) { st->evKeff = keff; st->evIrr = ~0ull; st->evNC = *nCp; }
 }
 // Each window: its candidates' base states and thresholds in shared memory,
-// then one warp per tabulated input.
-__global__ void __launch_bounds__(1024) k_evap_table(const long long* __restrict__ thr, const int* __restrict__ nCp,
-                                                     int t0, const uint32_t* __restrict__ sStart,
-                                                     const int* __restrict__ L, const DevStatus* __restrict__ st,
-                                                     uint32_t* __restrict__ bOut, unsigned short* __restrict__ table) {
+// then one warp per tabulated input. A surface of 20k candidates has five
+// windows, so blocks along y share a window's inputs: with one block of 32
+// warps per window five SMs worked through eight rounds, 114 us; now 24.
+constexpr int kEvTableThreads = 256;
+__global__ void __launch_bounds__(kEvTableThreads) k_evap_table(const long long* __restrict__ thr, const int* __restrict__ nCp,
+                                                                int t0, const uint32_t* __restrict__ sStart,
+                                                                const int* __restrict__ L, const DevStatus* __restrict__ st,
+                                                                uint32_t* __restrict__ bOut, unsigned short* __restrict__ table) {
   __shared__ uint32_t sb[kEvW];
   __shared__ long long sthr[kEvW];
-  const int nC = *nCp, w = blockIdx.x;
-  if (w >= ev_windows(nC, t0)) return;
+  constexpr int warps = kEvTableThreads / 32;
+  const int nC = *nCp, w = blockIdx.x, keff = st->evKeff;
+  if (w >= ev_windows(nC, t0) || (int)blockIdx.y * warps >= keff) return;
   const int lo = t0 + w * kEvW, n = min(kEvW, nC - lo);
-  const uint32_t s0 = *sStart;
-  for (int j = (int)threadIdx.x; j < n; j += blockDim.x) {
-    const uint32_t bj = lcg_jump(s0, (uint32_t)(lo - t0 + j + 1));
-    sb[j] = bj; bOut[lo + j] = bj;
+  uint32_t A, C, bj = lcg_jump(*sStart, (uint32_t)(lo - t0 + (int)threadIdx.x + 1));
+  lcg_affine(kEvTableThreads, A, C);
+  for (int j = (int)threadIdx.x; j < n; j += kEvTableThreads, bj = A * bj + C) {
+    sb[j] = bj;
+    if (blockIdx.y == 0) bOut[lo + j] = bj;
     sthr[j] = thr[lo + j];
   }
   __syncthreads();
-  const int keff = st->evKeff, Lw = L[w];
-  for (int k = (int)(threadIdx.x >> 5); k < keff; k += (int)(blockDim.x >> 5)) {
+  const int Lw = L[w];
+  for (int k = (int)blockIdx.y * warps + (int)(threadIdx.x >> 5); k < keff; k += warps * (int)gridDim.y) {
     const int eo = ev_resolve(sb, sthr, n, Lw + k, [](int, int, uint32_t) {});
     if ((threadIdx.x & 31) == 0) table[(size_t)w * kEvKMax + k] = (unsigned short)(eo - (Lw + k));
   }
@@ -385,15 +390,21 @@ __global__ void __launch_bounds__(32) k_evap_chain(const int* __restrict__ nCp, 
     st->evSEnd = lcg_jump(*sStart, (uint32_t)(nC > t0 ? nC - t0 : 0) + 6u * (uint32_t)E);
   }
 }
-// One warp per window: replay its resolve and record each ejector (particle and decision state).
-__global__ void k_evap_emit(const int* __restrict__ nCp, int t0, const uint32_t* __restrict__ b,
+// One block per window: its candidates into shared memory, then one warp
+// replays its resolve and records each ejector (particle and decision state).
+// Bound by that warp's chain of 128 and more steps (20 us; from global memory 35).
+__global__ void __launch_bounds__(256) k_evap_emit(const int* __restrict__ nCp, int t0, const uint32_t* __restrict__ b,
                             const long long* __restrict__ thr, const int* __restrict__ Ew, const int* __restrict__ list,
                             int eoff, int* __restrict__ ejP, uint32_t* __restrict__ ejS, DevStatus* st) {
-  const int nC = *nCp;
-  const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (w >= ev_windows(nC, t0)) return;          // uniform over the warp
-  const int lo = t0 + w * kEvW;
-  ev_resolve(b + lo, thr + lo, min(kEvW, nC - lo), Ew[w], [&](int j, int E, uint32_t u) {
+  __shared__ uint32_t sb[kEvW];
+  __shared__ long long sthr[kEvW];
+  const int nC = *nCp, w = (int)blockIdx.x;
+  if (w >= ev_windows(nC, t0)) return;
+  const int lo = t0 + w * kEvW, n = min(kEvW, nC - lo);
+  for (int j = (int)threadIdx.x; j < n; j += 256) { sb[j] = b[lo + j]; sthr[j] = thr[lo + j]; }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  ev_resolve(sb, sthr, n, Ew[w], [&](int j, int E, uint32_t u) {
     ejP[eoff + E] = list[lo + j];
     ejS[eoff + E] = u;
     // Regular kick: its three u1 draws (1, 3 and 5 after the decision) have states >= 5.
@@ -466,9 +477,11 @@ void launch_evap_pass(int nP, const int* list, const int* nC, const EvapScratch&
   const int nw = (int)ev_max_windows(nP);
   k_evap_wsum<<<nw, 256, 0, s>>>(es.thr, nC, t0, es.wsum);
   k_evap_band<<<1, 1024, 0, s>>>(es.wsum, nC, t0, es.L, st);
-  k_evap_table<<<nw, 1024, 0, s>>>(es.thr, nC, t0, sStart, es.L, st, es.b, es.table);
+  // up to one warp per input of the widest band, fewer where the windows alone fill the device
+  const int ny = std::max(1, std::min(kEvKMax * 32 / kEvTableThreads / 4, 148 * 16 / nw));
+  k_evap_table<<<dim3(nw, ny), kEvTableThreads, 0, s>>>(es.thr, nC, t0, sStart, es.L, st, es.b, es.table);
   k_evap_chain<<<1, 32, 0, s>>>(nC, t0, es.L, es.table, es.b, es.thr, sStart, es.Ew, st);
-  k_evap_emit<<<(nw + 3) / 4, 128, 0, s>>>(nC, t0, es.b, es.thr, es.Ew, list, eoff, es.ejP, es.ejS, st);
+  k_evap_emit<<<nw, 256, 0, s>>>(nC, t0, es.b, es.thr, es.Ew, list, eoff, es.ejP, es.ejS, st);
 }
 void launch_evap_apply(const Dims& d, const GridDev& g, const PartsDev& P, double freezeT, const EvapScratch& es,
                        int nEj, cudaStream_t s) {

@@ -290,10 +290,10 @@ def run_ours(args, rank, world, local_rank):
     return out, fs
 
 
-SOR_PATHS = {0: "none", 1: "grid-wide persistent (colour lists)", 2: "cluster-resident (DSMEM, colour lists)",
+SOR_PATHS = {0: "none", 1: "above 160^3: every SM, shared-memory regions (colour lists where they do not fit)", 2: "cluster-resident (DSMEM, colour lists)",
              3: "temporal-blocked (every SM, shared-memory regions)",
              4: "owned bricks in global memory (every SM, a grid barrier per half-sweep)"}
-SOR_KERNELS = {1: "k_sor_persistent", 2: "k_sor_cluster", 3: "k_sor_tb", 4: "k_sor_tb"}
+SOR_KERNELS = {1: "k_sor_tb", 2: "k_sor_cluster", 3: "k_sor_tb", 4: "k_sor_tb"}
 
 
 def workload_config(nP, world):

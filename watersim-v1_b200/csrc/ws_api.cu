@@ -602,6 +602,7 @@ static ws_status state_copy(ws_handle* h, const ws_host_arrays* a, bool up) {
       else WS_TRY(cudaMemcpyAsync(a->field[f], r.ptr, bytes, cudaMemcpyDeviceToHost, st));
     }
     if (pass == 0 && small.n) {
+      cudaSetDevice(h->device);                   // a launch, unlike a copy, wants the stream's device current
       launch_host_copies(small, h->stream);
       ws_status s = check_launch(h, 1); if (s) return s;
     }

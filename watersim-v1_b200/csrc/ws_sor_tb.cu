@@ -392,9 +392,11 @@ extern __shared__ __align__(16) unsigned char tb_smem_raw[];
 // exchange about 1.2 us, partly behind the first half-sweep. 1024 threads with
 // two entries each in flight: 512 with four were a third slower. Measured
 // (fixed-iteration fits, before -> now, us): 32^3 (2.9k fluid cells) plan
-// 32 -> 29, iteration 1.36 -> 1.15; 97^3 (75k) 67 -> 52, 4.05 -> 1.77; 128^3
-// (160k) 65 -> 55, 4.17 -> 2.18; 256^3 (1.09M, lists before) 143 -> 141,
-// 17.6 -> 5.9.
+// 32 -> 30, iteration 1.36 -> 1.14; 97^3 (75k) 67 -> 52, 4.05 -> 1.69; 128^3
+// (160k) 65 -> 55, 4.17 -> 2.13; 256^3 (1.09M, lists before) 143 -> 144,
+// 17.6 -> 5.9. A residual check costs 18 us more at 256^3 (the reload before
+// it overlaps nothing, and the pass); posted and collected an epoch later, with
+// the judged state stored meanwhile, a solve took 1612 instead of 1527 us.
 __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
   __shared__ int sAbort, sOverflow, nRegion, sT0, sT1, sA;
   __shared__ TbLayout sL;

@@ -50,7 +50,8 @@
 // foreign brick whose own fluid lies beyond the halo). So a list begins with
 // one word that stands for the CTA, and a CTA fetches that word of every owner
 // of an active brick around its own; brick adjacency is symmetric.
-// Tags count on from solve to solve (tagBase), so a word left by an earlier
+// Tags count on from solve to solve (tagBase; after a timed-out wait past the
+// epochs that any CTA can have run, ws_sor_tags.h), so a word left by an earlier
 // solve never matches and nothing has to be cleared.
 //
 // Overlap. Colour 0's owned cells are stored with those first that touch no
@@ -79,6 +80,7 @@
 // cooperative launch guarantees that all CTAs are resident, so a healthy
 // run never reaches the limit.
 #include "ws_kernels.cuh"
+#include "ws_sor_tags.h"
 #include <algorithm>
 #include <cstddef>
 
@@ -929,7 +931,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
 done:
   if (p == 0 && tid == 0) {
     // every CTA read the tag base before its first barrier, which this CTA has passed
-    *(volatile unsigned*)&a.ctl->tagBase = tag0 + epoch + 1u;
+    *(volatile unsigned*)&a.ctl->tagBase = tb_next_tag_base(tag0, epoch, sAbort, a.iters);
     if (solved || sAbort) a.ctl->solved = 1;         // after a timed-out wait nothing else runs either
     if (solved || sAbort) { *a.outIters = it; *a.outRel = rel; *a.outPath = path; }
   }

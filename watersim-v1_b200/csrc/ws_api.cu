@@ -586,7 +586,16 @@ static ws_status state_copy(ws_handle* h, const ws_host_arrays* a, bool up) {
     if (a->field[f] && field_ref(h, (ws_field)f, r)) total += (size_t)a->count * r.elem;
   }
   for (int pass = 0; pass < 2; pass++) {          // the temperature last
-    if (pass && scan && any_vapor_flag((const uint8_t*)a->field[WS_F_PFLAG], a->count)) h->vaporPossible = true;
+    if (pass && scan && any_vapor_flag((const uint8_t*)a->field[WS_F_PFLAG], a->count)) {
+      h->vaporPossible = true;
+      // from here on the substeps read the temperature, and an earlier upload's
+      // may still be on its way on the copy stream: both this call's and the
+      // next substep's use of it come after
+      if (h->copyPending) {
+        WS_TRY(cudaEventRecord(h->evCopy, h->copyStream));
+        WS_TRY(cudaStreamWaitEvent(h->stream, h->evCopy, 0));
+      }
+    }
     for (int f = 0; f < WS_NUM_PARTICLE_FIELDS; f++) {
       if (!a->field[f] || (f == WS_F_PT) != (pass == 1)) continue;
       FieldRef r;

@@ -777,7 +777,7 @@ static ws_status mt_volume(ws_handle* h, double iso, double* vol, int64_t* cnt) 
   void* scr = nullptr;
   ws_status s = mt_scratch(h, h->d.nCells, &scr); if (s) return s;
   const int n = launch_mt_list(h->d, h->dens, iso, scr, h->stream) +
-                launch_mt_emit(h->d, h->dens, iso, 0, nullptr, nullptr, h->redHost, scr, h->stream);
+                launch_mt_emit(h->d, h->dens, iso, 0, nullptr, nullptr, h->redHost, nullptr, scr, h->stream);
   s = check_launch(h, n); if (s) return s;
   WS_TRY(cudaStreamSynchronize(h->stream));
   if (vol) *vol = std::fabs(h->redHost[0]);
@@ -2018,7 +2018,9 @@ extern "C" ws_status ws_unet_load(ws_handle* h, const void* buf, int64_t size) {
 // ------------------------------------------------------------ surface mesh
 // MarchingTetrahedra.build (js/surface.js:66-177) of a corner field on the
 // lattice dd into mb, vertices in the reference's emission order. The buffers'
-// present size is tried first; a larger mesh grows them and emits once more.
+// present size is tried first; a larger mesh grows them and emits once more. A
+// fault latched before the call is its answer, and the last mesh stays (the
+// kernels look at the status word, so that no wait comes before them).
 static ws_status mt_build(ws_handle* h, const Dims& dd, const float* field, double iso, MeshBuf& mb, int64_t* vertices,
                           double* volume) {
   void* scr = nullptr;
@@ -2026,7 +2028,7 @@ static ws_status mt_build(ws_handle* h, const Dims& dd, const float* field, doub
   int n = launch_mt_list(dd, field, iso, scr, h->stream);
   long long cnt = 0;
   for (;;) {
-    n += launch_mt_emit(dd, field, iso, mb.cap, mb.pos, mb.nrm, h->redHost, scr, h->stream);
+    n += launch_mt_emit(dd, field, iso, mb.cap, mb.pos, mb.nrm, h->redHost, &h->st->err, scr, h->stream);
     if ((s = check_launch(h, n))) return s;
     if ((s = sync_status(h))) return s;            // the one wait: results, and faults latched before
     cnt = llround(h->redHost[1]);
@@ -2034,7 +2036,7 @@ static ws_status mt_build(ws_handle* h, const Dims& dd, const float* field, doub
     long long cap = std::max<long long>(cnt + cnt / 4, 1 << 16);
     if (mb.pos) cudaFree(mb.pos);
     if (mb.nrm) cudaFree(mb.nrm);
-    mb.pos = nullptr; mb.nrm = nullptr; mb.cap = 0;
+    mb.pos = nullptr; mb.nrm = nullptr; mb.cap = 0; mb.verts = 0;
     WS_TRY(cudaMalloc(&mb.pos, sizeof(float) * 3 * (size_t)cap));
     WS_TRY(cudaMalloc(&mb.nrm, sizeof(float) * 3 * (size_t)cap));
     mb.cap = cap;
@@ -2096,20 +2098,26 @@ extern "C" ws_status ws_metaball_mesh(ws_handle* h, double tension, double detai
   const double iso = 1.5 * std::pow((1.6 + 2.2 * t) / 1.6, 1.5);
   const int rad = std::min(3, (int)std::ceil(R));
   const long long corners = (long long)(m + 1) * (m + 1) * (m + 1), cells = (long long)m * m * m;
+  ws_status s;
   if (corners > h->mbCorners) {
+    if ((s = sync_status(h))) return s;              // a fault latched before: the field stays
+    h->mbM = 0;
     for (void* b : { (void*)h->mbAcc, (void*)h->mbField }) if (b) cudaFree(b);
     h->mbAcc = nullptr; h->mbField = nullptr; h->mbCorners = 0;
     WS_TRY(cudaMalloc(&h->mbAcc, sizeof(double) * (size_t)corners));
     WS_TRY(cudaMalloc(&h->mbField, sizeof(float) * (size_t)corners));
     h->mbCorners = corners;
   }
+  const int mBefore = h->mbM;
   h->mbM = m;
-  launch_metaball_field(parts_of(h), m, mdx, R * R, rad, h->mbAcc, h->mbField, h->stream);
-  ws_status s = check_launch(h, h->S.nP ? 2 : 1); if (s) return s;
+  launch_metaball_field(parts_of(h), m, mdx, R * R, rad, h->mbAcc, h->mbField, &h->st->err, h->stream);
+  if ((s = check_launch(h, h->S.nP ? 2 : 1))) return s;
   Dims dd = h->d;
   dd.nx = dd.ny = dd.nz = m; dd.dx = mdx; dd.nCells = cells;
   dims_fastdiv(dd);
-  return mt_build(h, dd, h->mbField, iso, h->mball, vertices, volume);
+  s = mt_build(h, dd, h->mbField, iso, h->mball, vertices, volume);
+  if (s == WS_ERR_DEVICE || s == WS_ERR_TIMEOUT) h->mbM = mBefore;   // latched before: nothing was written
+  return s;
 }
 extern "C" ws_status ws_metaball_download(ws_handle* h, float* pos, float* nrm, int64_t max_vertices) {
   if (h && h->asyncRunning.load(std::memory_order_acquire)) return WS_ERR_BUSY;

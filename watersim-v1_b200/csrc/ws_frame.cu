@@ -860,12 +860,14 @@ __global__ void __launch_bounds__(256) k_mt_list(const uint8_t* __restrict__ cfg
 // at 48^3, where its chain was the whole time); this, with the sums of the last
 // block, which writes them to host memory: 57 and 18. Rounds of 32
 // cells and 128 threads: the same.
-// pos null, or a mesh beyond maxVerts: the volume only, of whole cells
+// pos null, or a mesh beyond maxVerts: the volume only, of whole cells. A fault
+// latched in err before leaves the vertices of the last mesh as they are.
 constexpr int kMtCells = 16, kMtThreads = 4 * kMtCells;
 __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __restrict__ dens, double iso, float isoF,
                                                  const uint2* __restrict__ list, const unsigned long long* __restrict__ total,
-                                                 long long maxVerts, float* __restrict__ pos, float* __restrict__ nrm,
-                                                 double* __restrict__ partials, unsigned* ticket, double* __restrict__ out) {
+                                                 long long maxVerts, float* pos, float* __restrict__ nrm,
+                                                 double* __restrict__ partials, unsigned* ticket, double* __restrict__ out,
+                                                 const int* __restrict__ err) {
   __shared__ float cv[kMtCells][9];
   __shared__ double gr[3][kMtCells * 8];
   __shared__ double P[3][kMtCells * kMtVerts], N[3][kMtCells * kMtVerts];
@@ -879,6 +881,7 @@ __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __r
   const unsigned n = (unsigned)(*total >> 34);
   const unsigned blocks = min(gridDim.x, max((n + kMtCells - 1) / kMtCells, 1u));   // those with cells (one without any)
   if (blockIdx.x >= blocks) return;
+  if (pos && *err) pos = nullptr;
   for (int t = tid; t < 16 * 6; t += kMtThreads) ((uint8_t*)sCase)[t] = ((const uint8_t*)g_mt.cases)[t];
   if (tid < kMtEdges) { sFrom[tid] = g_mt.from[tid]; sTo[tid] = g_mt.to[tid]; }
   if (tid < 36) ((uint8_t*)sId)[tid] = ((const uint8_t*)g_mt.id)[tid];
@@ -1045,11 +1048,11 @@ int launch_mt_list(const Dims& d, const float* dens, double iso, void* scratch, 
   return 3;
 }
 int launch_mt_emit(const Dims& d, const float* dens, double iso, long long maxVerts, float* pos, float* nrm, double* out,
-                   void* scratch, cudaStream_t s) {
+                   const int* err, void* scratch, cudaStream_t s) {
   const MtScratch m = mt_carve(scratch, d.nCells);
   const int grid = (int)std::min<long long>(grid_for(d.nCells, kMtCells), kMtGrid);
   k_mt_emit<<<grid, kMtThreads, 0, s>>>(d, dens, iso, iso_floor(iso), m.list, m.tot + m.nb, maxVerts, pos, nrm, m.partials,
-                                           (unsigned*)(m.tot + m.nb + 1), out);
+                                           (unsigned*)(m.tot + m.nb + 1), out, err);
   return 1;
 }
 
@@ -1234,17 +1237,18 @@ __global__ void __launch_bounds__(256) k_mb_splat(PartsDev P, int m, double mdx,
     }
   }
 }
-__global__ void k_mb_round(const double* __restrict__ acc, float* __restrict__ field, long long n) {
+__global__ void k_mb_round(const double* __restrict__ acc, float* __restrict__ field, long long n, const int* __restrict__ err) {
+  if (*err) return;                                        // a latched fault leaves the last field
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
     field[c] = (float)acc[c];
 }
 void launch_metaball_field(const PartsDev& P, int m, double mdx, double R2, int rad, double* acc, float* field,
-                           cudaStream_t s) {
+                           const int* err, cudaStream_t s) {
   const long long corners = (long long)(m + 1) * (m + 1) * (m + 1);
   cudaMemsetAsync(acc, 0, sizeof(double) * (size_t)corners, s);
   // the bound along an axis a little wide: the exact test is on the squares
   if (P.nP > 0)
     k_mb_splat<<<grid_for(P.nP, 256), 256, 0, s>>>(P, m, mdx, 1.0 / mdx, is_pow2(mdx) ? 1 : 0, std::sqrt(R2) * (1 + 1e-12), R2,
                                                    1.0 / R2, rad, acc);
-  k_mb_round<<<(int)std::min<long long>(grid_for(corners, 256), 148 * 16), 256, 0, s>>>(acc, field, corners);
+  k_mb_round<<<(int)std::min<long long>(grid_for(corners, 256), 148 * 16), 256, 0, s>>>(acc, field, corners, err);
 }

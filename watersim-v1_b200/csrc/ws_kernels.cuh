@@ -97,12 +97,12 @@ void launch_currents(const Dims& d, const PartsDev& P, const CurrField& F, doubl
                      double oceanR, double coreR, double dt, cudaStream_t s);
 // marching tets in scratch (mt_scratch_bytes(d.nCells) bytes): the cells that
 // straddle iso, then (at the same iso) the signed volume and the vertex count
-// into out[0..1] (device or mapped host memory) and, with pos, the vertices of the cells that fit in maxVerts.
-// Both return the kernels launched.
+// into out[0..1] (device or mapped host memory) and, with pos, the vertices of the cells that fit in maxVerts,
+// unless *err holds a fault. Both return the kernels launched.
 size_t mt_scratch_bytes(long long nCells);
 int launch_mt_list(const Dims& d, const float* dens, double iso, void* scratch, cudaStream_t s);
 int launch_mt_emit(const Dims& d, const float* dens, double iso, long long maxVerts, float* pos, float* nrm, double* out,
-                   void* scratch, cudaStream_t s);
+                   const int* err, void* scratch, cudaStream_t s);
 // render-side particle prep: classify, bucket-sort far to near, emit the
 // draw list (ws_render.cu); counts land in the first five scratch words
 // balls (ws_balls.cu): moving-solid raster (after the static raster),
@@ -113,9 +113,9 @@ void launch_ball_push(const PartsDev& P, const double* balls, int nb, cudaStream
 void launch_ball_update(const Dims& d, const float* vel, const TerrainDev& t, const PartsDev& P, double* balls, int nb,
                         int* hist, float* surfY, const BallEnv& env, double dt, cudaStream_t s);
 // Metaballs.build's corner field on an (m+1)^3 lattice of spacing mdx
-// (FP64 accumulation, float result); 1 or 2 launches
+// (FP64 accumulation, float result; field untouched when *err holds a fault); 1 or 2 launches
 void launch_metaball_field(const PartsDev& P, int m, double mdx, double R2, int rad, double* acc, float* field,
-                           cudaStream_t s);
+                           const int* err, cudaStream_t s);
 size_t render_scratch_bytes(long long capacity);
 void launch_render_particles(const RenderCfg& c, const PartsDev& P, void* scratch, RenderOut o, cudaStream_t s);
 // ticket: zero before the first call (and after each); out: three doubles, device or mapped host memory

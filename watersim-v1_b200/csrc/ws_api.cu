@@ -777,7 +777,7 @@ static ws_status mt_volume(ws_handle* h, double iso, double* vol, int64_t* cnt) 
   void* scr = nullptr;
   ws_status s = mt_scratch(h, h->d.nCells, &scr); if (s) return s;
   const int n = launch_mt_list(h->d, h->dens, iso, scr, h->stream) +
-                launch_mt_emit(h->d, h->dens, iso, 0, nullptr, nullptr, h->redHost, nullptr, scr, h->stream);
+                launch_mt_emit(h->d, h->dens, iso, -1, nullptr, nullptr, h->redHost, nullptr, scr, h->stream);
   s = check_launch(h, n); if (s) return s;
   WS_TRY(cudaStreamSynchronize(h->stream));
   if (vol) *vol = std::fabs(h->redHost[0]);
@@ -2018,7 +2018,8 @@ extern "C" ws_status ws_unet_load(ws_handle* h, const void* buf, int64_t size) {
 // ------------------------------------------------------------ surface mesh
 // MarchingTetrahedra.build (js/surface.js:66-177) of a corner field on the
 // lattice dd into mb, vertices in the reference's emission order. The buffers'
-// present size is tried first; a larger mesh grows them and emits once more. A
+// present size is tried first; for a larger mesh the emission answers with its
+// count alone, and follows once they have grown. A
 // fault latched before the call is its answer, and the last mesh stays (the
 // kernels look at the status word, so that no wait comes before them).
 static ws_status mt_build(ws_handle* h, const Dims& dd, const float* field, double iso, MeshBuf& mb, int64_t* vertices,

@@ -860,8 +860,9 @@ __global__ void __launch_bounds__(256) k_mt_list(const uint8_t* __restrict__ cfg
 // at 48^3, where its chain was the whole time); this, with the sums of the last
 // block, which writes them to host memory: 57 and 18. Rounds of 32
 // cells and 128 threads: the same.
-// pos null, or a mesh beyond maxVerts: the volume only, of whole cells. A fault
-// latched in err before leaves the vertices of the last mesh as they are.
+// maxVerts negative: the volume only. A mesh beyond maxVerts: its vertex count
+// only, at once (the scan has it), so that the caller makes room and emits once.
+// A fault latched in err before leaves the vertices of the last mesh as they are.
 constexpr int kMtCells = 16, kMtThreads = 4 * kMtCells;
 __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __restrict__ dens, double iso, float isoF,
                                                  const uint2* __restrict__ list, const unsigned long long* __restrict__ total,
@@ -871,7 +872,7 @@ __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __r
   __shared__ float cv[kMtCells][9];
   __shared__ double gr[3][kMtCells * 8];
   __shared__ double P[3][kMtCells * kMtVerts], N[3][kMtCells * kMtVerts];
-  __shared__ unsigned short vdesc[kMtCells * kMtVerts], tdesc[kMtCells * 12], tv[kMtCells * 12][3];
+  __shared__ unsigned short vdesc[kMtCells * kMtVerts], tv[kMtCells * 12][3];
   __shared__ int ci[kMtCells], cj[kMtCells], ck[kMtCells], sNV, sNT;
   __shared__ unsigned mask[kMtCells], tri0;
   __shared__ unsigned short vBase[kMtCells], tBase[kMtCells];
@@ -879,6 +880,11 @@ __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __r
   __shared__ double sv[kMtThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31;
   const unsigned n = (unsigned)(*total >> 34);
+  const double nVerts = 3.0 * (double)(*total & ((1ull << 34) - 1));
+  if (maxVerts >= 0 && nVerts > (double)maxVerts) {
+    if (blockIdx.x == 0 && tid == 0) out[1] = nVerts;
+    return;
+  }
   const unsigned blocks = min(gridDim.x, max((n + kMtCells - 1) / kMtCells, 1u));   // those with cells (one without any)
   if (blockIdx.x >= blocks) return;
   if (pos && *err) pos = nullptr;
@@ -939,13 +945,11 @@ __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __r
         for (int t = 0; t < 6; t++) {
           const int code = (m >> sTet[t][0] & 1) | (m >> sTet[t][1] & 1) << 1 | (m >> sTet[t][2] & 1) << 2 | (m >> sTet[t][3] & 1) << 3;
           for (int u = 0; u < sNTri[code]; u++, at++)
-            if ((at & 3) == part) {
-              tdesc[at] = (unsigned short)cell;
+            if ((at & 3) == part)
               for (int vi = 0; vi < 3; vi++) {
                 const int id = sId[t][sCase[code][u][vi]];
                 tv[at][vi] = (unsigned short)(vBase[cell] + __popc(e & ((1u << id) - 1u)));
               }
-            }
         }
     }
     __syncthreads();
@@ -981,21 +985,13 @@ __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __r
               P[2][a] * (P[0][b] * P[1][c] - P[0][c] * P[1][b])) / 6;
     }
     __syncthreads();
-    if (pos) {
-      const bool whole = ((long long)tri0 + nT) * 3 <= maxVerts;
+    // the next round's corners, before its first barrier, touch none of what this reads
+    if (pos)
       for (int f = tid; f < nT * 9; f += kMtThreads) {
         const int t = f / 9, r = f - t * 9, vi = r / 3, q = r - vi * 3, v = tv[t][vi];
-        if (!whole) {
-          const int cell = tdesc[t];
-          if (((long long)tri0 + tBase[cell] + g_mt.tris[cfg[cell]]) * 3 > maxVerts) continue;
-        }
         pos[(long long)tri0 * 9 + f] = (float)P[q][v];
         nrm[(long long)tri0 * 9 + f] = (float)N[q][v];
       }
-    }
-    // the next round's corners touch none of what the output reads; cfg and
-    // tBase (read when the mesh overflows) are rewritten after its first barrier
-    if (pos && ((long long)tri0 + nT) * 3 > maxVerts) __syncthreads();
   }
   vol = warp_sum(vol);
   if (lane == 0) sv[tid >> 5] = vol;
@@ -1013,7 +1009,7 @@ __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __r
   __syncthreads();
   if (tid == 0) {
     for (int w = 1; w < kMtThreads / 32; w++) vol += sv[w];
-    out[0] = vol; out[1] = 3.0 * (double)(*total & ((1ull << 34) - 1));
+    out[0] = vol; out[1] = nVerts;
   }
 }
 // scratch: list (8 bytes a cell), block totals and ticket, partial volumes, sign patterns

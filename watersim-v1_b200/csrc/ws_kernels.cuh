@@ -97,8 +97,8 @@ void launch_currents(const Dims& d, const PartsDev& P, const CurrField& F, doubl
                      double oceanR, double coreR, double dt, cudaStream_t s);
 // marching tets in scratch (mt_scratch_bytes(d.nCells) bytes): the cells that
 // straddle iso, then (at the same iso) the signed volume and the vertex count
-// into out[0..1] (device or mapped host memory) and, with pos, the vertices of the cells that fit in maxVerts,
-// unless *err holds a fault. Both return the kernels launched.
+// into out[0..1] (device or mapped host memory) and, with pos, the vertices, unless *err holds a fault; a mesh of
+// more than maxVerts (0 or more) vertices: the count alone. Both return the kernels launched.
 size_t mt_scratch_bytes(long long nCells);
 int launch_mt_list(const Dims& d, const float* dens, double iso, void* scratch, cudaStream_t s);
 int launch_mt_emit(const Dims& d, const float* dens, double iso, long long maxVerts, float* pos, float* nrm, double* out,

@@ -213,7 +213,7 @@ ws_status ws_surface_device(ws_handle* h, const float** pos, const float** nrm, 
 /* ---- metaball skin: Metaballs.build (js/surface.js:203-284). Every liquid
  *      particle adds the kernel (1 - d²/R²)² to the corners of an (m+1)³ lattice
  *      over the box, m = max(6, round(nx·detail)) (detail clamped to 0.5..1.6;
- *      NaN or <= 0 means 1), R = (1.6 + 2.2·tension)·spacing in lattice cells
+ *      NaN or <= 0 means 1; m beyond 1624 is WS_ERR_RANGE), R = (1.6 + 2.2·tension)·spacing in lattice cells
  *      (tension clamped to 0..1, NaN means 0.5); the field is contoured at
  *      1.5·((1.6 + 2.2·tension)/1.6)^1.5 by the marching-tets mesher into a
  *      device buffer the handle owns (separate from the surface mesh). The

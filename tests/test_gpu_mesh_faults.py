@@ -66,3 +66,18 @@ def test_latched_fault_leaves_the_mesh(kind, arg, first):
     m, f = _field(fs)
     assert m == field[0] and np.array_equal(f.view(np.uint32), field[1].view(np.uint32))
     fs.close()
+
+
+def test_metaball_lattice_limit():
+    """A long thin grid asks for an nx^3 lattice: beyond 32-bit corner indices
+    (1625^3 < 2^32 < 1626^3 corners) the call is refused."""
+    from fluid_solver import FluidSolver
+    assert 1625 ** 3 < 2 ** 32 < 1626 ** 3
+    fs = FluidSolver(nx=1700, ny=4, nz=4, dx=1.0, coreR=1.0, targetParticles=10.0, capacity=100)
+    fs.set_scalars(spacing=0.5, nP=0)
+    for detail in (1.0, 1.6, 0.9558):                     # 0.9558 * 1700 = 1624.9, rounded to 1625
+        with pytest.raises(WsError) as ei:
+            _build(fs, "metaball", detail)
+        assert ei.value.code == -7
+    assert _mesh(fs, "metaball")[0] == 0
+    fs.close()

@@ -2092,6 +2092,9 @@ extern "C" ws_status ws_metaball_mesh(ws_handle* h, double tension, double detai
   if (std::isfinite(detail) && detail > 0) f = detail < 0.5 ? 0.5 : (detail > 1.6 ? 1.6 : detail);
   const int nx = h->d.nx;
   const int m = std::max(6, (int)js_round(nx * f));
+  // corner and cell indices are 32-bit; a grid this long (1016 cells at least, the
+  // other axes short) would also outrun the 64-bit corner count
+  if (m > 1624) return fail(h, WS_ERR_RANGE, "metaball lattice beyond 1624 cells an axis");
   const double mdx = m == nx ? h->d.dx : h->d.W / m;
   double t = std::isfinite(tension) ? tension : 0.5;
   t = t < 0 ? 0 : (t > 1 ? 1 : t);

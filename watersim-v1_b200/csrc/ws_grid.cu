@@ -503,7 +503,6 @@ void launch_mark_p2g(const Dims& d, const GridDev& g, const PartsDev& P, const T
 // only the order of the FP32 sums differs. A particle whose stencil leaves
 // the brick's faces (a ball pushed it after the binning) adds its terms to
 // global memory directly.
-static unsigned brick_grid(const BrickSet& B);
 
 // The stage-wise P2G, without a mark pass that counted: the particles P2G
 // scatters (pflag 0, finite state) counted per cell, each with its rank.
@@ -642,7 +641,12 @@ int launch_p2g_sorted(const Dims& d, const GridDev& g, const PartsDev& P, const 
     return -1;
   launches += 2;
   k_cell_scatter<<<grid_for(P.nP, 256), 256, 0, s>>>(P.nP, cs, &st->err);
-  k_p2g_bricks<<<brick_grid(B), 256, 0, s>>>(d, g, P, cs, B, binned ? 0 : 1, &st->err);
+  // A block takes a brick at a time; up to 16 rounds of them are evened out, as a
+  // ragged last round shows there (64^3 with 193k particles 97.5 -> 94.5 us, 97^3 with
+  // 0.7M 198 -> 190), beyond them all blocks run (128^3: 401, evened 433). The face
+  // passes' grid of four bricks a block took 64 us for 32^3 with 10k particles, this 42.
+  const int nB = B.nbx * B.nby * B.nbz, most = 148 * 8, rounds = (nB + most - 1) / most;
+  k_p2g_bricks<<<rounds <= 16 ? (nB + rounds - 1) / rounds : most, 256, 0, s>>>(d, g, P, cs, B, binned ? 0 : 1, &st->err);
   return launches + 2;
 }
 

@@ -337,8 +337,12 @@ __global__ void __launch_bounds__(1024) k_evap_band(const double* __restrict__ w
 }
 // Each window: its candidates' base states and thresholds in shared memory,
 // then one warp per tabulated input. A surface of 20k candidates has five
-// windows, so blocks along y share a window's inputs: with one block of 32
-// warps per window five SMs worked through eight rounds, 114 us; now 24.
+// windows, so several blocks share a window's inputs, as many as the grid has for
+// each of the windows that hold candidates (known on the device only; the
+// number of windows that the particles could fill, 3700 at 256^3 with 15.3M, left
+// eight warps each). The stage takes 145 us at 64^3 with 193k particles (250 with
+// one block of 32 warps a window), 357 at 128^3 with 1.86M (425), 2275 at 256^3
+// (2460; 3140 with eight warps).
 constexpr int kEvTableThreads = 256;
 __global__ void __launch_bounds__(kEvTableThreads) k_evap_table(const long long* __restrict__ thr, const int* __restrict__ nCp,
                                                                 int t0, const uint32_t* __restrict__ sStart,
@@ -347,21 +351,27 @@ __global__ void __launch_bounds__(kEvTableThreads) k_evap_table(const long long*
   __shared__ uint32_t sb[kEvW];
   __shared__ long long sthr[kEvW];
   constexpr int warps = kEvTableThreads / 32;
-  const int nC = *nCp, w = blockIdx.x, keff = st->evKeff;
-  if (w >= ev_windows(nC, t0) || (int)blockIdx.y * warps >= keff) return;
-  const int lo = t0 + w * kEvW, n = min(kEvW, nC - lo);
-  uint32_t A, C, bj = lcg_jump(*sStart, (uint32_t)(lo - t0 + (int)threadIdx.x + 1));
+  const int nC = *nCp, keff = st->evKeff, nW = ev_windows(nC, t0);
+  if (nW == 0) return;
+  const int parts = max(1, min((keff + warps - 1) / warps, (int)gridDim.x / nW));
+  uint32_t A, C;
   lcg_affine(kEvTableThreads, A, C);
-  for (int j = (int)threadIdx.x; j < n; j += kEvTableThreads, bj = A * bj + C) {
-    sb[j] = bj;
-    if (blockIdx.y == 0) bOut[lo + j] = bj;
-    sthr[j] = thr[lo + j];
-  }
-  __syncthreads();
-  const int Lw = L[w];
-  for (int k = (int)blockIdx.y * warps + (int)(threadIdx.x >> 5); k < keff; k += warps * (int)gridDim.y) {
-    const int eo = ev_resolve(sb, sthr, n, Lw + k, [](int, int, uint32_t) {});
-    if ((threadIdx.x & 31) == 0) table[(size_t)w * kEvKMax + k] = (unsigned short)(eo - (Lw + k));
+  for (int item = (int)blockIdx.x; item < nW * parts; item += (int)gridDim.x) {
+    const int w = item / parts, part = item - w * parts;
+    const int lo = t0 + w * kEvW, n = min(kEvW, nC - lo);
+    uint32_t bj = lcg_jump(*sStart, (uint32_t)(lo - t0 + (int)threadIdx.x + 1));
+    for (int j = (int)threadIdx.x; j < n; j += kEvTableThreads, bj = A * bj + C) {
+      sb[j] = bj;
+      if (part == 0) bOut[lo + j] = bj;
+      sthr[j] = thr[lo + j];
+    }
+    __syncthreads();
+    const int Lw = L[w];
+    for (int k = part * warps + (int)(threadIdx.x >> 5); k < keff; k += warps * parts) {
+      const int eo = ev_resolve(sb, sthr, n, Lw + k, [](int, int, uint32_t) {});
+      if ((threadIdx.x & 31) == 0) table[(size_t)w * kEvKMax + k] = (unsigned short)(eo - (Lw + k));
+    }
+    __syncthreads();                              // the window's states and thresholds are read
   }
 }
 // One warp: the ejection count entering every window.
@@ -477,9 +487,10 @@ void launch_evap_pass(int nP, const int* list, const int* nC, const EvapScratch&
   const int nw = (int)ev_max_windows(nP);
   k_evap_wsum<<<nw, 256, 0, s>>>(es.thr, nC, t0, es.wsum);
   k_evap_band<<<1, 1024, 0, s>>>(es.wsum, nC, t0, es.L, st);
-  // up to one warp per input of the widest band, fewer where the windows alone fill the device
-  const int ny = std::max(1, std::min(kEvKMax * 32 / kEvTableThreads / 4, 148 * 16 / nw));
-  k_evap_table<<<dim3(nw, ny), kEvTableThreads, 0, s>>>(es.thr, nC, t0, sStart, es.L, st, es.b, es.table);
+  // twelve rounds of the four blocks an SM holds: with four or eight a window's
+  // share is too coarse at 256^3 (3150 us), with 32 the windows' loads come back
+  const int blocks = (int)std::min<long long>((long long)nw * (kEvKMax / 32), 148 * 48);
+  k_evap_table<<<blocks, kEvTableThreads, 0, s>>>(es.thr, nC, t0, sStart, es.L, st, es.b, es.table);
   k_evap_chain<<<1, 32, 0, s>>>(nC, t0, es.L, es.table, es.b, es.thr, sStart, es.Ew, st);
   k_evap_emit<<<nw, 256, 0, s>>>(nC, t0, es.b, es.thr, es.Ew, list, eoff, es.ejP, es.ejS, st);
 }

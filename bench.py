@@ -290,10 +290,11 @@ def run_ours(args, rank, world, local_rank):
     return out, fs
 
 
-SOR_PATHS = {0: "none", 1: "above 160^3: every SM, shared-memory regions (colour lists where they do not fit)", 2: "cluster-resident (DSMEM, colour lists)",
+SOR_PATHS = {0: "none", 1: "above 160^3: every SM, shared-memory regions (colour lists where they do not fit)",
+             2: "cluster-resident (DSMEM, colour lists)",
              3: "temporal-blocked (every SM, shared-memory regions)",
              4: "owned bricks in global memory (every SM, a grid barrier per half-sweep)"}
-SOR_KERNELS = {1: "k_sor_tb", 2: "k_sor_cluster", 3: "k_sor_tb", 4: "k_sor_tb"}
+SOR_KERNELS = {1: "k_sor_persistent", 2: "k_sor_cluster", 3: "k_sor_tb", 4: "k_sor_tb"}
 
 
 def workload_config(nP, world):
@@ -425,6 +426,7 @@ def roofline(fs, ms_step, iters):
     keep = fs.pressureIters
     fs.pressureIters = it
     us_sor = fs.time_kernel(6, 5)                 # whole solve of `it` iterations
+    sor_name = SOR_KERNELS.get(fs.timed_solve()[0], "k_sor_tb")   # the kernel that solved it
     fs.pressureIters = keep
     # the face passes as the substep runs them: over the active-brick list of
     # the last substep (ids 8-11); their bytes count the faces of those bricks
@@ -447,8 +449,6 @@ def roofline(fs, ms_step, iters):
     #  G2P+advect    52 B per particle + 8 B per face (u and uO)
     #  faces pass 1  8 B acc + 9 B out per face; forces 12 B per face; project 8 B per face;
     #                extrapolation 5 B per face (flag + value), all over the active bricks' faces
-    # the path the timed solve took (its own diagnostics, read after it ran)
-    sor_name = SOR_KERNELS.get(fs.scalars.sorPath, "k_sor_tb")
     cand = {sor_name: (us_sor, 13.0 * nF * it),
             "k_p2g_runs": (us_p2g, 25.0 * nP + 8.0 * F),
             "k_g2p_advect": (us_g2p, 52.0 * nP + 8.0 * F),

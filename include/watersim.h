@@ -111,10 +111,11 @@ typedef struct {
   int32_t nP, capacity;
   int32_t airborneCount, vaporCount, nightVaporCount, evapCount, substepsLast, nFluid;
   int32_t sorIters;        /* iterations run by the last solve */
-  int32_t sorPath;         /* solve path of the last solve: 1 grids above 160^3, every SM's lists in shared
-                              memory or (where they do not fit) grid-wide, 2 cluster-resident colour lists,
-                              3 temporal-blocked on every SM (shared-memory regions),
-                              4 owned bricks in global memory on every SM (regions too large) */
+  int32_t sorPath;         /* solve path of the last solve: 1 grids above 160^3, regions in shared memory or
+                              (where they do not fit) grid-wide colour lists (ws_timed_solve tells them
+                              apart), 2 cluster-resident colour lists, 3 regions in shared memory on
+                              every SM, 4 owned bricks in global memory on every SM (regions too large, or
+                              fluid on the outermost layer) */
 } ws_scalars;
 
 /* Named fields — the typed arrays of FluidSolver (js/solver.js:94-129). */
@@ -381,7 +382,7 @@ ws_status ws_ocean_point(ws_handle* h, double minDepth, double* xyz);
  * microseconds. Runs on the current state (timing only; the state advances
  * as if the kernels ran). kernel: 0 one red-black SOR iteration (two
  * launches, reported per launch), 1 P2G scatter in particle index order (one
- * atomic per particle and face; the substep uses 12), 2 fused G2P + advection,
+ * atomic per particle and face; the substep's default), 2 fused G2P + advection,
  * 3 faces pass 1 (normalise + BC + snapshot), 4 forces pass, 5 projection,
  * 6 one whole SOR solve of pressureIters iterations on the default path
  * (reported per solve), 7 the same solve on the colour-list path (cluster-
@@ -392,6 +393,11 @@ ws_status ws_ocean_point(ws_handle* h, double minDepth, double* xyz);
  * cell sums with one atomic per touched face; every brick visited), reported
  * per whole P2G. */
 ws_status ws_time_kernel(ws_handle* h, int32_t kernel, int32_t reps, double* us_per_launch);
+/* The outcome of the last solve that ws_time_kernel 6 or 7 ran on the handle (0
+ * before): iterations, residual, and the path it took, numbered on every grid
+ * size as 1 grid-wide colour lists, 2 cluster-resident colour lists, 3 regions in
+ * shared memory, 4 owned bricks in global memory. NULL skips an output. */
+ws_status ws_timed_solve(ws_handle* h, int32_t* path, int32_t* iters, double* relres);
 ws_status ws_synchronize(ws_handle* h);
 /* Failure-detection check (no counterpart in the reference, whose solver
  * has no device waits): one device thread waits for a status word that

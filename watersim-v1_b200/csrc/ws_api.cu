@@ -1638,6 +1638,16 @@ extern "C" ws_status ws_time_kernel(ws_handle* h, int32_t kernel, int32_t reps, 
   return sync_status(h);
 }
 
+// what the last solve of ws_time_kernel left (that call ended with the status word on the host)
+extern "C" ws_status ws_timed_solve(ws_handle* h, int32_t* path, int32_t* iters, double* relres) {
+  if (h && h->asyncRunning.load(std::memory_order_acquire)) return WS_ERR_BUSY;
+  if (!h) return WS_ERR_INVALID;
+  if (path) *path = h->stHost->timedPath;
+  if (iters) *iters = h->stHost->timedIters;
+  if (relres) *relres = h->stHost->timedRel;
+  return WS_OK;
+}
+
 // ------------------------------------------------------------ learned warm start
 static ws_status net_ready(ws_handle* h) {
   if (!h) return WS_ERR_INVALID;

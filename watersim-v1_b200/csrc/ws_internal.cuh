@@ -134,7 +134,7 @@ struct DevStatus {
   unsigned int evSEnd, evSStart;   // stream after the pass; start state of a restarted pass
   int oddFluid;            // the pressure setup met a fluid cell on the domain's outermost layer (zeroed by the raster)
   double sorOmega;         // omega of the last pressure setup (pw = omega / diag)
-  double timedRel;         // the outcome of a solve that a timing call runs, apart from the substep's
+  double timedRel;         // the outcome of the last solve that a timing call ran (ws_timed_solve)
   int timedIters, timedPath;
 };
 // where a solve leaves its iteration count, relative residual and path

@@ -138,6 +138,7 @@ struct TbArgs {
   TbCtl* ctl;
   double om1;
   int iters, check, listFallback;
+  int regionPath;                // the path number that the solve in shared memory reports
   double tol;
   int* err;
   int* outIters;
@@ -412,7 +413,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
   const int P = gridDim.x, p = blockIdx.x, tid = threadIdx.x, T = kTbThreads;
   const int lane = tid & 31, warp = tid >> 5;
   const Dims& d = a.d;
-  int it = 0, path = a.listFallback ? 1 : 3;
+  int it = 0, path = a.regionPath;
   unsigned epoch = 0, nBar = 0;
   double rel = -1;
   bool solved = false;
@@ -1023,6 +1024,7 @@ cudaError_t launch_sor_tb(void* statePtr, const Dims& d, const GridDev& g, const
   a.xmap = S->xmap; a.glist = S->glist; a.plist = S->plist; a.dense = S->dense; a.flist = S->flist; a.resPart = S->resPart; a.ctl = S->ctl;
   a.om1 = 1 - omega; a.iters = iters; a.check = check; a.tol = tol; a.err = &st->err;
   a.listFallback = listFallback ? 1 : 0;
+  a.regionPath = report && listFallback ? 1 : 3;   // ws_scalars.sorPath has one number for both above 160^3
   const SorOut out(st, report);
   a.outIters = out.iters; a.outRel = out.rel; a.outPath = out.path;
   void* args[] = { &a };

@@ -156,7 +156,7 @@ SYMBOLS = ["ws_create", "ws_destroy", "ws_last_error", "ws_version", "ws_set_par
            "ws_substep", "ws_stage", "ws_residual", "ws_mt_volume", "ws_autotune_iso", "ws_census",
            "ws_kinetic_energy", "ws_apply_impulse_sphere", "ws_stir_at", "ws_stir_gaussian",
            "ws_wave_impulse", "ws_dry_land_fraction", "ws_sample_vel", "ws_terrain_radius_at", "ws_ocean_point",
-           "ws_synchronize", "ws_get_stream", "ws_launch_count", "ws_time_kernel", "ws_probe_wait",
+           "ws_synchronize", "ws_get_stream", "ws_launch_count", "ws_time_kernel", "ws_timed_solve", "ws_probe_wait",
            "ws_residual_noalloc", "ws_upload_state", "ws_download_state",
            "ws_unet_init", "ws_unet_init_levels", "ws_unet_collect", "ws_unet_enable", "ws_unet_train", "ws_unet_get_info",
            "ws_unet_get_weights", "ws_unet_set_weights", "ws_unet_set_gain", "ws_unet_get_pair",
@@ -202,6 +202,7 @@ def load_library(path=None):
         "ws_synchronize": [h], "ws_get_stream": [h, C.POINTER(C.c_void_p)],
         "ws_launch_count": [h, C.POINTER(C.c_int64)],
         "ws_time_kernel": [h, i32, i32, C.POINTER(C.c_double)],
+        "ws_timed_solve": [h, C.POINTER(i32), C.POINTER(i32), C.POINTER(d)],
         "ws_probe_wait": [h, C.c_int64],
         "ws_upload_state": [h, C.POINTER(WsHostArrays)], "ws_download_state": [h, C.POINTER(WsHostArrays)],
         "ws_unet_init": [h, u32], "ws_unet_init_levels": [h, u32, i32], "ws_unet_collect": [h, i32], "ws_unet_enable": [h, i32],
@@ -751,3 +752,9 @@ class FluidSolver:
         us = C.c_double()
         self._check(self._L.ws_time_kernel(self._h, int(kernel), int(reps), C.byref(us)))
         return us.value
+
+    def timed_solve(self):
+        """(path, iterations, relative residual) of the last solve that time_kernel(6) or (7) ran."""
+        path, iters, rel = C.c_int32(), C.c_int32(), C.c_double()
+        self._check(self._L.ws_timed_solve(self._h, C.byref(path), C.byref(iters), C.byref(rel)))
+        return path.value, iters.value, rel.value

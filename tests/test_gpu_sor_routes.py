@@ -132,4 +132,8 @@ def test_fluid_on_the_outermost_layer(n, path, timed):
     fs.time_kernel(6, 1)
     assert fs.timed_solve()[:2] == (timed, 5)
     assert _bitwise(fs.q.copy(), q)
+    fs.upload("q", q0)
+    fs.time_kernel(7, 1)                     # the lists: grid-wide, though a cluster would hold the small ones
+    assert fs.timed_solve()[:2] == (1, 5)
+    assert _bitwise(fs.q.copy(), q)
     fs.close()

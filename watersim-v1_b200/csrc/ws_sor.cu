@@ -216,6 +216,7 @@ struct SorArgs {
   const int* offs;     // per 256-cell chunk b: its first list entry of colour 0 and 1 (offs[2 b], offs[2 b + 1])
   int nChunks;
   const int* solved;   // the region solve's flag (null: none ran)
+  const int* odd;      // fluid on the outermost layer: its pressure is read, which the cluster solve does not hold
 };
 
 // One colour's half-sweep over the lists in global memory, three cells per
@@ -443,7 +444,7 @@ __global__ void __launch_bounds__(1024, 1) k_sor_persistent(SorArgs a) {
   const unsigned T = gridDim.x * blockDim.x;
   const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int n0 = a.L.count[0], n1 = a.L.count[1];
-  if (n0 <= a.clusterCap && n1 <= a.clusterCap) return;      // the cluster solve ran
+  if (n0 <= a.clusterCap && n1 <= a.clusterCap && !*a.odd) return;      // the cluster solve ran
   if (n0 + n1 == 0) {                  // no fluid cell: no sweep (js/solver.js:1330)
     if (tid == 0) { *a.outIters = 0; *a.outRel = 0; *a.outPath = 1; }
     return;
@@ -472,6 +473,7 @@ struct ClusterArgs {
   int* outIters;
   double* outRel;
   int* outPath;
+  const int* odd;
 };
 extern __shared__ __align__(16) unsigned char sor_smem[];
 
@@ -506,7 +508,7 @@ __global__ void __launch_bounds__(1024, 1) k_sor_cluster(ClusterArgs a) {
   const int C = (int)cl.num_blocks();
   const int rank = (int)cl.block_rank();
   const int n0 = a.L.count[0], n1 = a.L.count[1];
-  if (n0 > C * kSmax || n1 > C * kSmax) return;         // uniform: the grid solve takes it
+  if (n0 > C * kSmax || n1 > C * kSmax || *a.odd) return;   // uniform: the grid solve takes it
   if (n0 + n1 == 0) {                                    // no fluid cell: no sweep (js/solver.js:1330)
     if (rank == 0 && threadIdx.x == 0) { *a.outIters = 0; *a.outRel = 0; *a.outPath = 2; }
     return;
@@ -730,7 +732,7 @@ static cudaError_t run_lists(SorState* S, const Dims& d, const GridDev& g, doubl
   if (C) {
     ClusterArgs ca;
     ca.d = d; ca.q = g.q; ca.L = S->L; ca.om1 = 1 - omega; ca.iters = iters; ca.check = check; ca.tol = tol;
-    ca.outIters = out.iters; ca.outRel = out.rel; ca.outPath = out.path;
+    ca.outIters = out.iters; ca.outRel = out.rel; ca.outPath = out.path; ca.odd = &st->oddFluid;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -746,7 +748,7 @@ static cudaError_t run_lists(SorState* S, const Dims& d, const GridDev& g, doubl
   a.outIters = out.iters; a.outRel = out.rel; a.outPath = out.path;
   a.clusterCap = C ? C * kSmax : -1;
   a.offs = S->blockOffs; a.nChunks = (int)grid_for(d.nCells, 256);
-  a.solved = solved;
+  a.solved = solved; a.odd = &st->oddFluid;
   void* args[] = { &a };
   return cudaLaunchCooperativeKernel((void*)k_sor_persistent, dim3(S->grid), dim3(S->block), args, 0, s);
 }

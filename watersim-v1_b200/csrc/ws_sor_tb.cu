@@ -93,8 +93,8 @@ constexpr int kRbMax = 896;                 // region bricks per CTA
 constexpr int kHMax = 4;                    // half-sweeps per epoch where the regions fit
 constexpr int kHashSlots = 2048;            // open-addressing table of region bricks
 constexpr int kQMax = 16384;                // stored cells per CTA (the neighbour indices hold 16 bits)
-constexpr int kPubMax = 8192;               // published cells per CTA
-constexpr int kFetchMax = 8192;             // halo cells per CTA
+constexpr int kPubMax = 8192;               // published words per CTA
+constexpr int kFetchMax = 8192;             // fetched words per CTA
 constexpr long long kTbSpinLimit = 4000000LL;
 constexpr int kMaxCtas = 1024;
 constexpr int kTbSmem = 229376;             // dynamic shared memory: the 227 KB of a block less the static part
@@ -115,11 +115,15 @@ struct TbCtl {
   unsigned tagBase;              // exchange tags of this solve start after it
 };
 
+// What one CTA can hold on this grid (tb_caps); the plan checks its counts
+// against them, so a list never outgrows its place.
+struct TbCaps { int own, pub, fetch, rows; };
+
 struct TbArgs {
   Dims d;
   float* q;
-  u64* xq;                       // exchange: per CTA two lists of kPubMax words (q bits | tag << 32)
-  unsigned* xmap;                // [2][nCells]: place of a published cell (owner * 2 * kPubMax + position), H = 2 and 4
+  u64* xq;                       // exchange: per CTA two lists of caps.pub words (q bits | tag << 32)
+  unsigned* xmap;                // [2][nCells]: place of a published cell (owner * 2 * caps.pub + position), H = 2 and 4
   const float* rhs;
   const float* pw;               // omega/diag, negative off the fluid
   const uint8_t* diag8;
@@ -130,10 +134,11 @@ struct TbArgs {
   int* actLin;                   // active brick t -> linear brick index
   int* wPre;                     // linear (active) brick -> chunk weight before it
   int* chunkStart;               // CTA -> first owned active brick ([P] = number of active bricks)
-  unsigned* glist;               // per CTA: global cell of each owned cell by its stored index (kQMax)
-  unsigned short* dense;         // per CTA: stored index of each region cell (64 kRbMax), where shared memory has no room
-  unsigned short* plist;         // per CTA: stored index of each published cell (kPubMax)
-  uint2* flist;                  // per CTA: (place in xq, stored index) of each halo cell (kFetchMax)
+  TbCaps caps;
+  unsigned* glist;               // per CTA: global cell of each owned cell, colour 0 first (caps.own)
+  unsigned short* dense;         // per CTA: stored index of each region cell (64 caps.rows), where shared memory has no room
+  unsigned short* plist;         // per CTA: stored index of each published cell (caps.pub)
+  uint2* flist;                  // per CTA: (place in xq, stored index) of each halo cell (caps.fetch)
   double2* resPart;              // 2 x P residual partials
   TbCtl* ctl;
   double om1;
@@ -362,9 +367,15 @@ struct TbLayout {
   int pub, fetch;                // words published and fetched: the cells and the CTAs' own words
 };
 // bytes of the solve's values and records: the cells, the zero cell and one that takes the CTAs' own words, then the entries
-__device__ __forceinline__ int record_at(int NQ) { return (4 * (NQ + 2) + 15) & ~15; }
+__host__ __device__ __forceinline__ int record_at(int NQ) { return (4 * (NQ + 2) + 15) & ~15; }
+// where a region of R bricks has its dense index table in shared memory: before
+// the second tables, clear of the first and of the records; -1 without room
+__host__ __device__ __forceinline__ int dense_at(int R, int NQ, int NE) {
+  const int at = (kTbSmem - (int)sizeof(TbPlan2)) / 16 * 16 - R * 128;
+  return at >= (int)sizeof(TbPlan) && at >= record_at(NQ) + 16 * NE ? at : -1;
+}
 // whether the solve's values and records fit with epochs of H half-sweeps
-__device__ __forceinline__ bool make_layout(TbLayout& L, int H, int pub, int fetch) {
+__device__ __forceinline__ bool make_layout(TbLayout& L, const TbCaps& c, int R, int H, int pub, int fetch) {
   L.H = H; L.pub = pub; L.fetch = fetch;
   int at = 0;
   for (int d = 0; d < H; d++) { L.off[0][d] = at; at += L.n[0][d]; }
@@ -374,12 +385,13 @@ __device__ __forceinline__ bool make_layout(TbLayout& L, int H, int pub, int fet
     L.off[1][d] = at; at += L.n[1][d];
   }
   L.NQ = at;
-  for (int c = 0; c < 2; c++) {
+  for (int col = 0; col < 2; col++) {
     int sum = 0;
-    for (int d = 0; d < kHMax; d++) { sum += L.n[c][d]; L.cum[c][d] = sum; }
+    for (int d = 0; d < kHMax; d++) { sum += L.n[col][d]; L.cum[col][d] = sum; }
   }
-  return L.NQ < kQMax && pub <= kPubMax && fetch <= kFetchMax &&
-         record_at(L.NQ) + 16 * L.NE <= (kTbSmem - (int)sizeof(TbPlan2)) / 16 * 16;
+  return L.NQ < kQMax && pub <= c.pub && fetch <= c.fetch && L.n[0][0] + L.n[1][0] <= c.own &&
+         record_at(L.NQ) + 16 * L.NE <= (kTbSmem - (int)sizeof(TbPlan2)) / 16 * 16 &&
+         (R <= c.rows || dense_at(R, L.NQ, L.NE) >= 0);
 }
 
 }  // namespace
@@ -600,8 +612,8 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
       sL.n[0][0] = sCnt[0] + sCnt[4]; sL.n[1][0] = sCnt[1];
       for (int q = 0; q < kHMax; q++) { sL.n[0][q + 1] = sCnt[5 + 2 * q]; sL.n[1][q + 1] = sCnt[6 + 2 * q]; }
       const bool no = sOverflow || a.st->oddFluid != 0;
-      if (no || !make_layout(sL, 2, sCnt[2], sCnt[13])) atomicOr(&a.ctl->over2, 1);
-      if (no || !make_layout(sL, 4, sCnt[3], sCnt[14])) atomicOr(&a.ctl->over4, 1);
+      if (no || !make_layout(sL, a.caps, R, 2, sCnt[2], sCnt[13])) atomicOr(&a.ctl->over2, 1);
+      if (no || !make_layout(sL, a.caps, R, 4, sCnt[3], sCnt[14])) atomicOr(&a.ctl->over4, 1);
     }
     // where the other CTAs find this one's cells, for both epoch lengths
     for (int x = tid; x < std::min(O, R) * 64; x += T) {
@@ -611,7 +623,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
         const u64 m = S.cm[w][s];
         if ((m >> c) & 1ull)
           __stcg(a.xmap + (size_t)w * (size_t)d.nCells + cell_global(a, S2, s, c),
-                 (unsigned)p * (2u * kPubMax) + 1u + (unsigned)(S.base[2 + w][s] + bits_below(m, c)));
+                 (unsigned)p * (2u * (unsigned)a.caps.pub) + 1u + (unsigned)(S.base[2 + w][s] + bits_below(m, c)));
       }
     }
     if (!tb_grid_barrier(a.ctl, ++nBar, a.err, &sAbort)) goto done;
@@ -619,7 +631,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
       const bool over4 = ld_acquire(reinterpret_cast<const unsigned*>(&a.ctl->over4)) != 0;
       const bool over2 = ld_acquire(reinterpret_cast<const unsigned*>(&a.ctl->over2)) != 0;
       sOverflow = over4 && over2;
-      if (!sOverflow) make_layout(sL, over4 ? 2 : 4, sCnt[over4 ? 2 : 3], sCnt[over4 ? 13 : 14]);
+      if (!sOverflow) make_layout(sL, a.caps, R, over4 ? 2 : 4, sCnt[over4 ? 2 : 3], sCnt[over4 ? 13 : 14]);
     }
     __syncthreads();
 
@@ -627,18 +639,18 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
       const TbLayout& L = sL;
       const int which = L.H == 2 ? 0 : 1;
       uint4* rec = reinterpret_cast<uint4*>(tb_smem_raw + record_at(L.NQ));
-      unsigned char* room = reinterpret_cast<unsigned char*>(&S2) - (size_t)R * 128;
-      const bool clear = room >= tb_smem_raw + sizeof(TbPlan) && room >= reinterpret_cast<unsigned char*>(rec + L.NE);
-      unsigned short* dense = clear ? reinterpret_cast<unsigned short*>(room) : a.dense + (size_t)p * 64 * kRbMax;
-      unsigned* gl = a.glist + (size_t)p * kQMax;
-      unsigned short* pl = a.plist + (size_t)p * kPubMax;
-      uint2* fl = a.flist + (size_t)p * kFetchMax;
+      const int room = dense_at(R, L.NQ, L.NE);
+      unsigned short* dense = room >= 0 ? reinterpret_cast<unsigned short*>(tb_smem_raw + room)
+                                        : a.dense + (size_t)p * 64 * a.caps.rows;
+      unsigned* gl = a.glist + (unsigned)p * (unsigned)a.caps.own;
+      unsigned short* pl = a.plist + (unsigned)p * (unsigned)a.caps.pub;
+      uint2* fl = a.flist + (unsigned)p * (unsigned)a.caps.fetch;
       if (tid == 0) pl[0] = (unsigned short)L.NQ;
       if (tid < P && ((sOwn[tid >> 5] >> (tid & 31)) & 1u)) {
         int at = L.fetch - 1;                      // the list's end: the CTAs' own words
         for (int w = kMaxCtas / 32 - 1; w > (tid >> 5); w--) at -= __popc(sOwn[w]);
         at -= __popc(sOwn[tid >> 5] & ~((2u << (tid & 31)) - 1u));
-        fl[at] = make_uint2((unsigned)tid * (2u * kPubMax), (unsigned)L.NQ + 1u);
+        fl[at] = make_uint2((unsigned)tid * (2u * (unsigned)a.caps.pub), (unsigned)L.NQ + 1u);
       }
       // the stored index of every region cell (NQ, the zero cell, for the
       // others), its global cell, and the lists of published and fetched cells
@@ -663,7 +675,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
         if (e == L.NQ) continue;
         const unsigned g = cell_global(a, S2, s, c);
         if (s < O) {
-          gl[e] = g;
+          gl[col ? e - L.c1 + L.n[0][0] : e] = g;
           const u64 m = S.cm[which][s];
           if ((m >> c) & 1ull) pl[1 + S.base[2 + which][s] + bits_below(m, c)] = (unsigned short)e;
         } else {
@@ -704,9 +716,9 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
     const int nPub = sL.pub, nFetch = sL.fetch;
     float* sq = reinterpret_cast<float*>(tb_smem_raw);
     const uint4* rec = reinterpret_cast<const uint4*>(tb_smem_raw + record_at(NQ));
-    const unsigned* gl = a.glist + (size_t)p * kQMax;
-    const unsigned short* pl = a.plist + (size_t)p * kPubMax;
-    const uint2* fl = a.flist + (size_t)p * kFetchMax;
+    const unsigned* gl = a.glist + (unsigned)p * (unsigned)a.caps.own;
+    const unsigned short* pl = a.plist + (unsigned)p * (unsigned)a.caps.pub;
+    const uint2* fl = a.flist + (unsigned)p * (unsigned)a.caps.fetch;
     // a thread keeps its first four cells to fetch and to publish
     unsigned fg[4];
     unsigned short fe[4], pe[4];
@@ -724,7 +736,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
     // the halo values of epoch `ep`: four loads in flight per thread, then
     // each word polled again (bounded) until its tag is the epoch's
     auto wait_and_reload = [&](unsigned ep) -> bool {
-      const u64* src = a.xq + (ep & 1u) * (size_t)kPubMax;
+      const u64* src = a.xq + (ep & 1u) * (unsigned)a.caps.pub;
       const unsigned target = tag0 + ep;
       u64 v[4];
       auto settle = [&](int e, const u64* w, u64 val) {
@@ -751,7 +763,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
       return *(volatile int*)&sAbort == 0;
     };
     auto publish = [&](unsigned ep) {
-      u64* dst = a.xq + ((size_t)p * 2 + (ep & 1u)) * (size_t)kPubMax;
+      u64* dst = a.xq + ((unsigned)p * 2u + (ep & 1u)) * (unsigned)a.caps.pub;
       const u64 tag = (u64)(tag0 + ep) << 32;
 #pragma unroll
       for (int u = 0; u < 4; u++) if (tid + u * T < nPub) st_relaxed_u64(dst + tid + u * T, tag | __float_as_uint(sq[pe[u]]));
@@ -854,7 +866,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) k_sor_tb(TbArgs a) {
     // the result lands in the solve's own q buffer
     for (int x = tid; x < n00 + n10; x += T) {
       const int e = x < n00 ? x : c1s + (x - n00);
-      __stcg(a.q + gl[e], sq[e]);
+      __stcg(a.q + gl[x], sq[e]);
     }
     solved = true;
   } else if (!a.listFallback) {
@@ -950,7 +962,26 @@ struct TbState {
   uint2* flist = nullptr;
   double2* resPart = nullptr;
   int P = 0, nbx = 0, nby = 0, nbz = 0, mbits = 0;
+  TbCaps caps{};
 };
+// The most that one of P CTAs can hold on a grid of nB bricks. Its owned bricks but
+// the last weigh less than its share of the total (at most 80 a brick) together, and
+// a brick weighs 17 at least. A halo cell lies within L1 distance 4 of an
+// owned brick: 704 cells around each. The dense tables need global memory only
+// where they may have no room beside the records. With every list at its maximum a
+// 24^3 handle held 58 MB for the solve, so 10.
+static TbCaps tb_caps(const Dims& d, long long nB, int P) {
+  const long long weight = (kBrickWeight + 64) * nB / P + kBrickWeight + 64, bricks = std::min(nB, weight / (kBrickWeight + 1));
+  const long long cells = (long long)(d.nx - 2) * (d.ny - 2) * (d.nz - 2);
+  const long long own = std::min(cells, std::min(64 * bricks, weight)), halo = std::min(cells, 704 * bricks);
+  const long long region = std::min<long long>(kRbMax, std::min(nB, 27 * bricks)), all = std::min<long long>(kQMax - 1, own + halo);
+  TbCaps c;
+  c.own = (int)std::min<long long>(kQMax, own);
+  c.pub = (int)std::min<long long>(kPubMax, own + 1);
+  c.fetch = (int)std::min<long long>(kFetchMax, halo + P);
+  c.rows = dense_at((int)region, (int)all, (int)all) >= 0 ? 0 : (int)region;
+  return c;
+}
 
 // null when the solve cannot run on this device (too little shared memory or
 // co-residency) or grid (a brick coordinate beyond 8 bits); the state is
@@ -980,15 +1011,16 @@ cudaError_t sor_tb_init(void** statePtr, const Dims& d, int device) {
   S->mbits = mb;
   const long long nB = (long long)S->nbx * S->nby * S->nbz;
   // every buffer from one allocation (exchange words zeroed: tags start at 1)
-  const size_t P = (size_t)smCount, words = 2 * kPubMax * P;
+  S->caps = tb_caps(d, nB, smCount);
+  const size_t P = (size_t)smCount, words = 2 * (size_t)S->caps.pub * P;
   size_t at = 0;
   auto place = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~(size_t)255; return o; };
   const size_t oCtl = place(sizeof(TbCtl)), oXq = place(sizeof(u64) * words), oCnt = place(sizeof(int2) * P);
   const size_t zeroed = at;
   const size_t oAct = place(sizeof(int) * (size_t)nB), oPre = place(sizeof(int) * (size_t)nB);
   const size_t oChunk = place(sizeof(int) * (P + 1)), oMap = place(sizeof(unsigned) * 2 * (size_t)d.nCells);
-  const size_t oG = place(sizeof(unsigned) * kQMax * P), oP = place(sizeof(unsigned short) * kPubMax * P);
-  const size_t oD = place(sizeof(unsigned short) * 64 * kRbMax * P), oF = place(sizeof(uint2) * kFetchMax * P);
+  const size_t oG = place(sizeof(unsigned) * S->caps.own * P), oP = place(sizeof(unsigned short) * S->caps.pub * P);
+  const size_t oD = place(sizeof(unsigned short) * 64 * S->caps.rows * P), oF = place(sizeof(uint2) * S->caps.fetch * P);
   const size_t oRes = place(sizeof(double2) * 2 * P);
   cudaError_t e;
   if ((e = cudaMalloc(&S->slab, at)) != cudaSuccess) return e;
@@ -1021,7 +1053,7 @@ cudaError_t launch_sor_tb(void* statePtr, const Dims& d, const GridDev& g, const
   a.d = d; a.q = g.q; a.xq = S->xq; a.rhs = g.rhs; a.pw = g.pw; a.diag8 = diag8; a.fmask = g.fmask; a.st = st;
   a.nbx = S->nbx; a.nby = S->nby; a.nbz = S->nbz; a.mbits = S->mbits;
   a.cntPart = S->cntPart; a.actLin = S->actLin; a.wPre = S->wPre; a.chunkStart = S->chunkStart;
-  a.xmap = S->xmap; a.glist = S->glist; a.plist = S->plist; a.dense = S->dense; a.flist = S->flist; a.resPart = S->resPart; a.ctl = S->ctl;
+  a.xmap = S->xmap; a.glist = S->glist; a.plist = S->plist; a.dense = S->dense; a.caps = S->caps; a.flist = S->flist; a.resPart = S->resPart; a.ctl = S->ctl;
   a.om1 = 1 - omega; a.iters = iters; a.check = check; a.tol = tol; a.err = &st->err;
   a.listFallback = listFallback ? 1 : 0;
   a.regionPath = report && listFallback ? 1 : 3;   // ws_scalars.sorPath has one number for both above 160^3

@@ -137,3 +137,20 @@ def test_fluid_on_the_outermost_layer(n, path, timed):
     assert fs.timed_solve()[:2] == (1, 5)
     assert _bitwise(fs.q.copy(), q)
     fs.close()
+
+
+def test_route_after_the_outermost_layer_has_dried():
+    """The next cell types, with a closed layer and no raster pass between, take the regions again."""
+    fs, q0, _ = _system(33, 0.3, 5, False)
+    assert fs.scalars.sorPath == 4
+    ct = fs.cellType.reshape(33, 33, 33).copy()
+    for a in range(3):
+        np.moveaxis(ct, a, 0)[[0, -1]] = 2
+    fs.upload("cellType", ct.ravel())
+    q0 = np.where(ct.ravel() == 1, q0, 0).astype(np.float32)
+    fs.upload("q", q0)
+    fs.stage("PRESSURE")
+    assert fs.scalars.sorPath == 3
+    q = fs.q.copy()
+    assert _bitwise(q, _colours(fs, q0, 5))
+    fs.close()

@@ -1193,6 +1193,8 @@ __global__ void __launch_bounds__(256) k_pressure_setup(Dims d, GridDev g, uint8
 }
 void launch_pressure_setup(const Dims& d, const GridDev& g, uint8_t* diag8, double omega, DevStatus* st,
                            const BrickSet& B, bool allBricks, cudaStream_t s) {
+  // a stage on its own may follow cell types of a caller's, without a raster pass between
+  if (allBricks) cudaMemsetAsync(&st->oddFluid, 0, sizeof(int), s);
   k_pressure_setup<<<brick_grid(B), 256, 0, s>>>(d, g, diag8, omega, st, B, allBricks ? 1 : 0);
 }
 

@@ -132,7 +132,7 @@ struct DevStatus {
   unsigned long long evIrr;   // evaporation pass: (ejection << 32 | candidate) of the first irregular kick
   int evNEj, evNC, evKeff;    // ejections in the pass, candidates, tabulated band width
   unsigned int evSEnd, evSStart;   // stream after the pass; start state of a restarted pass
-  int oddFluid;            // the pressure setup met a fluid cell on the domain's outermost layer (zeroed by the raster)
+  int oddFluid;            // the pressure setup met a fluid cell on the domain's outermost layer (zeroed by the raster and by a setup on its own)
   double sorOmega;         // omega of the last pressure setup (pw = omega / diag)
   double timedRel;         // the outcome of the last solve that a timing call ran (ws_timed_solve)
   int timedIters, timedPath;

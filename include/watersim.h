@@ -15,9 +15,15 @@
  *    wait that ran out) are latched in a device status word and reported by
  *    the next call that synchronises.
  *  - Host pointers are owned by the caller and read or written only during
- *    the call. Device memory is owned by the handle.
- *  - One CUDA stream per handle (ws_get_stream): all of a call's work is
- *    ordered after earlier work on it and before later work on it.
+ *    the call (ws_upload_state: some until a later one, see there). Device
+ *    memory is owned by the handle.
+ *  - One CUDA stream per handle (ws_get_stream): a call's work is ordered
+ *    after earlier work on it and before later work on it, except the copies
+ *    of the fields that no substep uses in ws_upload_state and
+ *    ws_download_state: they run on a second, internal stream, and the
+ *    handle's stream waits for them at the next call other than ws_substep
+ *    and ws_download_state. A caller's own work on the handle's stream that
+ *    reads those arrays comes after such a call (ws_synchronize, say).
  *    Calls on one handle must be serialised by
  *    the caller (a frame started by ws_step_async holds the handle until it
  *    is collected; other calls meanwhile return WS_ERR_BUSY). There is no

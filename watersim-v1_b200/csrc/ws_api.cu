@@ -263,7 +263,7 @@ extern "C" ws_status ws_create(const ws_config* cfg, ws_handle** out) {
     if (h->evCopy) cudaEventDestroy(h->evCopy);
     if (h->evMain) cudaEventDestroy(h->evMain);
     if (h->copyStream) cudaStreamDestroy(h->copyStream);
-      if (h->stream) cudaStreamDestroy(h->stream);
+    if (h->stream) cudaStreamDestroy(h->stream);
     delete h; return r;
   }
   Dims& d = h->d;

@@ -1,5 +1,9 @@
 // ws_sor.cu — the pressure solve of _pressureSolve (js/solver.js:1368-1404)
-// as one persistent cooperative kernel.
+// as one persistent cooperative kernel over colour lists. It solves what the
+// region solve (ws_sor_tb.cu) leaves: above 160^3 cells a system whose regions do
+// not fit or that has fluid on the outermost layer, every system of a grid beyond
+// 1020 cells an axis (there in one cluster where that holds the lists), and
+// ws_time_kernel 7.
 //
 // The fluid cells (about 5% of the 128^3 box) are compacted per red-black
 // colour into lists in cell order (rhs, omega/diag and diag copied beside

@@ -79,13 +79,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 }
 
 // Output planes per work item. 16 channels: eight (a whole tile), bound by the
-// MMAs' operand reads, which more planes per halo plane share. 32: four, since
-// the half-resolution level of a 128^3 grid has about as many tiles (151) as
-// SMs, and with a tile per item each SM staged and multiplied in turn (4500 and
-// 5500 cycles a slice): the layers' mean 32.1 us with eight planes, 25.3 with
-// four, 29.8 with two. 48 to 128: two, as on the coarse levels a tile per item
-// would leave most SMs idle (the 32^3 level has 32 tiles) and each CTA would
-// walk four or more input slices in turn; four for 48 changed nothing.
+// MMAs' operand reads, which more planes per halo plane share. 32: four, so that
+// two or three CTAs an SM overlap staging and MMAs (4500 and 5500 cycles a slice)
+// where a tile per item gives it one: a whole prediction takes 207 us at 64^3 (229
+// with eight planes), 267 at 97^3 (269), 327 at 128^3 (327), 1304 at 256^3 with four
+// levels (1320); in the training at 128^3, whose half-resolution level has about as
+// many tiles as SMs, those layers' mean is 25.3 us (32.1; 29.8 with two). 48 to 128:
+// two, as on the coarse levels a tile per item would leave most SMs idle (the 32^3
+// level has 32 tiles) and each CTA would walk four or more input slices in turn;
+// four for 48 changed nothing.
 template <int COUT> struct ConvShape {
   static constexpr int ZT = COUT == 16 ? 8 : COUT == 32 ? 4 : COUT <= 128 ? 2 : 1;
   static constexpr int HX = kTX + 2, HY = kTY + 2, HZ = ZT + 2;

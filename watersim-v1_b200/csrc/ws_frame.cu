@@ -890,6 +890,7 @@ __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __r
   __shared__ uint8_t cfg[kMtCells], sFrom[kMtEdges], sTo[kMtEdges], sId[6][6], sTet[6][4], sCase[16][2][3], sNTri[16];
   __shared__ double sv[kMtThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31;
+  const int fault = err ? *err : 0;                        // in flight with the total
   const unsigned n = (unsigned)(*total >> 34);
   const double nVerts = 3.0 * (double)(*total & ((1ull << 34) - 1));
   if (maxVerts >= 0 && nVerts > (double)maxVerts) {
@@ -898,7 +899,7 @@ __global__ void __launch_bounds__(kMtThreads) k_mt_emit(Dims d, const float* __r
   }
   const unsigned blocks = min(gridDim.x, max((n + kMtCells - 1) / kMtCells, 1u));   // those with cells (one without any)
   if (blockIdx.x >= blocks) return;
-  if (pos && *err) pos = nullptr;
+  if (fault) pos = nullptr;
   for (int t = tid; t < 16 * 6; t += kMtThreads) ((uint8_t*)sCase)[t] = ((const uint8_t*)g_mt.cases)[t];
   if (tid < kMtEdges) { sFrom[tid] = g_mt.from[tid]; sTo[tid] = g_mt.to[tid]; }
   if (tid < 36) ((uint8_t*)sId)[tid] = ((const uint8_t*)g_mt.id)[tid];
@@ -1245,9 +1246,9 @@ __global__ void __launch_bounds__(256) k_mb_splat(PartsDev P, int m, double mdx,
   }
 }
 __global__ void k_mb_round(const double* __restrict__ acc, float* __restrict__ field, long long n, const int* __restrict__ err) {
-  if (*err) return;                                        // a latched fault leaves the last field
+  const bool keep = *err != 0;                             // a latched fault leaves the last field
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
-    field[c] = (float)acc[c];
+    { const float v = (float)acc[c]; if (!keep) field[c] = v; }
 }
 void launch_metaball_field(const PartsDev& P, int m, double mdx, double R2, int rad, double* acc, float* field,
                            const int* err, cudaStream_t s) {

@@ -154,3 +154,24 @@ def test_route_after_the_outermost_layer_has_dried():
     q = fs.q.copy()
     assert _bitwise(q, _colours(fs, q0, 5))
     fs.close()
+
+
+def test_grid_longer_than_the_region_plan():
+    """Brick coordinates of the plan hold 8 bits: beyond 1020 cells an axis the lists solve, in one cluster."""
+    shape = (9, 10, 1032)
+    fs = FluidSolver(nx=shape[2], ny=shape[1], nz=shape[0], dx=1.0, coreR=1.0, targetParticles=1000.0, capacity=1000)
+    r = np.random.default_rng(5)
+    ct = np.where(r.random(shape) < 0.4, 1, 0).astype(np.uint8)
+    for a in range(3):
+        np.moveaxis(ct, a, 0)[[0, -1]] = 2
+    fs.set_params(sorTol=0.0, pressureIters=7, omega=1.7)
+    fs.upload("cellType", ct.ravel())
+    for k in ("u", "v", "w"):
+        fs.upload(k, r.normal(size=fs.field_size(k)).astype(np.float32))
+    q0 = np.where(ct.ravel() == 1, r.normal(size=ct.size), 0).astype(np.float32)
+    fs.upload("q", q0)
+    fs.stage("PRESSURE")
+    assert fs.scalars.sorPath == 2 and fs.scalars.sorIters == 7
+    q = fs.q.copy()
+    assert _bitwise(q, _colours(fs, q0, 7)) and not _bitwise(q, q0)
+    fs.close()
